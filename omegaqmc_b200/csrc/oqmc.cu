@@ -106,6 +106,7 @@ static bool nocc_supported(int n) {
 static OqLaunch make_launch(const oqmc_ctx* ctx, void* stream, size_t smem) {
   OqLaunch L;
   L.sys = ctx->d_sys; L.split = ctx->d_split; L.C64 = ctx->d_C64; L.C32 = ctx->d_C32;
+  L.ao = ctx->d_ao; L.ao_bytes = ctx->ao_bytes; L.ext = ctx->ao_ext;
   L.flags = ctx->d_flags; L.stream = (cudaStream_t)stream; L.smem = smem;
   return L;
 }
@@ -382,6 +383,62 @@ extern "C" int oqmc_spec_source_desc(const oqmc_system_desc* d, char* buf, size_
   return (int)src.size();
 }
 
+// The packed tables of the FP64 evaluation (layout at OqAoHead): groups in
+// atom order, groups of more than two contraction columns split into pairs.
+static std::vector<unsigned char> pack_ao(const OqSystem& S, const double* C) {
+  const int N = S.nocc, NP = (N + 1) / 2 * 2;
+  std::vector<OqAoAtom> atoms(S.natm);
+  std::vector<int4> groups;
+  std::vector<double2> prim;
+  bool ext = S.has_bs1 || S.has_bs2 || S.has_j3;
+  for (int ia = 0; ia < S.natm; ++ia) {
+    OqAoAtom& a = atoms[ia];
+    memset(&a, 0, sizeof(a));
+    a.x = S.nuc[ia][0]; a.y = S.nuc[ia][1]; a.z = S.nuc[ia][2];
+    a.Z = S.Z[ia]; a.j1a = S.j1a[ia]; a.j1b = S.j1b[ia];
+    a.g0 = (int)groups.size();
+    for (int g = 0; g < S.ngroup; ++g) {
+      if (S.g_iat[g] != ia) continue;
+      for (int k = 0; k < S.g_ncol[g]; k += 2) {
+        const int sh = S.g_shell0[g] + k, nc = S.g_ncol[g] - k >= 2 ? 2 : 1;
+        int bits = 0;
+        for (int c = 0; c < nc; ++c) {
+          if (S.g_am[g] == 0 && S.s_cusp[sh + c]) bits |= 0x100 << c;
+          if (S.has_spl && S.s_spl[sh + c] >= 0) bits |= 0x400 << c;
+        }
+        ext = ext || bits || S.g_am[g] > 2;
+        groups.push_back(make_int4(S.g_am[g] | nc << 4 | bits | sh << 16, S.g_n[g],
+                                   (int)prim.size(), S.s_ao[sh]));
+        for (int p = 0; p < S.g_n[g]; ++p) {
+          prim.push_back(make_double2(S.alpha[S.g_off[g] + p], S.norm[S.s_norm[sh] + p]));
+          if (nc == 2) prim.push_back(make_double2(S.norm[S.s_norm[sh + 1] + p], 0.0));
+        }
+      }
+    }
+    a.g1 = (int)groups.size();
+  }
+  OqAoHead h;
+  memset(&h, 0, sizeof(h));
+  h.natm = S.natm; h.has_j1 = S.has_j1; h.has_j2 = S.has_j2; h.e_nn = S.e_nn;
+  h.ext = ext;
+  memcpy(h.j2, S.j2, sizeof(h.j2));
+  h.off_group = (int)(sizeof(h) + atoms.size() * sizeof(OqAoAtom));
+  h.off_prim = h.off_group + (int)(groups.size() * sizeof(int4));
+  h.off_C = h.off_prim + (int)(prim.size() * sizeof(double2));
+  h.bytes = h.off_C + (int)(sizeof(double) * S.nbf * NP);
+  std::vector<unsigned char> b(h.bytes, 0);
+  memcpy(b.data(), &h, sizeof(h));
+  memcpy(b.data() + sizeof(h), atoms.data(), atoms.size() * sizeof(OqAoAtom));
+  memcpy(b.data() + h.off_group, groups.data(), groups.size() * sizeof(int4));
+  memcpy(b.data() + h.off_prim, prim.data(), prim.size() * sizeof(double2));
+  double* c = reinterpret_cast<double*>(b.data() + h.off_C);
+  for (int a = 0; a < S.nbf; ++a)
+    for (int m = 0; m < N; ++m) c[(size_t)a * NP + m] = C[(size_t)a * N + m];
+  return b;
+}
+static_assert(sizeof(OqAoHead) % 16 == 0 && sizeof(OqAoAtom) % 16 == 0,
+              "the packed tables are copied in 16-byte chunks");
+
 extern "C" int oqmc_create(oqmc_ctx** out, const oqmc_system_desc* d) {
   if (!out || !d) return set_err(nullptr, OQ_ERR_ARG, "null argument%s");
   *out = nullptr;
@@ -431,6 +488,11 @@ extern "C" int oqmc_create(oqmc_ctx** out, const oqmc_system_desc* d) {
     S.spl_knots = ctx->d_spl_knots;
     S.spl_coef = ctx->d_spl_coef;
   }
+  const std::vector<unsigned char> ao = pack_ao(S, d->C);
+  ctx->ao_bytes = (int)ao.size();
+  ctx->ao_ext = reinterpret_cast<const OqAoHead*>(ao.data())->ext;
+  e = (e == cudaSuccess) ? cudaMalloc(&ctx->d_ao, ao.size()) : e;
+  e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_ao, ao.data(), ao.size(), cudaMemcpyHostToDevice) : e;
   e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_sys, &S, sizeof(OqSystem), cudaMemcpyHostToDevice) : e;
   e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_split, &ctx->hsplit, sizeof(OqSplit), cudaMemcpyHostToDevice) : e;
   e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_C64, d->C, sizeof(double) * c32.size(), cudaMemcpyHostToDevice) : e;
@@ -455,6 +517,7 @@ int oqmc_destroy(oqmc_ctx* ctx) {
   cudaFree(ctx->d_split);
   cudaFree(ctx->d_C64);
   cudaFree(ctx->d_C32);
+  cudaFree(ctx->d_ao);
   cudaFree(ctx->d_flags);
   cudaFree(ctx->d_j3);
   cudaFree(ctx->d_spl_knots);

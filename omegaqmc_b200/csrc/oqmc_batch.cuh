@@ -323,7 +323,7 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
   const int w = w0 + wl;
   double logdet = 0.0;
   {
-    // FP64 refresh of the spin blocks (as k_refresh): both on the walker's
+    // FP64 refresh of the spin blocks: both on the walker's
     // thread when P = 1, spin s on lane s otherwise
     bool ok = true;
     if (live && lane < 2) {

@@ -26,6 +26,8 @@ struct oqmc_ctx {
   OqSplit* d_split;
   double* d_C64;
   float* d_C32;
+  unsigned char* d_ao;     // packed tables of the FP64 evaluation (OqAoHead ...)
+  int ao_bytes, ao_ext;    // ao_ext: OqAoHead::ext
   unsigned* d_flags;
   double* d_j3;            // three-body Jastrow gamma blocks (or null)
   double* d_spl_knots;     // radial spline tables (or null)

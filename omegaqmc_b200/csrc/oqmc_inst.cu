@@ -22,50 +22,59 @@ static cudaError_t oq_smem_attr(K kernel, size_t smem) {
   return cudaSuccess;
 }
 
-cudaError_t OQ_FN(oq_eval)(const OqLaunch& L, const double* X, int W, double* logpsi,
-                           double* grad, double* lap, double* eparts) {
-  const int tpb = 128, nb = (W + tpb - 1) / tpb;
-  cudaError_t e = oq_smem_attr(k_eval<OQ_N>, L.smem);
+// One tile kernel (oqmc_team.cuh); the tile's arrays follow the packed tables.
+template <int MODE, typename Real, bool EXT>
+static cudaError_t team_ext(const OqLaunch& L, OqTeamArgs a) {
+  a.wb = oq_team_walkers<OQ_N>(a.W);
+  a.flags = L.flags;
+  // at least 128 threads, so that a small tile copies the system tables fast
+  const int act = a.wb * 2 * OQ_N, tpb = act < 128 ? 128 : (act + 31) / 32 * 32;
+  const size_t smem = L.ao_bytes + oq_team_tile_bytes(OQ_N, a.wb);
+  cudaError_t e = oq_smem_attr(k_team<OQ_N, MODE, Real, EXT>, smem);
   if (e != cudaSuccess) return e;
-  k_eval<OQ_N><<<nb, tpb, L.smem, L.stream>>>(L.sys, L.C64, X, W, logpsi, grad, lap,
-                                                eparts, L.flags);
+  k_team<OQ_N, MODE, Real, EXT><<<(a.W + a.wb - 1) / a.wb, tpb, smem, L.stream>>>(L.sys, L.ao,
+                                                                            L.ao_bytes, a);
   return cudaGetLastError();
 }
 
+template <int MODE, typename Real>
+static cudaError_t team(const OqLaunch& L, const OqTeamArgs& a) {
+  return L.ext ? team_ext<MODE, Real, true>(L, a) : team_ext<MODE, Real, false>(L, a);
+}
+
+cudaError_t OQ_FN(oq_eval)(const OqLaunch& L, const double* X, int W, double* logpsi,
+                           double* grad, double* lap, double* eparts) {
+  OqTeamArgs a{};
+  a.X = X; a.W = W; a.logpsi = logpsi; a.grad = grad; a.lap = lap; a.eparts = eparts;
+  return team<OQ_TEAM_EVAL, double>(L, a);
+}
+
 cudaError_t OQ_FN(oq_logpsi)(const OqLaunch& L, const double* X, int W, double* logpsi) {
-  const int tpb = 128, nb = (W + tpb - 1) / tpb;
-  cudaError_t e = oq_smem_attr(k_logpsi<OQ_N>, L.smem);
+  OqTeamArgs a{};
+  a.X = X; a.W = W; a.logpsi = logpsi;
+  return team<OQ_TEAM_LOGPSI, double>(L, a);
+}
+
+template <bool EXT>
+static cudaError_t movals(const OqLaunch& L, const double* X, int W, double* out) {
+  const int tpb = 128;
+  const long long n = (long long)W * 2 * OQ_N;
+  const int nb = (int)((n + tpb - 1) / tpb);
+  cudaError_t e = oq_smem_attr(k_mo_values<OQ_N, EXT>, L.ao_bytes);
   if (e != cudaSuccess) return e;
-  k_logpsi<OQ_N><<<nb, tpb, L.smem, L.stream>>>(L.sys, L.C64, X, W, logpsi, L.flags);
+  k_mo_values<OQ_N, EXT><<<nb, tpb, L.ao_bytes, L.stream>>>(L.sys, L.ao, L.ao_bytes, X, W, out);
   return cudaGetLastError();
 }
 
 cudaError_t OQ_FN(oq_movals)(const OqLaunch& L, const double* X, int W, double* out) {
-  const int tpb = 128;
-  const long long n = (long long)W * 2 * OQ_N;
-  const int nb = (int)((n + tpb - 1) / tpb);
-  cudaError_t e = oq_smem_attr(k_mo_values<OQ_N>, L.smem);
-  if (e != cudaSuccess) return e;
-  k_mo_values<OQ_N><<<nb, tpb, L.smem, L.stream>>>(L.sys, L.C64, X, W, out);
-  return cudaGetLastError();
+  return L.ext ? movals<true>(L, X, W, out) : movals<false>(L, X, W, out);
 }
 
 cudaError_t OQ_FN(oq_refresh)(const OqLaunch& L, const double* pos, int W, void* ainv,
                               double* logdet, int mixed) {
-  const int tpb = 128, nb = (W + tpb - 1) / tpb;
-  cudaError_t e;
-  if (mixed) {
-    e = oq_smem_attr(k_refresh<OQ_N, float>, L.smem);
-    if (e != cudaSuccess) return e;
-    k_refresh<OQ_N, float><<<nb, tpb, L.smem, L.stream>>>(L.sys, L.C64, pos, W, (float*)ainv,
-                                                           logdet, L.flags);
-  } else {
-    e = oq_smem_attr(k_refresh<OQ_N, double>, L.smem);
-    if (e != cudaSuccess) return e;
-    k_refresh<OQ_N, double><<<nb, tpb, L.smem, L.stream>>>(L.sys, L.C64, pos, W,
-                                                            (double*)ainv, logdet, L.flags);
-  }
-  return cudaGetLastError();
+  OqTeamArgs a{};
+  a.X = pos; a.W = W; a.ainv = ainv; a.logpsi = logdet;
+  return mixed ? team<OQ_TEAM_REFRESH, float>(L, a) : team<OQ_TEAM_REFRESH, double>(L, a);
 }
 
 template <int PROP>
@@ -190,7 +199,7 @@ cudaError_t OQ_FN(oq_moves_alle)(const OqLaunch& L, const OqMoveArgs& a, int mix
 }
 
 // Per-thread local memory (bytes) of one kernel this size launches: kind 0
-// k_refresh, 1 k_moves (prop 0/1/2), 2 k_eloc, 3 k_eloc_tc, 4 k_md_refresh,
+// k_team (refresh), 1 k_moves (prop 0/1/2), 2 k_eloc, 3 k_eloc_tc, 4 k_md_refresh,
 // 5 k_md_moves, 6 k_md_local (M = 8 or 16 columns), 7 k_moves_alle.
 template <typename K>
 static cudaError_t oq_lmem(K kernel, size_t* out) {
@@ -210,7 +219,8 @@ static cudaError_t md_lmem(int kind, size_t* out) {
 cudaError_t OQ_FN(oq_local_bytes)(int kind, int mixed, int prop, int M, size_t* out) {
   switch (kind) {
     case 0:
-      return mixed ? oq_lmem(k_refresh<OQ_N, float>, out) : oq_lmem(k_refresh<OQ_N, double>, out);
+      return mixed ? oq_lmem(k_team<OQ_N, OQ_TEAM_REFRESH, float, true>, out)
+                   : oq_lmem(k_team<OQ_N, OQ_TEAM_REFRESH, double, true>, out);
     case 1:
       if (prop == 2)
         return mixed ? oq_lmem(k_moves<OQ_N, float, float, 2>, out)

@@ -5,12 +5,15 @@
 #include <cuda_runtime.h>
 #include "oqmc_eloc_tc.cuh"
 #include "oqmc_multidet.cuh"
+#include "oqmc_team.cuh"
 
 struct OqLaunch {
   const OqSystem* sys;
   const OqSplit* split;
   const double* C64;
   const float* C32;
+  const unsigned char* ao;   // packed tables of the FP64 evaluation (oqmc_team.cuh)
+  int ao_bytes, ext;
   unsigned* flags;
   cudaStream_t stream;
   size_t smem;

@@ -18,7 +18,7 @@
 // Precision (template T/Real): T is the type of the AO/MO arithmetic and
 // Real the storage type of the inverse.  FP64 build: T = Real = double.
 // Mixed build: T = Real = float for moves and the MO VGL, with FP64 kept for
-// positions, the periodic LU refresh (k_refresh), the Coulomb terms and all
+// positions, the periodic refresh of the inverses (k_team), the Coulomb terms and all
 // energy accumulation.  Exponent groups whose tightest exponent exceeds
 // `tight` are evaluated in FP64 for electrons within the group's split
 // radius of their nucleus (the large-exponent Laplacian term
@@ -299,48 +299,6 @@ struct OqBasisTable {
 //   ainv   [2*N*N][W] Real         ainv[((s*N + m)*N + j)*W + w] = (S_s^-1)[m][j]
 //   logdet [W] double              log|det up| + log|det down|
 // ---------------------------------------------------------------------------
-
-// Refresh: FP64 Slater matrices from positions, Gauss-Jordan inverse,
-// stored as Real.  One thread per walker.
-template <int NOCC, typename Real>
-__global__ void __launch_bounds__(128)
-k_refresh(const OqSystem* __restrict__ gsys, const double* __restrict__ gC,
-          const double* __restrict__ pos, int W, Real* __restrict__ ainv,
-          double* __restrict__ logdet, unsigned* __restrict__ flags) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  OqSystem& S = *reinterpret_cast<OqSystem*>(smem);
-  double* C = reinterpret_cast<double*>(smem + sizeof(OqSystem));
-  oq_load_system(&S, gsys);
-  // the count comes from global memory: the shared copy S is complete only
-  // after the barrier below
-  const int nbf_g = gsys->nbf;
-  for (int i = threadIdx.x; i < nbf_g * NOCC; i += blockDim.x) C[i] = gC[i];
-  __syncthreads();
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
-  if (w >= W) return;
-  double ld_tot = 0.0;
-  bool ok = true;
-  for (int s = 0; s < 2; ++s) {
-    double Sm[NOCC][NOCC], Ai[NOCC][NOCC];
-    for (int i = 0; i < NOCC; ++i) {
-      const int e = 2 * i + s;
-      double mv[NOCC];
-      oq_mo_val<NOCC>(S, C, pos[(size_t)(3 * e) * W + w], pos[(size_t)(3 * e + 1) * W + w],
-                      pos[(size_t)(3 * e + 2) * W + w], mv);
-#pragma unroll
-      for (int m = 0; m < NOCC; ++m) Sm[i][m] = mv[m];
-    }
-    double ld;
-    const bool oks = oq_invert<NOCC>(Sm, Ai, ld);
-    ok = ok && oks;
-    ld_tot += ld;
-    for (int m = 0; m < NOCC; ++m)
-      for (int j = 0; j < NOCC; ++j)
-        ainv[(size_t)((s * NOCC + m) * NOCC + j) * W + w] = oks ? (Real)Ai[m][j] : (Real)0;
-  }
-  logdet[w] = ok ? ld_tot : -INFINITY;
-  if (!ok) atomicOr(flags, OQ_FLAG_SINGULAR);
-}
 
 // All-electron Metropolis steps, the reference's move (metropolis_move_alle
 // and metropolis_move_1w, OmegaQMC/vmc_gto.py:815-905): every electron is
