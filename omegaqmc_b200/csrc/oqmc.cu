@@ -134,8 +134,8 @@ int oq_ctx_sweep_local_bytes(oqmc_ctx* ctx, int precision, size_t* out) {
   const int mixed = precision == OQ_PREC_MIXED;
   size_t best = 0, v = 0;
   cudaError_t err = cudaSuccess;
-  auto take = [&](int kind, int prop, int M) -> bool {
-#define OQ_X(N) err = oq_local_bytes_##N(kind, mixed, prop, M, &v)
+  auto take = [&](int kind, int M) -> bool {
+#define OQ_X(N) err = oq_local_bytes_##N(kind, mixed, M, &v)
     OQ_SWITCH(ctx->nocc, OQ_X)
 #undef OQ_X
     if (err != cudaSuccess) return false;
@@ -150,20 +150,21 @@ int oq_ctx_sweep_local_bytes(oqmc_ctx* ctx, int precision, size_t* out) {
   };
   bool ok = true;
   if (ctx->md) {
-    ok = take(4, 0, ctx->md->M) && take(5, 0, ctx->md->M) && take(6, 0, ctx->md->M);
+    ok = take(4, ctx->md->M) && take(5, ctx->md->M) && take(6, ctx->md->M);
   } else {
-    ok = take(0, 0, 0);
+    ok = take(0, 0);
+    const bool alle = ctx->move_kind == 1, tc = mixed && ctx->use_tc;
     if (ok) {
-      if (ctx->move_kind == 1) ok = take(7, 0, 0);
+      if (alle) ok = take(7, 0);
       else if (ctx->mlp) ok = take_rtc(ctx->mlp_fn[ctx->mlp_groups == 4 ? 1 : 0]);
-      else if (ctx->spec)
-        ok = take_rtc(oq_spec_function(ctx->spec, (ctx->proposal == 1 ? 4 : 0) + mixed));
-      else ok = take(1, ctx->proposal == 1 ? 1 : 0, 0);
+      else if (ctx->spec) ok = take_rtc(oq_spec_function(ctx->spec, mixed));
+      else ok = take(1, 0);
     }
-    if (ok) {
-      if (mixed && ctx->use_tc) ok = take(3, 0, 0);
+    // the fused sweeps hold the local energy themselves
+    if (ok && (alle || ctx->mlp || tc)) {
+      if (tc) ok = take(3, 0);
       else if (ctx->spec) ok = take_rtc(oq_spec_function(ctx->spec, 2 + mixed));
-      else ok = take(2, 0, 0);
+      else ok = take(2, 0);
     }
   }
   if (!ok)
@@ -475,6 +476,7 @@ extern "C" int oqmc_create(oqmc_ctx** out, const oqmc_system_desc* d) {
     e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_j3, d->j3_gamma, sizeof(double) * n3,
                                         cudaMemcpyHostToDevice) : e;
     S.j3_gamma = ctx->d_j3;
+    ctx->j3_len = (int)n3;
   }
   if (S.has_spl) {
     const size_t nk = (size_t)d->spl_ntab * d->spl_npts;
@@ -654,7 +656,8 @@ int oqmc_set_mlp_proposal(oqmc_ctx* ctx, const oqmc_mlp* m) {
   if (ctx->n_e > 32)
     return set_err(ctx, OQ_ERR_UNSUPPORTED, "the learned proposal handles up to 32 electrons%s");
   if (!ctx->mlp_fn[0]) {
-    const std::string src = std::string("#include \"oqmc_mlp_sweep.cuh\"\n\n") +
+    const std::string src = oq_spec_term_defines({&ctx->hsys}) +
+                            "#include \"oqmc_mlp_sweep.cuh\"\n\n" +
                             oq_spec_basis_source(ctx->hsys, ctx->hsplit, ctx->h_C, ctx->nocc,
                                                  "OqSpecBasis");
     const std::string n = std::to_string(ctx->nocc);
@@ -1056,6 +1059,8 @@ int oqmc_set_split(oqmc_ctx* ctx, double tight_alpha) {
   return OQ_OK;
 }
 
+static size_t real_size(int precision);
+
 static size_t smem_sys_c64(const oqmc_ctx* ctx) {
   return sizeof(OqSystem) + sizeof(double) * ctx->nbf * ctx->nocc;
 }
@@ -1323,22 +1328,69 @@ static int launch_moves(oqmc_ctx* ctx, const OqMoveArgs& m, int wpb, size_t sm, 
       return set_err(ctx, OQ_ERR_CUDA, "learned-proposal move kernel launch failed%s");
     return OQ_OK;
   }
-  if (ctx->spec && m.mode == 0) {
-    OqMoveArgs mm = m;
-    const void* C = mixed ? (const void*)ctx->d_C32 : (const void*)ctx->d_C64;
-    void* args[4] = {(void*)&L.sys, (void*)&L.split, (void*)&C, (void*)&mm};
-    const int which = (m.proposal == 1 ? 4 : 0) + (mixed ? 1 : 0);
-    if (oq_spec_launch(ctx->spec, which, dim3((m.W + wpb - 1) / wpb), dim3(wpb), sm,
-                       L.stream, args) != 0)
-      return set_err(ctx, OQ_ERR_CUDA, "specialised move kernel launch failed%s");
-    return OQ_OK;
-  }
   cudaError_t err = cudaSuccess;
-#define OQ_X(N) err = oq_moves_##N(L, m, wpb, mixed)
+#define OQ_X(N) err = oq_basin_##N(L, m, wpb, mixed)
   OQ_SWITCH(ctx->nocc, OQ_X)
 #undef OQ_X
   OQ_CUDA(ctx, err);
   return OQ_OK;
+}
+
+// Lanes per walker of the fused sweeps: as many as there are electrons (all
+// orbital rows of a sweep at once; 32 with three-body terms in FP64, whose
+// nucleus-electron list fills them), halved while the threads would exceed
+// 512 per SM.  Beyond that the register file (128 per thread) is full and
+// lanes only add shuffles.
+static int sweep_lanes(const oqmc_ctx* ctx, int W, int mixed) {
+  int P = 1;
+  while (P < ctx->n_e && P < 32) P <<= 1;
+  if (!mixed && ctx->hsys.has_j3) P = 32;
+  while (P > 1 && (long long)W * P > 148ll * 512) P >>= 1;
+  return P;
+}
+
+// Launch the fused sweeps `a` describes.  wpb: walkers per CTA asked for by the
+// caller (one lane per walker then), 0 for the library's choice; wpb1 is the
+// CTA size that fits with one lane.
+static int launch_sweeps(oqmc_ctx* ctx, OqSweepArgs a, int wpb, int wpb1, int precision,
+                         void* stream) {
+  const int mixed = precision == OQ_PREC_MIXED;
+  a.lanes = wpb ? 1 : sweep_lanes(ctx, a.W, mixed);
+  int nthr = a.lanes == 1 ? wpb1 : 128;
+  a.j3_cache = !mixed && a.lanes > 1 && ctx->hsys.has_j3;
+  a.j3_len = a.j3_cache && ctx->j3_len <= 2048 ? ctx->j3_len : 0;
+  size_t head = sizeof(OqSystem) + sizeof(OqSplit);
+  head += ((size_t)ctx->nbf * ctx->nocc * real_size(precision) + 15) & ~(size_t)15;
+  auto bytes = [&](int n) {
+    return head + oq_sweep_tile_bytes(ctx->nocc, ctx->natm, n / a.lanes, real_size(precision),
+                                      a.j3_cache, a.j3_len);
+  };
+  while (bytes(nthr) > 227 * 1024 && nthr > 32) nthr >>= 1;
+  const OqLaunch L = make_launch(ctx, stream, bytes(nthr));
+  if (ctx->spec) {
+    const void* C = mixed ? (const void*)ctx->d_C32 : (const void*)ctx->d_C64;
+    void* args[4] = {(void*)&L.sys, (void*)&L.split, (void*)&C, (void*)&a};
+    const int wt = nthr / a.lanes;
+    if (oq_spec_launch(ctx->spec, mixed, dim3((a.W + wt - 1) / wt), dim3(nthr), L.smem, L.stream,
+                       args) != 0)
+      return set_err(ctx, OQ_ERR_CUDA, "specialised sweep kernel launch failed%s");
+    return OQ_OK;
+  }
+  cudaError_t err = cudaSuccess;
+#define OQ_X(N) err = oq_sweeps_##N(L, a, nthr, mixed)
+  OQ_SWITCH(ctx->nocc, OQ_X)
+#undef OQ_X
+  OQ_CUDA(ctx, err);
+  return OQ_OK;
+}
+
+static OqSweepArgs sweep_args(const oqmc_ctx* ctx, double* X, int W, const OqStatePtrs& st) {
+  OqSweepArgs a;
+  memset(&a, 0, sizeof(a));
+  a.X = X; a.pos = st.pos; a.ainv = st.ainv; a.logdet = st.logdet; a.W = W;
+  a.proposal = ctx->proposal; a.scale_r0 = ctx->scale_r0; a.scale_fmin = ctx->scale_fmin;
+  a.flags = ctx->d_flags;
+  return a;
 }
 
 static int md_moves(oqmc_ctx* ctx, const OqMoveArgs& m, double* sgn, void* stream) {
@@ -1426,36 +1478,52 @@ int oqmc_sweeps(oqmc_ctx* ctx, double* X, int W, void* state, int precision, int
     return md_sweeps(ctx, X, W, state, precision, n_sweeps, measure_every, step, seed, step_base,
                      sums, el_trace, eparts_last, stream);
   size_t sm;
+  const int wpb_asked = wpb;
   wpb = pick_wpb(ctx, wpb, precision, &sm);
   if (wpb == -1) return set_err(ctx, OQ_ERR_ARG, "walkers_per_block must be 32, 64 or 128%s");
   if (wpb < 0)
     return set_err(ctx, OQ_ERR_UNSUPPORTED, "system too large for the shared-memory move kernel%s");
   cudaStream_t s = (cudaStream_t)stream;
   const OqStatePtrs st = state_ptrs(ctx, state, W, precision);
+  const int mixed = precision == OQ_PREC_MIXED;
+  const bool tc = mixed && ctx->use_tc;
+  OqSweepArgs sa = sweep_args(ctx, X, W, st);
+  sa.step = step; sa.seed = seed; sa.step_base = step_base;
+  if (ctx->move_kind == 0 && !ctx->mlp && !tc) {
+    sa.n_sweeps = n_sweeps; sa.measure_every = n_sweeps >= measure_every ? measure_every : 0;
+    sa.sums = sums; sa.el_trace = el_trace; sa.eparts_last = eparts_last;
+    return launch_sweeps(ctx, sa, wpb_asked, wpb, precision, stream);
+  }
+  // all-electron steps, the learned proposal, the tensor-core local energy:
+  // moves and local energies in separate launches
+  const bool fused_moves = ctx->move_kind == 0 && !ctx->mlp;
   OQ_CUDA(ctx, to_soa(ctx, X, st.pos, W, s));
   OqMoveArgs m;
   memset(&m, 0, sizeof(m));
   m.pos = st.pos; m.ainv = st.ainv; m.logdet = st.logdet; m.W = W; m.mode = 0;
   m.step = step; m.seed = seed; m.flags = ctx->d_flags;
   m.proposal = ctx->proposal; m.scale_r0 = ctx->scale_r0; m.scale_fmin = ctx->scale_fmin;
+  auto moves = [&](int n, int at, double* acc) -> int {
+    m.n_steps = sa.n_sweeps = n;
+    m.step_base = sa.step_base = step_base + at;
+    m.acc_sum = sa.acc_sum = acc;
+    return fused_moves ? launch_sweeps(ctx, sa, wpb_asked, wpb, precision, stream)
+                       : launch_moves(ctx, m, wpb, sm, precision, stream);
+  };
   OqElocArgs el;
   memset(&el, 0, sizeof(el));
   el.pos = st.pos; el.ainv = st.ainv; el.W = W; el.flags = ctx->d_flags;
   const OqLaunch Le = make_launch(ctx, stream, eloc_smem(ctx, precision));
-  const int mixed = precision == OQ_PREC_MIXED;
   const int n_meas = n_sweeps / measure_every;
   int done = 0;
   for (int k = 0; k < n_meas; ++k) {
-    m.n_steps = measure_every;
-    m.step_base = step_base + done;
-    m.acc_sum = sums + (size_t)k * OQ_NSUM + 5;
-    int rc = launch_moves(ctx, m, wpb, sm, precision, stream);
+    int rc = moves(measure_every, done, sums + (size_t)k * OQ_NSUM + 5);
     if (rc != OQ_OK) return rc;
     done += measure_every;
     el.sums = sums + (size_t)k * OQ_NSUM;
     el.el_trace = el_trace ? el_trace + (size_t)k * W : nullptr;
     el.eparts = (k == n_meas - 1) ? eparts_last : nullptr;
-    if (mixed && ctx->use_tc) {
+    if (tc) {
       cudaError_t err = cudaSuccess;
 #define OQ_X(N) err = oq_eloc_tc_##N(Le, el, ctx->d_Btc, ctx->nbf)
       OQ_SWITCH(ctx->nocc, OQ_X)
@@ -1479,29 +1547,11 @@ int oqmc_sweeps(oqmc_ctx* ctx, double* X, int W, void* state, int precision, int
     OQ_CUDA(ctx, err);
   }
   if (done < n_sweeps) {
-    m.n_steps = n_sweeps - done;
-    m.step_base = step_base + done;
-    m.acc_sum = nullptr;
-    int rc = launch_moves(ctx, m, wpb, sm, precision, stream);
+    int rc = moves(n_sweeps - done, done, nullptr);
     if (rc != OQ_OK) return rc;
   }
   OQ_CUDA(ctx, to_aos(ctx, st.pos, X, W, s));
   return OQ_OK;
-}
-
-// One step of the reference's step-size rule (_adapt_step_size,
-// OmegaQMC/vmc_gto.py:121-126): with the acceptance ratio
-// acc = (*accepted) * inv_moves of the sweep just made,
-// log s <- log s + rate (acc - target).  Records the ratio in place of the
-// count and the new width in step_trace (if set).  One thread.
-__global__ void k_adapt_step(double* __restrict__ step, double* __restrict__ accepted,
-                             double inv_moves, double rate, double target,
-                             double* __restrict__ step_trace) {
-  const double acc = *accepted * inv_moves;
-  const double s = exp(log(*step) + rate * (acc - target));
-  *step = s;
-  *accepted = acc;
-  if (step_trace) *step_trace = s;
 }
 
 int oqmc_equilibrate(oqmc_ctx* ctx, double* X, int W, void* state, int precision,
@@ -1523,26 +1573,26 @@ int oqmc_equilibrate(oqmc_ctx* ctx, double* X, int W, void* state, int precision
     return set_err(ctx, OQ_ERR_UNSUPPORTED, "system too large for the shared-memory move kernel%s");
   cudaStream_t s = (cudaStream_t)stream;
   const OqStatePtrs st = state_ptrs(ctx, state, W, precision);
-  OQ_CUDA(ctx, to_soa(ctx, X, st.pos, W, s));
   OQ_CUDA(ctx, cudaMemsetAsync(acc_trace, 0, sizeof(double) * (size_t)n_steps, s));
-  OqMoveArgs m;
-  memset(&m, 0, sizeof(m));
-  m.pos = st.pos; m.ainv = st.ainv; m.logdet = st.logdet; m.W = W; m.mode = 0;
-  m.n_steps = 1; m.step = 0.0; m.step_dev = step; m.seed = seed; m.flags = ctx->d_flags;
-  m.proposal = ctx->proposal; m.scale_r0 = ctx->scale_r0; m.scale_fmin = ctx->scale_fmin;
-  const OqLaunch Lr = make_launch(ctx, stream, smem_sys_c64(ctx));
+  OqSweepArgs a = sweep_args(ctx, X, W, st);
+  a.n_sweeps = 1; a.seed = seed; a.step_dev = step; a.rate = rate; a.target = target;
+  a.inv_moves = 1.0 / ((double)W * ctx->n_e);
+  a.tick = 1.0;
+  while (a.tick <= (double)W * ctx->n_e) a.tick *= 2.0;
+  const OqLaunch Lr = make_launch(ctx, stream, 0);
   const int mixed = precision == OQ_PREC_MIXED;
-  const double inv_moves = 1.0 / ((double)W * ctx->n_e);
   int since = since_refresh;
   for (int t = 0; t < n_steps; ++t) {
-    m.step_base = step_base + t;
-    m.acc_sum = acc_trace + t;
-    int rc = launch_moves(ctx, m, wpb, sm, precision, stream);
+    const bool refresh = since + 1 >= refresh_every;
+    a.step_base = step_base + t;
+    a.acc_sum = acc_trace + t;
+    a.step_trace = step_trace ? step_trace + t : nullptr;
+    // the state's own positions are read by the refresh and after the call
+    a.pos = refresh || t == n_steps - 1 ? st.pos : nullptr;
+    int rc = launch_sweeps(ctx, a, 0, wpb, precision, stream);
     if (rc != OQ_OK) return rc;
-    k_adapt_step<<<1, 1, 0, s>>>(step, acc_trace + t, inv_moves, rate, target,
-                                 step_trace ? step_trace + t : nullptr);
-    OQ_CUDA(ctx, cudaGetLastError());
-    if (++since >= refresh_every) {
+    ++since;
+    if (refresh) {
       cudaError_t err = cudaSuccess;
 #define OQ_X(N) err = oq_refresh_##N(Lr, st.pos, W, st.ainv, st.logdet, mixed)
       OQ_SWITCH(ctx->nocc, OQ_X)
@@ -1551,7 +1601,6 @@ int oqmc_equilibrate(oqmc_ctx* ctx, double* X, int W, void* state, int precision
       since = 0;
     }
   }
-  OQ_CUDA(ctx, to_aos(ctx, st.pos, X, W, s));
   return OQ_OK;
 }
 

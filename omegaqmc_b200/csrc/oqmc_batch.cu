@@ -64,7 +64,7 @@ std::string batch_source(const std::vector<const OqSystem*>& S,
                          const std::vector<const OqSplit*>& SP,
                          const std::vector<const double*>& C, const std::vector<int>& nocc,
                          const std::vector<int>& modes = {}) {
-  std::string src = "#include \"oqmc_batch.cuh\"\n\n";
+  std::string src = oq_spec_term_defines(S) + "#include \"oqmc_batch.cuh\"\n\n";
   for (size_t k = 0; k < S.size(); ++k)
     src += oq_spec_basis_source(*S[k], *SP[k], C[k], nocc[k], "OqSpecBasis_" + std::to_string(k)) +
            "\n" + jas_source(*S[k], "oq_jas_" + std::to_string(k)) + "\n";

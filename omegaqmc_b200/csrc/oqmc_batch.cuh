@@ -157,7 +157,7 @@ __device__ __forceinline__ T oq_jastrow_delta_lane(const SJ& J, const OqSystem& 
       dJ += oq_pade_diff((T)J.j2[o], (T)J.j2[o + 1], rn2t * oq_rsqrt(rn2t),
                          ro2t * oq_rsqrt(ro2t));
     }
-    if (S.has_bs2) {
+    if (OQ_HAS_BS2(S)) {
       const double* c = like ? S.bs2_like : S.bs2_unlike;
       const int n = like ? S.bs2_n_like : S.bs2_n_unlike;
       const T dinv = (T)(like ? S.bs2_dinv_like : S.bs2_dinv_unlike), rc = (T)S.bs2_rcut;
@@ -173,14 +173,14 @@ __device__ __forceinline__ T oq_jastrow_delta_lane(const SJ& J, const OqSystem& 
     const T rn2t = (T)rn2, ro2t = (T)(bx * bx + by * by + bz * bz);
     if (J.has_j1)
       dJ += oq_pade_diff((T)J.j1a[I], (T)J.j1b[I], rn2t * oq_rsqrt(rn2t), ro2t * oq_rsqrt(ro2t));
-    if (S.has_bs1 && S.bs1_type[I] >= 0) {
+    if (OQ_HAS_BS1(S) && S.bs1_type[I] >= 0) {
       const int ty = S.bs1_type[I];
       const T dinv = (T)S.bs1_dinv[ty], rc = (T)S.bs1_rcut[ty];
       dJ += oq_bs_val<T>(S.bs1_c[ty], S.bs1_n[ty], dinv, rc, rn2t * oq_rsqrt(rn2t)) -
             oq_bs_val<T>(S.bs1_c[ty], S.bs1_n[ty], dinv, rc, ro2t * oq_rsqrt(ro2t));
     }
   }
-  if (S.has_j3 && lane == 0)
+  if (OQ_HAS_J3(S) && lane == 0)
     dJ -= oq_j3_electron<T>(S, pos, (size_t)ps, NE, e, 0, nx, ny, nz) -
           oq_j3_electron<T>(S, pos, (size_t)ps, NE, e, 0, ox, oy, oz);
   return dJ;

@@ -82,6 +82,19 @@ struct OqSystem {
   OqHarmTable harm;
 };
 
+// Optional Jastrow terms.  A module generated for given molecules defines
+// OQ_GEN_* as 0 where none of them has the term, which compiles its code, and
+// the registers it takes, out of the kernels.
+#ifdef OQ_GEN_J3
+#define OQ_HAS_J3(S) (OQ_GEN_J3 && (S).has_j3)
+#define OQ_HAS_BS1(S) (OQ_GEN_BS1 && (S).has_bs1)
+#define OQ_HAS_BS2(S) (OQ_GEN_BS2 && (S).has_bs2)
+#else
+#define OQ_HAS_J3(S) ((S).has_j3)
+#define OQ_HAS_BS1(S) ((S).has_bs1)
+#define OQ_HAS_BS2(S) ((S).has_bs2)
+#endif
+
 // Status codes shared by host and device.
 enum OqStatus {
   OQ_OK = 0,
@@ -376,6 +389,28 @@ __device__ __forceinline__ void oq_j3_partials(const double* __restrict__ g, int
   u11 = P11 * E + (T)2 * P1 * E1 + P * E11;
   uee = R * E;
   u1e = Q1 * E + Q * E1;
+}
+
+// The same with the orders known to the compiler for the two usual ones (2, 2
+// and 3, 3): the loops unroll and the table loads no longer wait in line.
+template <typename T>
+__device__ __forceinline__ T oq_j3_u_n(const double* __restrict__ g, int nI, int nE, T L, T r12,
+                                       T r1, T r2) {
+  if (nI == 2 && nE == 2) return oq_j3_u<T>(g, 2, 2, L, r12, r1, r2);
+  if (nI == 3 && nE == 3) return oq_j3_u<T>(g, 3, 3, L, r12, r1, r2);
+  return oq_j3_u<T>(g, nI, nE, L, r12, r1, r2);
+}
+template <typename T>
+__device__ __forceinline__ void oq_j3_partials_n(const double* __restrict__ g, int nI, int nE,
+                                                 T L, T r12, T r1, T r2, T& u1, T& ue, T& u11,
+                                                 T& uee, T& u1e) {
+  if (nI == 2 && nE == 2) {
+    oq_j3_partials<T>(g, 2, 2, L, r12, r1, r2, u1, ue, u11, uee, u1e);
+  } else if (nI == 3 && nE == 3) {
+    oq_j3_partials<T>(g, 3, 3, L, r12, r1, r2, u1, ue, u11, uee, u1e);
+  } else {
+    oq_j3_partials<T>(g, nI, nE, L, r12, r1, r2, u1, ue, u11, uee, u1e);
+  }
 }
 
 // Sum of u over the triplets of electron e at (x, y, z) with the electrons

@@ -30,6 +30,7 @@ struct oqmc_ctx {
   int ao_bytes, ao_ext;    // ao_ext: OqAoHead::ext
   unsigned* d_flags;
   double* d_j3;            // three-body Jastrow gamma blocks (or null)
+  int j3_len;              // their length in doubles
   double* d_spl_knots;     // radial spline tables (or null)
   double* d_spl_coef;
   double tight_alpha;

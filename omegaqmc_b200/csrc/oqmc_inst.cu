@@ -77,26 +77,35 @@ cudaError_t OQ_FN(oq_refresh)(const OqLaunch& L, const double* pos, int W, void*
   return mixed ? team<OQ_TEAM_REFRESH, float>(L, a) : team<OQ_TEAM_REFRESH, double>(L, a);
 }
 
-template <int PROP>
-static cudaError_t moves_prop(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed) {
+// basin relocations
+cudaError_t OQ_FN(oq_basin)(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed) {
   const int nb = (a.W + wpb - 1) / wpb;
   cudaError_t e;
   if (mixed) {
-    e = oq_smem_attr(k_moves<OQ_N, float, float, PROP>, L.smem);
+    e = oq_smem_attr(k_moves<OQ_N, float, float, 2>, L.smem);
     if (e != cudaSuccess) return e;
-    k_moves<OQ_N, float, float, PROP><<<nb, wpb, L.smem, L.stream>>>(L.sys, L.split, L.C32, a);
+    k_moves<OQ_N, float, float, 2><<<nb, wpb, L.smem, L.stream>>>(L.sys, L.split, L.C32, a);
   } else {
-    e = oq_smem_attr(k_moves<OQ_N, double, double, PROP>, L.smem);
+    e = oq_smem_attr(k_moves<OQ_N, double, double, 2>, L.smem);
     if (e != cudaSuccess) return e;
-    k_moves<OQ_N, double, double, PROP><<<nb, wpb, L.smem, L.stream>>>(L.sys, L.split, L.C64, a);
+    k_moves<OQ_N, double, double, 2><<<nb, wpb, L.smem, L.stream>>>(L.sys, L.split, L.C64, a);
   }
   return cudaGetLastError();
 }
 
-cudaError_t OQ_FN(oq_moves)(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed) {
-  if (a.mode == 1) return moves_prop<2>(L, a, wpb, mixed);
-  if (a.proposal == 1) return moves_prop<1>(L, a, wpb, mixed);
-  return moves_prop<0>(L, a, wpb, mixed);
+cudaError_t OQ_FN(oq_sweeps)(const OqLaunch& L, const OqSweepArgs& a, int nthr, int mixed) {
+  const int wt = nthr / a.lanes, nb = (a.W + wt - 1) / wt;
+  cudaError_t e;
+  if (mixed) {
+    e = oq_smem_attr(k_sweeps<OQ_N, float, float>, L.smem);
+    if (e != cudaSuccess) return e;
+    k_sweeps<OQ_N, float, float><<<nb, nthr, L.smem, L.stream>>>(L.sys, L.split, L.C32, a);
+  } else {
+    e = oq_smem_attr(k_sweeps<OQ_N, double, double>, L.smem);
+    if (e != cudaSuccess) return e;
+    k_sweeps<OQ_N, double, double><<<nb, nthr, L.smem, L.stream>>>(L.sys, L.split, L.C64, a);
+  }
+  return cudaGetLastError();
 }
 
 cudaError_t OQ_FN(oq_eloc)(const OqLaunch& L, const OqElocArgs& a, int mixed) {
@@ -199,7 +208,7 @@ cudaError_t OQ_FN(oq_moves_alle)(const OqLaunch& L, const OqMoveArgs& a, int mix
 }
 
 // Per-thread local memory (bytes) of one kernel this size launches: kind 0
-// k_team (refresh), 1 k_moves (prop 0/1/2), 2 k_eloc, 3 k_eloc_tc, 4 k_md_refresh,
+// k_team (refresh), 1 k_sweeps, 2 k_eloc, 3 k_eloc_tc, 4 k_md_refresh,
 // 5 k_md_moves, 6 k_md_local (M = 8 or 16 columns), 7 k_moves_alle.
 template <typename K>
 static cudaError_t oq_lmem(K kernel, size_t* out) {
@@ -216,20 +225,14 @@ static cudaError_t md_lmem(int kind, size_t* out) {
   return oq_lmem(k_md_local<OQ_N, M>, out);
 }
 
-cudaError_t OQ_FN(oq_local_bytes)(int kind, int mixed, int prop, int M, size_t* out) {
+cudaError_t OQ_FN(oq_local_bytes)(int kind, int mixed, int M, size_t* out) {
   switch (kind) {
     case 0:
       return mixed ? oq_lmem(k_team<OQ_N, OQ_TEAM_REFRESH, float, true>, out)
                    : oq_lmem(k_team<OQ_N, OQ_TEAM_REFRESH, double, true>, out);
     case 1:
-      if (prop == 2)
-        return mixed ? oq_lmem(k_moves<OQ_N, float, float, 2>, out)
-                     : oq_lmem(k_moves<OQ_N, double, double, 2>, out);
-      if (prop == 1)
-        return mixed ? oq_lmem(k_moves<OQ_N, float, float, 1>, out)
-                     : oq_lmem(k_moves<OQ_N, double, double, 1>, out);
-      return mixed ? oq_lmem(k_moves<OQ_N, float, float, 0>, out)
-                   : oq_lmem(k_moves<OQ_N, double, double, 0>, out);
+      return mixed ? oq_lmem(k_sweeps<OQ_N, float, float>, out)
+                   : oq_lmem(k_sweeps<OQ_N, double, double>, out);
     case 2:
       return mixed ? oq_lmem(k_eloc<OQ_N, float, float>, out)
                    : oq_lmem(k_eloc<OQ_N, double, double>, out);

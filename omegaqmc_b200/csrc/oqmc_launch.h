@@ -26,7 +26,8 @@ struct OqLaunch {
   cudaError_t oq_movals_##N(const OqLaunch& L, const double* X, int W, double* out);  \
   cudaError_t oq_refresh_##N(const OqLaunch& L, const double* pos, int W, void* ainv, \
                              double* logdet, int mixed);                              \
-  cudaError_t oq_moves_##N(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed); \
+  cudaError_t oq_basin_##N(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed); \
+  cudaError_t oq_sweeps_##N(const OqLaunch& L, const OqSweepArgs& a, int nthr, int mixed); \
   cudaError_t oq_moves_alle_##N(const OqLaunch& L, const OqMoveArgs& a, int mixed);     \
   cudaError_t oq_eloc_##N(const OqLaunch& L, const OqElocArgs& a, int mixed);           \
   cudaError_t oq_eloc_tc_##N(const OqLaunch& L, const OqElocArgs& a, const void* Bpack, \
@@ -38,7 +39,7 @@ struct OqLaunch {
   cudaError_t oq_md_local_##N(const OqLaunch& L, const OqMdTables& T,                  \
                               const OqMdState& st, const OqElocArgs& a, double* logpsi, \
                               double* grad, double* lap, int M);                \
-  cudaError_t oq_local_bytes_##N(int kind, int mixed, int prop, int M, size_t* out);
+  cudaError_t oq_local_bytes_##N(int kind, int mixed, int M, size_t* out);
 
 #define OQ_NOCC_LIST(X) X(1) X(2) X(3) X(4) X(5) X(6) X(7) X(8) X(10) X(12) X(14) X(16)
 

@@ -455,8 +455,23 @@ std::string generate_basis(const OqSystem& S, const OqSplit& SP, const double* C
   return src;
 }
 
+}  // namespace
+
+std::string oq_spec_term_defines(const std::vector<const OqSystem*>& S) {
+  bool j3 = false, b1 = false, b2 = false;
+  for (const OqSystem* s : S) {
+    j3 = j3 || s->has_j3;
+    b1 = b1 || s->has_bs1;
+    b2 = b2 || s->has_bs2;
+  }
+  return std::string("#define OQ_GEN_J3 ") + (j3 ? "1" : "0") + "\n#define OQ_GEN_BS1 " +
+         (b1 ? "1" : "0") + "\n#define OQ_GEN_BS2 " + (b2 ? "1" : "0") + "\n";
+}
+
+namespace {
+
 std::string generate(const OqSystem& S, const OqSplit& SP, const double* C, int nocc) {
-  return "#include \"oqmc_sweep.cuh\"\n\n" + generate_basis(S, SP, C, nocc, "OqSpecBasis");
+  return oq_spec_term_defines({&S}) + "#include \"oqmc_sweep.cuh\"\n\n" + generate_basis(S, SP, C, nocc, "OqSpecBasis");
 }
 
 }  // namespace
@@ -594,19 +609,16 @@ int oq_rtc_local_bytes(void* fn) {
 
 struct OqSpecModule {
   CUmodule mod = nullptr;
-  // moves fixed-width d/f, eloc d/f, moves nucleus-scaled d/f
-  CUfunction fn[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+  CUfunction fn[4] = {nullptr, nullptr, nullptr, nullptr};   // fused sweeps d/f, local energy d/f
 };
 
 int oq_spec_build(const OqSystem& S, const OqSplit& SP, const double* C, int nocc,
                   OqSpecModule** out, std::string* err) {
   std::vector<std::string> names;
-  const char* forms[6] = {"k_moves<%d, double, double, 0, OqSpecBasis>",
-                          "k_moves<%d, float, float, 0, OqSpecBasis>",
+  const char* forms[4] = {"k_sweeps<%d, double, double, OqSpecBasis>",
+                          "k_sweeps<%d, float, float, OqSpecBasis>",
                           "k_eloc<%d, double, double, OqSpecBasis>",
-                          "k_eloc<%d, float, float, OqSpecBasis>",
-                          "k_moves<%d, double, double, 1, OqSpecBasis>",
-                          "k_moves<%d, float, float, 1, OqSpecBasis>"};
+                          "k_eloc<%d, float, float, OqSpecBasis>"};
   for (const char* f : forms) {
     char b[128];
     snprintf(b, sizeof b, f, nocc);
@@ -617,7 +629,7 @@ int oq_spec_build(const OqSystem& S, const OqSplit& SP, const double* C, int noc
   if (oq_rtc_build(generate(S, SP, C, nocc), names, &mod, &fns, err) != 0) return -1;
   OqSpecModule* m = new OqSpecModule();
   m->mod = (CUmodule)mod;
-  for (int i = 0; i < 6; ++i) m->fn[i] = (CUfunction)fns[i];
+  for (int i = 0; i < 4; ++i) m->fn[i] = (CUfunction)fns[i];
   *out = m;
   return 0;
 }
@@ -629,7 +641,7 @@ void oq_spec_destroy(OqSpecModule* m) {
 }
 
 void* oq_spec_function(OqSpecModule* m, int which) {
-  return (m && which >= 0 && which < 6) ? (void*)m->fn[which] : nullptr;
+  return (m && which >= 0 && which < 4) ? (void*)m->fn[which] : nullptr;
 }
 
 int oq_spec_launch(OqSpecModule* m, int which, dim3 grid, dim3 block, size_t smem,

@@ -12,13 +12,16 @@ struct OqSpecModule;
 int oq_spec_build(const OqSystem& S, const OqSplit& SP, const double* C, int nocc,
                   OqSpecModule** out, std::string* err);
 void oq_spec_destroy(OqSpecModule* m);
-// which: 0/1 = fixed-width moves FP64/mixed, 2/3 = local energy FP64/mixed,
-// 4/5 = nucleus-scaled moves FP64/mixed
+// which: 0/1 = fused sweeps FP64/mixed, 2/3 = local energy FP64/mixed
 int oq_spec_launch(OqSpecModule* m, int which, dim3 grid, dim3 block, size_t smem,
                    cudaStream_t stream, void** args);
 // The CUfunction behind `which` (numbering as for oq_spec_launch).
 void* oq_spec_function(OqSpecModule* m, int which);
 std::string oq_spec_source(const OqSystem& S, const OqSplit& SP, const double* C, int nocc);
+
+// Which optional Jastrow terms any of the systems has, as #define lines for the
+// top of a generated source (oqmc_common.cuh, OQ_HAS_J3 ...).
+std::string oq_spec_term_defines(const std::vector<const OqSystem*>& S);
 
 // The basis policy of one system as C++ source for a struct named `name`.
 std::string oq_spec_basis_source(const OqSystem& S, const OqSplit& SP, const double* C, int nocc,

@@ -520,7 +520,7 @@ __device__ __forceinline__ T oq_jastrow_delta(const SJ& J, const OqSystem& S, co
       const T pa = (T)J.j2[o], pb = (T)J.j2[o + 1];
       dJ += oq_pade_diff(pa, pb, rn2t * oq_rsqrt(rn2t), ro2t * oq_rsqrt(ro2t));
     }
-    if (S.has_bs2) {
+    if (OQ_HAS_BS2(S)) {
       const double bx = ox - xj, by = oy - yj, bz = oz - zj;
       const T rn2t = (T)rn2, ro2t = (T)(bx * bx + by * by + bz * bz);
       const bool like = (e & 1) == (j & 1);
@@ -541,7 +541,7 @@ __device__ __forceinline__ T oq_jastrow_delta(const SJ& J, const OqSystem& S, co
       const T pa = (T)J.j1a[I], pb = (T)J.j1b[I];
       dJ += oq_pade_diff(pa, pb, rn2t * oq_rsqrt(rn2t), ro2t * oq_rsqrt(ro2t));
     }
-    if (S.has_bs1 && S.bs1_type[I] >= 0) {
+    if (OQ_HAS_BS1(S) && S.bs1_type[I] >= 0) {
       const int ty = S.bs1_type[I];
       const double bx = ox - J.nuc[I][0], by = oy - J.nuc[I][1], bz = oz - J.nuc[I][2];
       const T rn2t = (T)rn2, ro2t = (T)(bx * bx + by * by + bz * bz);
@@ -550,7 +550,7 @@ __device__ __forceinline__ T oq_jastrow_delta(const SJ& J, const OqSystem& S, co
             oq_bs_val<T>(S.bs1_c[ty], S.bs1_n[ty], dinv, rc, ro2t * oq_rsqrt(ro2t));
     }
   }
-  if (S.has_j3)
+  if (OQ_HAS_J3(S))
     dJ -= oq_j3_electron<T>(S, pos, (size_t)ps, NE, e, 0, nx, ny, nz) -
           oq_j3_electron<T>(S, pos, (size_t)ps, NE, e, 0, ox, oy, oz);
   return dJ;
@@ -667,8 +667,9 @@ __device__ __forceinline__ int oq_basin_propose(const OqSystem& S, const double*
   return e;
 }
 
-// Metropolis moves, one thread per walker, state resident in shared memory
-// for the whole launch.  PROP (compile time) selects the proposal: 0 fixed-
+// Metropolis moves alone, one thread per walker, state resident in shared
+// memory for the whole launch; the library launches it for basin relocations
+// (sweeps run in k_sweeps).  PROP (compile time) selects the proposal: 0 fixed-
 // width Gaussian, 1 nucleus-scaled Gaussian, 2 basin relocation.  mode 0: n_steps sweeps over all electrons with
 // Gaussian proposals (metropolis_move_1w, OmegaQMC/vmc_gto.py:841-905, as
 // single-electron moves).  mode 1: n_steps basin relocations: one random
@@ -774,7 +775,7 @@ __device__ __forceinline__ void oq_jastrow_vgl_coulomb(const SJ& J, const OqSyst
                                                        const double* pos, size_t ps, int e,
                                                        double xe, double ye, double ze, T& jx,
                                                        T& jy, T& jz, T& jl, double& ee,
-                                                       double& en) {
+                                                       double& en, bool j3 = true) {
   // The gradient sums run in FP64 on the FP64 displacements: in the mixed
   // build that converts one value per pair (u'(r)/r) to FP64 instead of
   // three displacement components to FP32.  The working-precision Coulomb
@@ -804,7 +805,7 @@ __device__ __forceinline__ void oq_jastrow_vgl_coulomb(const SJ& J, const OqSyst
       const double u = (double)upr;
       gx += u * dx; gy += u * dy; gz += u * dz; jl += l;
     }
-    if (S.has_bs2) {
+    if (OQ_HAS_BS2(S)) {
       const bool like = (e & 1) == (j & 1);
       T upr, l;
       oq_bs_vgl<T>(like ? S.bs2_like : S.bs2_unlike, like ? S.bs2_n_like : S.bs2_n_unlike,
@@ -828,7 +829,7 @@ __device__ __forceinline__ void oq_jastrow_vgl_coulomb(const SJ& J, const OqSyst
       const double u = (double)upr;
       gx += u * dx; gy += u * dy; gz += u * dz; jl += l;
     }
-    if (S.has_bs1 && S.bs1_type[I] >= 0) {
+    if (OQ_HAS_BS1(S) && S.bs1_type[I] >= 0) {
       const int ty = S.bs1_type[I];
       T upr, l;
       oq_bs_vgl<T>(S.bs1_c[ty], S.bs1_n[ty], (T)S.bs1_dinv[ty], (T)S.bs1_rcut[ty], r2t * rinv,
@@ -842,7 +843,7 @@ __device__ __forceinline__ void oq_jastrow_vgl_coulomb(const SJ& J, const OqSyst
     en += (double)ent;
   }
   jx += (T)gx; jy += (T)gy; jz += (T)gz;
-  if (S.has_j3) oq_j3_vgl_electron<T>(S, pos, ps, NE, e, xe, ye, ze, jx, jy, jz, jl);
+  if (j3 && OQ_HAS_J3(S)) oq_j3_vgl_electron<T>(S, pos, ps, NE, e, xe, ye, ze, jx, jy, jz, jl);
 }
 
 // Local-energy contributions of electron e of one walker: its Coulomb terms
@@ -913,7 +914,7 @@ __device__ __forceinline__ double oq_jastrow_value_electron(const OqSystem& S, c
       const int o = like ? 0 : 2;
       J += (double)oq_pade<T>((T)S.j2[o], (T)S.j2[o + 1], r);
     }
-    if (S.has_bs2)
+    if (OQ_HAS_BS2(S))
       J += (double)oq_bs_val<T>(like ? S.bs2_like : S.bs2_unlike,
                                 like ? S.bs2_n_like : S.bs2_n_unlike,
                                 (T)(like ? S.bs2_dinv_like : S.bs2_dinv_unlike),
@@ -923,13 +924,13 @@ __device__ __forceinline__ double oq_jastrow_value_electron(const OqSystem& S, c
     const double dx = xe - S.nuc[I][0], dy = ye - S.nuc[I][1], dz = ze - S.nuc[I][2];
     const T r = sqrt((T)(dx * dx + dy * dy + dz * dz));
     if (S.has_j1) J += (double)oq_pade<T>((T)S.j1a[I], (T)S.j1b[I], r);
-    if (S.has_bs1 && S.bs1_type[I] >= 0) {
+    if (OQ_HAS_BS1(S) && S.bs1_type[I] >= 0) {
       const int ty = S.bs1_type[I];
       J += (double)oq_bs_val<T>(S.bs1_c[ty], S.bs1_n[ty], (T)S.bs1_dinv[ty],
                                 (T)S.bs1_rcut[ty], r);
     }
   }
-  if (S.has_j3) J -= (double)oq_j3_electron<T>(S, pos, ps, NE, e, e + 1, xe, ye, ze);
+  if (OQ_HAS_J3(S)) J -= (double)oq_j3_electron<T>(S, pos, ps, NE, e, e + 1, xe, ye, ze);
   return J;
 }
 
@@ -1040,5 +1041,512 @@ k_eloc(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
 #pragma unroll
     for (int k = 0; k < 5; ++k) atomicAdd(a.sums + k, vals[k]);
     atomicAdd(a.sums + 6, vals[5]);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Fused sweeps: moves and local energies of n_sweeps sweeps in one launch, with
+// P lanes (threads of one warp) per walker, P a power of two chosen from the
+// walker count (oq_sweep_lanes).
+//
+// Why.  Separate move and local-energy launches per sweep with one thread per
+// walker leave most of the chip idle below some ten thousand walkers: 1,000
+// H2O walkers are 8 CTAs, each thread a serial chain of 10 orbital rows, 90
+// pair terms and 10 updates per sweep, and every launch copies the tables and
+// the state again.  The proposal of an electron and its orbital row depend on
+// that electron alone, so the lanes of a walker form the rows of P electrons
+// at once; the moves are then decided in order, every lane taking part (pair
+// terms and columns of the update split over the lanes), and in the local
+// energy each lane takes electrons of its own.
+//
+// In FP32 the Jastrow change is summed over all pairs on every lane, in the
+// order of the one-lane form: a different order of summation would round
+// differently and flip a decision in some 10^7.  In FP64 the pairs are split
+// and added by shuffles (the rounding is below any decision's resolution).
+// ---------------------------------------------------------------------------
+struct OqSweepArgs {
+  double* X;               // walkers (W, n_e, 3), updated in place
+  double* pos;             // the state's positions (SoA), written at the end (may be null)
+  void* ainv;
+  double* logdet;
+  int W;
+  int n_sweeps;
+  int measure_every;       // 0: no local energies
+  int proposal;            // 0 fixed width, 1 nucleus-scaled width
+  int lanes;               // P
+  int j3_cache;            // three-body terms on several lanes: distances kept per walker
+  int j3_len;              // doubles of the gamma table to copy to shared memory (0: none)
+  int pad;
+  double step, scale_r0, scale_fmin;
+  uint64_t seed, step_base;
+  double* sums;            // [n_meas][OQ_NSUM] or null
+  double* el_trace;        // [n_meas][W] or null
+  double* eparts_last;     // (W, 4) of the last measurement, or null
+  unsigned* flags;
+  double* acc_sum;         // += accepted moves outside measurements (may be null)
+  // Equilibration (one sweep per launch): the width is read from step_dev and
+  // the last CTA adapts it, see below.
+  double* step_dev;
+  double* step_trace;
+  double tick, inv_moves, rate, target;
+};
+
+// Bytes of a tile of wt walkers after the system tables, split radii and
+// coefficients: positions, inverses and, for three-body terms on several
+// lanes, the nucleus-electron distances and the gamma table.
+inline size_t oq_sweep_tile_bytes(int nocc, int natm, int wt, size_t real, int j3_cache,
+                                  int j3_len) {
+  return (size_t)6 * nocc * wt * 8 + (((size_t)2 * nocc * nocc * wt * real + 15) & ~(size_t)15) +
+         (j3_cache ? (size_t)2 * nocc * natm * wt * 8 + (size_t)j3_len * 8 : 0);
+}
+
+// This lane's share of the change of J3 when electron e moves to n (terms
+// t = lane, lane + P, ... of the nucleus-electron list).  rI holds the
+// walker's nucleus-electron distances [I][j], stride rs.
+template <int NE, typename T>
+__device__ __forceinline__ T oq_j3_delta_lane(const OqSystem& S, const double* pos, int ps,
+                                              const double* rI, int rs, int e, int lane, int P,
+                                              double ox, double oy, double oz, double nx,
+                                              double ny, double nz) {
+  const int nI = S.j3_nI, nE = S.j3_nE, bsz = (nI + 1) * (nI + 1) * (nE + 1);
+  const T L = (T)S.j3_L;
+  T acc = (T)0;
+  for (int t = lane; t < S.natm * NE; t += P) {
+    const int I = t / NE, j = t - I * NE, ty = S.j3_type[I], blk = (e ^ j) & 1;
+    if (j == e || ty < 0 || !S.j3_on[ty][blk]) continue;
+    const T r2 = (T)rI[t * rs];
+    if (!(r2 < L)) continue;
+    const T r1o = (T)rI[(I * NE + e) * rs];
+    const double ax = nx - S.nuc[I][0], ay = ny - S.nuc[I][1], az = nz - S.nuc[I][2];
+    const T r1n = sqrt((T)(ax * ax + ay * ay + az * az));
+    const double* g = S.j3_gamma + (size_t)(2 * ty + blk) * bsz;
+    const double xj = pos[(3 * j) * ps], yj = pos[(3 * j + 1) * ps], zj = pos[(3 * j + 2) * ps];
+    if (r1n < L) {
+      const double dx = nx - xj, dy = ny - yj, dz = nz - zj;
+      acc += oq_j3_u_n<T>(g, nI, nE, L, sqrt((T)(dx * dx + dy * dy + dz * dz)), r1n, r2);
+    }
+    if (r1o < L) {
+      const double dx = ox - xj, dy = oy - yj, dz = oz - zj;
+      acc -= oq_j3_u_n<T>(g, nI, nE, L, sqrt((T)(dx * dx + dy * dy + dz * dz)), r1o, r2);
+    }
+  }
+  return -acc;
+}
+
+// This lane's share of the Padé and B-spline change (pairs j and nuclei I
+// congruent to lane modulo P; the terms of oq_jastrow_delta) and of the
+// MIN_DIST_THRESHOLD test.
+template <int NE, typename T>
+__device__ __forceinline__ T oq_jastrow_part(const OqSystem& S, const double* pos, int ps, int e,
+                                             int lane, int P, double ox, double oy, double oz,
+                                             double nx, double ny, double nz, bool& valid) {
+  const double thr2 = 1e-4 * 1e-4;
+  T dJ = (T)0;
+  valid = true;
+  for (int j = lane; j < NE; j += P) {
+    if (j == e) continue;
+    const double xj = pos[(3 * j) * ps], yj = pos[(3 * j + 1) * ps], zj = pos[(3 * j + 2) * ps];
+    const double ax = nx - xj, ay = ny - yj, az = nz - zj;
+    const double bx = ox - xj, by = oy - yj, bz = oz - zj;
+    const double rn2 = ax * ax + ay * ay + az * az;
+    valid = valid && (rn2 >= thr2);
+    const T rn2t = (T)rn2, ro2t = (T)(bx * bx + by * by + bz * bz);
+    const bool like = (e & 1) == (j & 1);
+    if (S.has_j2) {
+      const int o = like ? 0 : 2;
+      dJ += oq_pade_diff((T)S.j2[o], (T)S.j2[o + 1], rn2t * oq_rsqrt(rn2t),
+                         ro2t * oq_rsqrt(ro2t));
+    }
+    if (OQ_HAS_BS2(S)) {
+      const double* c = like ? S.bs2_like : S.bs2_unlike;
+      const int n = like ? S.bs2_n_like : S.bs2_n_unlike;
+      const T dinv = (T)(like ? S.bs2_dinv_like : S.bs2_dinv_unlike), rc = (T)S.bs2_rcut;
+      dJ += oq_bs_val<T>(c, n, dinv, rc, rn2t * oq_rsqrt(rn2t)) -
+            oq_bs_val<T>(c, n, dinv, rc, ro2t * oq_rsqrt(ro2t));
+    }
+  }
+  // the nuclei go to the lanes that the pairs load least
+  for (int I = P - 1 - lane; I < S.natm; I += P) {
+    const double ax = nx - S.nuc[I][0], ay = ny - S.nuc[I][1], az = nz - S.nuc[I][2];
+    const double rn2 = ax * ax + ay * ay + az * az;
+    valid = valid && (rn2 >= thr2);
+    const double bx = ox - S.nuc[I][0], by = oy - S.nuc[I][1], bz = oz - S.nuc[I][2];
+    const T rn2t = (T)rn2, ro2t = (T)(bx * bx + by * by + bz * bz);
+    if (S.has_j1)
+      dJ += oq_pade_diff((T)S.j1a[I], (T)S.j1b[I], rn2t * oq_rsqrt(rn2t), ro2t * oq_rsqrt(ro2t));
+    if (OQ_HAS_BS1(S) && S.bs1_type[I] >= 0) {
+      const int ty = S.bs1_type[I];
+      const T dinv = (T)S.bs1_dinv[ty], rc = (T)S.bs1_rcut[ty];
+      dJ += oq_bs_val<T>(S.bs1_c[ty], S.bs1_n[ty], dinv, rc, rn2t * oq_rsqrt(rn2t)) -
+            oq_bs_val<T>(S.bs1_c[ty], S.bs1_n[ty], dinv, rc, ro2t * oq_rsqrt(ro2t));
+    }
+  }
+  return dJ;
+}
+
+template <typename V>
+__device__ __forceinline__ V oq_group_sum(V v, int P) {
+  for (int o = P >> 1; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// One sweep of a walker on its P lanes; returns the accepted moves (the same
+// on every lane).  All lanes of the warp call it; walkers beyond the tile
+// (live = false) never accept.
+template <int NOCC, typename T, typename Real, class B>
+__device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const OqSystem& S,
+                                              const OqSplit& SP, const Real* C, double* pos,
+                                              Real* Ai, double* rI, int WT, int lane, int P,
+                                              bool live, uint32_t w, uint32_t gstep, double step,
+                                              const OqScaledF& pf, double& logdet) {
+  constexpr int NE = 2 * NOCC;
+  constexpr int NN = NOCC * NOCC;
+  double det = 1.0;         // product of the accepted |R|: one logarithm per sweep
+  const unsigned gbits = P == 32 ? 0xffffffffu : (1u << P) - 1u;
+  const int gshift = (threadIdx.x & 31) & ~(P - 1);
+  int nacc = 0;
+  for (int e0 = 0; e0 < NE; e0 += P) {
+    // this lane's electron of the block: proposal and orbital row
+    const int e = e0 + lane;
+    double nx = 0.0, ny = 0.0, nz = 0.0;
+    T u = (T)2, mul = (T)1, lx = (T)0;
+    T v[NOCC];
+#pragma unroll
+    for (int m = 0; m < NOCC; ++m) v[m] = (T)0;
+    if (live && e < NE) {
+      float nf[3];
+      uint32_t ub;
+      oq_move_normals(a.seed, w, gstep, (uint32_t)e, nf, ub);
+      u = oq_uniform<T>(ub);
+      const double ox = pos[(3 * e) * WT], oy = pos[(3 * e + 1) * WT], oz = pos[(3 * e + 2) * WT];
+      if (a.proposal == 0) {
+        nx = ox + step * (double)nf[0];
+        ny = oy + step * (double)nf[1];
+        nz = oz + step * (double)nf[2];
+      } else {
+        oq_scaled_propose_t<T>(S, ox, oy, oz, nf, pf, nx, ny, nz, mul, lx);
+      }
+      B::template mo_val<T, Real>(S, SP, C, nx, ny, nz, v);
+    }
+    // the block's moves in order
+    const int nb = min(P, NE - e0);
+    for (int q = 0; q < nb; ++q) {
+      const int ee = e0 + q, s = ee & 1, i = ee >> 1;
+      const double bx = __shfl_sync(0xffffffffu, nx, q, P);
+      const double by = __shfl_sync(0xffffffffu, ny, q, P);
+      const double bz = __shfl_sync(0xffffffffu, nz, q, P);
+      const T bu = __shfl_sync(0xffffffffu, u, q, P);
+      const T bmul = __shfl_sync(0xffffffffu, mul, q, P);
+      const T blx = __shfl_sync(0xffffffffu, lx, q, P);
+      T bv[NOCC];
+#pragma unroll
+      for (int m = 0; m < NOCC; ++m) bv[m] = __shfl_sync(0xffffffffu, v[m], q, P);
+      const double ox = pos[(3 * ee) * WT], oy = pos[(3 * ee + 1) * WT],
+                   oz = pos[(3 * ee + 2) * WT];
+      bool valid;
+      T dJ;
+      if (sizeof(T) == 8) {
+        dJ = oq_jastrow_part<NE, T>(S, pos, WT, ee, lane, P, ox, oy, oz, bx, by, bz, valid);
+        if (OQ_HAS_J3(S))
+          dJ += oq_j3_delta_lane<NE, T>(S, pos, WT, rI, WT, ee, lane, P, ox, oy, oz, bx, by, bz);
+        dJ = oq_group_sum(dJ, P);
+        valid = ((__ballot_sync(0xffffffffu, !valid) >> gshift) & gbits) == 0u;
+      } else {
+        dJ = oq_jastrow_delta<NE, T>(S, S, pos, WT, ee, ox, oy, oz, bx, by, bz, valid);
+      }
+      Real* As = Ai + (size_t)s * NN * WT;
+      T R = (T)0;
+      T coli[NOCC];
+#pragma unroll
+      for (int k = 0; k < NOCC; ++k) {
+        coli[k] = (T)As[(k * NOCC + i) * WT];
+        R += bv[k] * coli[k];
+      }
+      const bool acc = live && oq_accept<T>(R, dJ, blx, bmul, bu, valid);
+      // every lane has read column i before any lane updates it
+      __syncwarp();
+      if (acc) {
+        const T rinv = oq_rcp(R);
+        for (int j = lane; j < NOCC; j += P) {
+          T wj = (T)0;
+#pragma unroll
+          for (int m = 0; m < NOCC; ++m) wj += bv[m] * (T)As[(m * NOCC + j) * WT];
+          const T f = (wj - (j == i ? (T)1 : (T)0)) * rinv;
+#pragma unroll
+          for (int k = 0; k < NOCC; ++k) {
+            Real& ref = As[(k * NOCC + j) * WT];
+            ref = (Real)((T)ref - coli[k] * f);
+          }
+        }
+        if (lane == 0) {
+          pos[(3 * ee) * WT] = bx;
+          pos[(3 * ee + 1) * WT] = by;
+          pos[(3 * ee + 2) * WT] = bz;
+        }
+        if (sizeof(T) == 8 && OQ_HAS_J3(S))
+          for (int I = lane; I < S.natm; I += P) {
+            const double ax = bx - S.nuc[I][0], ay = by - S.nuc[I][1], az = bz - S.nuc[I][2];
+            rI[(I * NE + ee) * WT] = sqrt(ax * ax + ay * ay + az * az);
+          }
+        ++nacc;
+        det *= fabs((double)R);
+        if (!(det > 1e-150 && det < 1e150)) {
+          logdet += log(det);
+          det = 1.0;
+        }
+      }
+      // the move is visible to every lane before the next one
+      __syncwarp();
+    }
+  }
+  logdet += log(det);
+  return nacc;
+}
+
+// Three-body part of the local energy of electron e: terms t = q, q + Q, ...
+// of the nucleus-electron list (the terms of oq_j3_vgl_electron).
+template <int NE, typename T>
+__device__ __forceinline__ void oq_j3_vgl_part(const OqSystem& S, const double* pos, int ps,
+                                               int e, int q, int Q, double x, double y, double z,
+                                               T& gx, T& gy, T& gz, T& lp) {
+  const int nI = S.j3_nI, nE = S.j3_nE, bsz = (nI + 1) * (nI + 1) * (nE + 1);
+  const T L = (T)S.j3_L;
+  for (int t = q; t < S.natm * NE; t += Q) {
+    const int I = t / NE, j = t - I * NE, ty = S.j3_type[I], blk = (e ^ j) & 1;
+    if (j == e || ty < 0 || !S.j3_on[ty][blk]) continue;
+    const T ax = (T)(x - S.nuc[I][0]), ay = (T)(y - S.nuc[I][1]), az = (T)(z - S.nuc[I][2]);
+    const T r1 = sqrt(ax * ax + ay * ay + az * az);
+    if (!(r1 < L)) continue;
+    const double xj = pos[(3 * j) * ps], yj = pos[(3 * j + 1) * ps], zj = pos[(3 * j + 2) * ps];
+    const T bx = (T)(xj - S.nuc[I][0]), by = (T)(yj - S.nuc[I][1]), bz = (T)(zj - S.nuc[I][2]);
+    const T r2 = sqrt(bx * bx + by * by + bz * bz);
+    if (!(r2 < L)) continue;
+    const T dx = (T)(x - xj), dy = (T)(y - yj), dz = (T)(z - zj);
+    const T r12 = sqrt(dx * dx + dy * dy + dz * dz);
+    const T i1 = (T)1 / r1, i12 = (T)1 / r12;
+    const T e1x = ax * i1, e1y = ay * i1, e1z = az * i1;
+    const T ex = dx * i12, ey = dy * i12, ez = dz * i12;
+    T u1, ue, u11, uee, u1e;
+    oq_j3_partials_n<T>(S.j3_gamma + (size_t)(2 * ty + blk) * bsz, nI, nE, L, r12, r1, r2, u1, ue,
+                        u11, uee, u1e);
+    gx -= u1 * e1x + ue * ex;
+    gy -= u1 * e1y + ue * ey;
+    gz -= u1 * e1z + ue * ez;
+    lp -= u11 + (T)2 * u1 * i1 + uee + (T)2 * ue * i12 +
+          (T)2 * u1e * (e1x * ex + e1y * ey + e1z * ez);
+  }
+}
+
+template <int NOCC, typename T, typename Real, class B = OqBasisTable<NOCC>>
+__global__ void __launch_bounds__(128, 4)
+k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
+         const void* __restrict__ gC, OqSweepArgs a) {
+  constexpr int NE = 2 * NOCC;
+  constexpr int NN = NOCC * NOCC;
+  extern __shared__ __align__(16) unsigned char smem[];
+  OqSystem& S = *reinterpret_cast<OqSystem*>(smem);
+  OqSplit& SP = *reinterpret_cast<OqSplit*>(smem + sizeof(OqSystem));
+  unsigned char* p = smem + sizeof(OqSystem) + sizeof(OqSplit);
+  Real* C = reinterpret_cast<Real*>(p);
+  const int nbf = gsys->nbf, natm = gsys->natm;
+  p += ((size_t)nbf * NOCC * sizeof(Real) + 15) & ~(size_t)15;
+  const int P = a.lanes, WT = blockDim.x / P, tid = threadIdx.x;
+  const int lane = tid & (P - 1), wl = tid / P, W = a.W;
+  double* pos0 = reinterpret_cast<double*>(p);          // [3 NE][WT]
+  p += (size_t)3 * NE * WT * 8;
+  Real* Ai0 = reinterpret_cast<Real*>(p);               // [2 NN][WT]
+  p += ((size_t)2 * NN * WT * sizeof(Real) + 15) & ~(size_t)15;
+  double* rI0 = reinterpret_cast<double*>(p);           // [natm][NE][WT], three-body terms only
+  double* gam = rI0 + (size_t)natm * NE * WT;
+  const int w0 = blockIdx.x * WT, cnt = min(WT, W - w0);
+  oq_load_system(&S, gsys);
+  {
+    const double* src = reinterpret_cast<const double*>(gsplit);
+    double* dst = reinterpret_cast<double*>(&SP);
+    for (int i = tid; i < OQ_MAX_GROUP; i += blockDim.x) dst[i] = src[i];
+    const Real* gc = reinterpret_cast<const Real*>(gC);
+    for (int i = tid; i < nbf * NOCC; i += blockDim.x) C[i] = gc[i];
+    const double* x = a.X + (size_t)w0 * 3 * NE;
+    for (int q = tid; q < cnt * 3 * NE; q += blockDim.x) {
+      const int j = q / (3 * NE), k = q - j * 3 * NE;
+      pos0[k * WT + j] = x[q];
+    }
+    const Real* gA = reinterpret_cast<const Real*>(a.ainv);
+    for (int q = tid; q < 2 * NN * WT; q += blockDim.x) {
+      const int k = q / WT, j = q - k * WT;
+      if (j < cnt) Ai0[q] = gA[(size_t)k * W + w0 + j];
+    }
+    for (int i = tid; i < a.j3_len; i += blockDim.x) gam[i] = gsys->j3_gamma[i];
+  }
+  __syncthreads();
+  if (a.j3_cache) {
+    // the three-body code reads the table through S
+    if (tid == 0 && a.j3_len) S.j3_gamma = gam;
+    for (int q = tid; q < natm * NE * cnt; q += blockDim.x) {
+      const int j = q % cnt, t = q / cnt, I = t / NE, e = t - I * NE;
+      const double dx = pos0[(3 * e) * WT + j] - S.nuc[I][0],
+                   dy = pos0[(3 * e + 1) * WT + j] - S.nuc[I][1],
+                   dz = pos0[(3 * e + 2) * WT + j] - S.nuc[I][2];
+      rI0[t * WT + j] = sqrt(dx * dx + dy * dy + dz * dz);
+    }
+    __syncthreads();
+  }
+  const bool live = wl < cnt;
+  const uint32_t w = (uint32_t)(w0 + wl);
+  double* pos = pos0 + wl;
+  Real* Ai = Ai0 + wl;
+  double* rI = rI0 + wl;
+  const double step = a.step_dev ? *a.step_dev : a.step;
+  const OqScaledF pf = oq_scaled_f(step, a.scale_r0, a.scale_fmin);
+  double logdet = live ? a.logdet[w] : 0.0;
+  const int n_meas = a.measure_every > 0 ? a.n_sweeps / a.measure_every : 0;
+  // lanes of one electron in the local energy: Q lanes share its pair terms
+  int PE = 1;
+  while (PE < P && PE < NE) PE <<= 1;
+  const int Q = P / PE, le = lane & (PE - 1), lq = lane / PE;
+  int nacc = 0, meas = 0;
+  for (int t = 0; t < a.n_sweeps; ++t) {
+    const uint32_t gstep = (uint32_t)(a.step_base + t);
+    if (P > 1) {
+      nacc += oq_sweep_lanes<NOCC, T, Real, B>(a, S, SP, C, pos, Ai, rI, WT, lane, P, live, w,
+                                               gstep, step, pf, logdet);
+    } else if (live) {
+      for (int e = 0; e < NE; ++e) {
+        float nf[3];
+        uint32_t ub;
+        oq_move_normals(a.seed, w, gstep, (uint32_t)e, nf, ub);
+        const T u = oq_uniform<T>(ub);
+        const double ox = pos[(3 * e) * WT], oy = pos[(3 * e + 1) * WT],
+                     oz = pos[(3 * e + 2) * WT];
+        double nx, ny, nz;
+        T mul = (T)1, lx = (T)0;
+        if (a.proposal == 0) {
+          nx = ox + step * (double)nf[0];
+          ny = oy + step * (double)nf[1];
+          nz = oz + step * (double)nf[2];
+        } else {
+          oq_scaled_propose_t<T>(S, ox, oy, oz, nf, pf, nx, ny, nz, mul, lx);
+        }
+        nacc += oq_try_move_s<NOCC, T, Real, B>(S, S, SP, C, pos, WT, Ai, WT, e, nx, ny, nz, lx,
+                                                mul, u, logdet);
+      }
+    }
+    if (meas == n_meas || (t + 1) % a.measure_every != 0) continue;
+    // a walker's state is read and written only by its own lanes, which
+    // share one warp: the moves are complete for them after a warp barrier
+    __syncwarp();
+    double see = 0.0, sen = 0.0, slp = 0.0, sg2 = 0.0;
+    if (sizeof(T) == 4) {
+      if (live && lq == 0)
+        for (int e = le; e < NE; e += PE)
+          oq_eloc_electron<NOCC, T, Real, B>(S, S, SP, C, pos, (size_t)WT, Ai, (size_t)WT, e, see,
+                                             sen, slp, sg2);
+    } else {
+      // one electron per lane; its three-body terms split over Q lanes
+      for (int e0 = 0; e0 < NE; e0 += PE) {
+        const bool mine_e = live && e0 + le < NE;
+        const int e = mine_e ? e0 + le : 0, s = e & 1, i = e >> 1;
+        const double xe = pos[(3 * e) * WT], ye = pos[(3 * e + 1) * WT],
+                     ze = pos[(3 * e + 2) * WT];
+        T jx = (T)0, jy = (T)0, jz = (T)0, jl = (T)0;
+        if (OQ_HAS_J3(S)) {
+          if (mine_e) oq_j3_vgl_part<NE, T>(S, pos, WT, e, lq, Q, xe, ye, ze, jx, jy, jz, jl);
+          for (int o = PE; o < P; o <<= 1) {
+            jx += __shfl_xor_sync(0xffffffffu, jx, o);
+            jy += __shfl_xor_sync(0xffffffffu, jy, o);
+            jz += __shfl_xor_sync(0xffffffffu, jz, o);
+            jl += __shfl_xor_sync(0xffffffffu, jl, o);
+          }
+        }
+        if (mine_e && lq == 0) {
+          T ac[NOCC];
+#pragma unroll
+          for (int m = 0; m < NOCC; ++m) ac[m] = (T)Ai[((s * NOCC + m) * NOCC + i) * WT];
+          T gx, gy, gz, lp;
+          B::template mo_vgl_contract<T, Real>(S, SP, C, xe, ye, ze, ac, gx, gy, gz, lp);
+          oq_jastrow_vgl_coulomb<NE, T>(S, S, pos, (size_t)WT, e, xe, ye, ze, jx, jy, jz, jl, see,
+                                        sen, false);
+          const double sx = (double)gx, sy = (double)gy, sz = (double)gz;
+          const double Gx = sx + (double)jx, Gy = sy + (double)jy, Gz = sz + (double)jz;
+          slp += (double)lp - (sx * sx + sy * sy + sz * sz) + (double)jl;
+          sg2 += Gx * Gx + Gy * Gy + Gz * Gz;
+        }
+      }
+    }
+    see = oq_group_sum(see, P);
+    sen = oq_group_sum(sen, P);
+    slp = oq_group_sum(slp, P);
+    sg2 = oq_group_sum(sg2, P);
+    const double ke = -0.5 * (slp + sg2);
+    const double el = see + sen + ke + S.e_nn;
+    const bool mine = live && lane == 0;
+    const bool ok = mine && isfinite(el);
+    if (mine) {
+      if (a.el_trace) a.el_trace[(size_t)meas * W + w] = el;
+      if (a.eparts_last && meas == n_meas - 1) {
+        double* ep = a.eparts_last + (size_t)w * 4;
+        ep[0] = see; ep[1] = sen; ep[2] = ke; ep[3] = el;
+      }
+      if (!ok) atomicOr(a.flags, OQ_FLAG_NAN);
+    }
+    double vals[7] = {ok ? see : 0.0, ok ? sen : 0.0, ok ? ke : 0.0, ok ? el : 0.0,
+                      ok ? el * el : 0.0, mine ? (double)nacc : 0.0, ok ? 1.0 : 0.0};
+#pragma unroll
+    for (int k = 0; k < 7; ++k) vals[k] = oq_group_sum(vals[k], 32);
+    if ((tid & 31) == 0) {
+      double* sm = a.sums + (size_t)meas * OQ_NSUM;
+#pragma unroll
+      for (int k = 0; k < 7; ++k) atomicAdd(sm + k, vals[k]);
+    }
+    // the next sweep's moves change state this measurement read
+    __syncwarp();
+    nacc = 0;
+    ++meas;
+  }
+  __syncthreads();
+  {
+    double* x = a.X + (size_t)w0 * 3 * NE;
+    for (int q = tid; q < cnt * 3 * NE; q += blockDim.x) {
+      const int j = q / (3 * NE), k = q - j * 3 * NE;
+      x[q] = pos0[k * WT + j];
+    }
+    Real* gA = reinterpret_cast<Real*>(a.ainv);
+    for (int q = tid; q < 2 * NN * WT; q += blockDim.x) {
+      const int k = q / WT, j = q - k * WT;
+      if (j < cnt) gA[(size_t)k * W + w0 + j] = Ai0[q];
+    }
+    if (a.pos)
+      for (int q = tid; q < 3 * NE * WT; q += blockDim.x) {
+        const int k = q / WT, j = q - k * WT;
+        if (j < cnt) a.pos[(size_t)k * W + w0 + j] = pos0[q];
+      }
+  }
+  if (live && lane == 0) a.logdet[w] = logdet;
+  if (!a.acc_sum) return;
+  const int mine = (int)oq_group_sum(live && lane == 0 ? nacc : 0, 32);
+  if (!a.step_dev) {
+    if ((tid & 31) == 0) atomicAdd(a.acc_sum, (double)mine);
+    return;
+  }
+  // Step adaptation (_adapt_step_size, OmegaQMC/vmc_gto.py:121-126): log s <-
+  // log s + rate (acc - target).  Every CTA adds its accepted moves plus one
+  // `tick`, a power of two above all moves of the sweep, to the sweep's slot;
+  // the sum is exact, so the CTA that brings it to gridDim.x ticks is the last
+  // one, knows the total, and every CTA has read the old width by then.  A
+  // kernel of one thread for this cost a launch per equilibration step.
+  int* part = reinterpret_cast<int*>(pos0);     // the walkers are written out
+  __syncthreads();
+  if ((tid & 31) == 0) part[tid >> 5] = mine;
+  __syncthreads();
+  if (tid != 0) return;
+  int tot = 0;
+  for (int k = 0; k < (int)blockDim.x / 32; ++k) tot += part[k];
+  const double now = atomicAdd(a.acc_sum, (double)tot + a.tick) + (double)tot + a.tick;
+  if (now >= a.tick * (double)gridDim.x) {
+    const double acc = (now - a.tick * (double)gridDim.x) * a.inv_moves;
+    const double sn = exp(log(step) + a.rate * (acc - a.target));
+    *a.acc_sum = acc;
+    *a.step_dev = sn;
+    if (a.step_trace) *a.step_trace = sn;
   }
 }
