@@ -1337,9 +1337,8 @@ static int launch_moves(oqmc_ctx* ctx, const OqMoveArgs& m, int wpb, size_t sm, 
 }
 
 // Lanes per walker of the fused sweeps: as many as there are electrons (all
-// orbital rows of a sweep at once; 32 with three-body terms in FP64, whose
-// nucleus-electron list fills them), halved while the threads would exceed
-// 512 per SM.  Beyond that the register file (128 per thread) is full and
+// orbital rows of a sweep at once; 32 with three-body terms in FP64, which
+// fill them), halved while the threads would exceed 512 per SM.  Beyond that the register file (128 per thread) is full and
 // lanes only add shuffles.
 static int sweep_lanes(const oqmc_ctx* ctx, int W, int mixed) {
   int P = 1;

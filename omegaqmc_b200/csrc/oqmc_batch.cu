@@ -107,7 +107,7 @@ std::string kernel_name(int precision, int v) {
 size_t tile_smem(int nocc, int wt, int nt, int precision) {
   (void)nt;
   const size_t real = precision == OQ_PREC_MIXED ? 4 : 8;
-  return (size_t)6 * nocc * wt * 8 + (size_t)2 * nocc * nocc * wt * real;
+  return (size_t)(6 * nocc + 1) * wt * 8 + (size_t)(2 * nocc * nocc + 1) * wt * real;
 }
 
 }  // namespace

@@ -194,8 +194,8 @@ template <int NOCC, typename T, typename Real, class B, class SJ>
 __device__ __forceinline__ int oq_batch_sweep_lanes(const OqBatchArgs& a, const OqBatchSys& d,
                                                     const SJ& J, const OqSystem& S,
                                                     const OqSplit& SP, const Real* C,
-                                                    double* pos, Real* Ai, int WT, int wl,
-                                                    int lane, int P, bool live, uint32_t w,
+                                                    double* pos, Real* Ai, int lane,
+                                                    int P, bool live, uint32_t w,
                                                     uint32_t gstep, const OqScaledF& pf,
                                                     double& logdet) {
   constexpr int NE = 2 * NOCC;
@@ -214,8 +214,8 @@ __device__ __forceinline__ int oq_batch_sweep_lanes(const OqBatchArgs& a, const 
       uint32_t ub;
       oq_move_normals(a.seed, w, gstep, (uint32_t)e, nf, ub);
       u = oq_uniform<T>(ub);
-      const double ox = pos[(3 * e) * WT + wl], oy = pos[(3 * e + 1) * WT + wl],
-                   oz = pos[(3 * e + 2) * WT + wl];
+      const double ox = pos[3 * e], oy = pos[3 * e + 1],
+                   oz = pos[3 * e + 2];
       if (d.proposal == 0) {
         nx = ox + d.step * (double)nf[0];
         ny = oy + d.step * (double)nf[1];
@@ -238,19 +238,19 @@ __device__ __forceinline__ int oq_batch_sweep_lanes(const OqBatchArgs& a, const 
       T bv[NOCC];
 #pragma unroll
       for (int m = 0; m < NOCC; ++m) bv[m] = __shfl_sync(0xffffffffu, v[m], q, P);
-      const double ox = pos[(3 * ee) * WT + wl], oy = pos[(3 * ee + 1) * WT + wl],
-                   oz = pos[(3 * ee + 2) * WT + wl];
+      const double ox = pos[3 * ee], oy = pos[3 * ee + 1],
+                   oz = pos[3 * ee + 2];
       bool valid;
-      T dJ = oq_jastrow_delta_lane<NE, T>(J, S, pos + wl, WT, ee, lane, P, ox, oy, oz, bx, by,
+      T dJ = oq_jastrow_delta_lane<NE, T>(J, S, pos, 1, ee, lane, P, ox, oy, oz, bx, by,
                                           bz, valid);
       dJ = oq_lanes_sum(dJ, P);
       valid = oq_lanes_and(valid, P);
-      Real* As = Ai + (size_t)s * NN * WT;
+      Real* As = Ai + s * NN;
       T R = (T)0;
       T coli[NOCC];
 #pragma unroll
       for (int k = 0; k < NOCC; ++k) {
-        coli[k] = (T)As[(k * NOCC + i) * WT + wl];
+        coli[k] = (T)As[k * NOCC + i];
         R += bv[k] * coli[k];
       }
       const bool acc = live && oq_accept<T>(R, dJ, blx, bmul, bu, valid);
@@ -261,18 +261,18 @@ __device__ __forceinline__ int oq_batch_sweep_lanes(const OqBatchArgs& a, const 
         for (int j = lane; j < NOCC; j += P) {
           T wj = (T)0;
 #pragma unroll
-          for (int m = 0; m < NOCC; ++m) wj += bv[m] * (T)As[(m * NOCC + j) * WT + wl];
+          for (int m = 0; m < NOCC; ++m) wj += bv[m] * (T)As[m * NOCC + j];
           const T f = (wj - (j == i ? (T)1 : (T)0)) * rinv;
 #pragma unroll
           for (int k = 0; k < NOCC; ++k) {
-            Real& ref = As[(k * NOCC + j) * WT + wl];
+            Real& ref = As[k * NOCC + j];
             ref = (Real)((T)ref - coli[k] * f);
           }
         }
         if (lane == 0) {
-          pos[(3 * ee) * WT + wl] = bx;
-          pos[(3 * ee + 1) * WT + wl] = by;
-          pos[(3 * ee + 2) * WT + wl] = bz;
+          pos[3 * ee] = bx;
+          pos[3 * ee + 1] = by;
+          pos[3 * ee + 2] = bz;
           ++nacc;
         }
         logdet += log(fabs((double)R));
@@ -284,8 +284,13 @@ __device__ __forceinline__ int oq_batch_sweep_lanes(const OqBatchArgs& a, const 
   return nacc;
 }
 
-// Shared memory of one tile: [positions [3 NE][WT] doubles][inverses
-// [2 NOCC^2][WT] Real].  The nuclei and Jastrow constants (J) are the
+// Shared memory of one tile: [positions [WT][3 NE + 1] doubles][inverses
+// [WT][2 NOCC^2 + 1] Real].  A walker's state is contiguous, so that every
+// access is a base register plus an immediate offset, and the odd pitches put
+// the walkers of a warp on different banks (walker-minor, the offsets were
+// multiplied out at run time: 65,536 H2O walkers, 50 sweeps, 4,196 -> 3,956
+// us; 524,288 walkers, 683 -> 661 us per sweep although one CTA fewer fits an
+// SM).  The nuclei and Jastrow constants (J) are the
 // system's OqJas in constant memory, written into the generated module, so
 // every lane of a warp reads the same word (a broadcast) and the tile's
 // shared memory holds walker state only.  With P = NT / WT lanes per walker
@@ -302,8 +307,10 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
   constexpr int NE = 2 * NOCC;
   const int NT = blockDim.x, tid = threadIdx.x, WT = d.wt;
   const int P = NT / WT, lane = tid & (P - 1), wl = tid / P;
-  double* pos = reinterpret_cast<double*>(smem);                    // [3 NE][WT]
-  Real* Ai = reinterpret_cast<Real*>(pos + 3 * NE * WT);           // [2 NOCC^2][WT]
+  constexpr int PP = 3 * NE + 1, AP = 2 * NOCC * NOCC + 1;
+  double* pos0 = reinterpret_cast<double*>(smem);                   // [WT][PP]
+  double* pos = pos0 + wl * PP;
+  Real* Ai = reinterpret_cast<Real*>(pos0 + PP * WT) + wl * AP;     // [WT][AP]
   const OqSystem& S = *d.sys;
   const OqSplit& SP = *d.split;
   const Real* C = sizeof(Real) == 4 ? reinterpret_cast<const Real*>(d.C32)
@@ -315,7 +322,7 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
     const double* src = d.walkers + (size_t)w0 * 3 * NE;
     for (int q = tid; q < cnt * 3 * NE; q += NT) {
       const int wq = q / (3 * NE), k = q - wq * 3 * NE;
-      pos[k * WT + wq] = src[q];
+      pos0[wq * PP + k] = src[q];
     }
   }
   __syncthreads();
@@ -332,8 +339,8 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
         for (int i = 0; i < NOCC; ++i) {
           const int e = 2 * i + s;
           double mv[NOCC];
-          oq_mo_val<NOCC>(S, d.C64, pos[(3 * e) * WT + wl], pos[(3 * e + 1) * WT + wl],
-                          pos[(3 * e + 2) * WT + wl], mv);
+          oq_mo_val<NOCC>(S, d.C64, pos[3 * e], pos[3 * e + 1],
+                          pos[3 * e + 2], mv);
 #pragma unroll
           for (int m = 0; m < NOCC; ++m) Sm[i][m] = mv[m];
         }
@@ -343,7 +350,7 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
         logdet += ld;
         for (int m = 0; m < NOCC; ++m)
           for (int j = 0; j < NOCC; ++j)
-            Ai[((s * NOCC + m) * NOCC + j) * WT + wl] = oks ? (Real)Ainv[m][j] : (Real)0;
+            Ai[(s * NOCC + m) * NOCC + j] = oks ? (Real)Ainv[m][j] : (Real)0;
       }
     }
     if (P > 1) {
@@ -361,18 +368,17 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
   for (int t = 0; t < a.n_sweeps; ++t) {
     const uint32_t gstep = (uint32_t)(step0 + t);
     if (MODE != 1 && P > 1) {
-      nacc += oq_batch_sweep_lanes<NOCC, T, Real, B>(a, d, J, S, SP, C, pos, Ai, WT, wl, lane,
-                                                     P, live, (uint32_t)w, gstep, pf, logdet);
+      nacc += oq_batch_sweep_lanes<NOCC, T, Real, B>(a, d, J, S, SP, C, pos, Ai, lane, P, live, (uint32_t)w, gstep, pf, logdet);
     } else if (MODE != 2 && live) {
       for (int e = 0; e < NE; ++e) {
         float nf[3];
         uint32_t ub;
         oq_move_normals(a.seed, (uint32_t)w, gstep, (uint32_t)e, nf, ub);
         const T u = oq_uniform<T>(ub);
-        const double ox = pos[(3 * e) * WT + wl], oy = pos[(3 * e + 1) * WT + wl],
-                     oz = pos[(3 * e + 2) * WT + wl];
+        const double ox = pos[3 * e], oy = pos[3 * e + 1],
+                     oz = pos[3 * e + 2];
         if (d.proposal == 0) {
-          nacc += oq_try_move<NOCC, T, Real, B>(J, S, SP, C, pos, Ai, WT, wl, e,
+          nacc += oq_try_move_s<NOCC, T, Real, B>(J, S, SP, C, pos, 1, Ai, 1, e,
                                                 ox + d.step * (double)nf[0],
                                                 oy + d.step * (double)nf[1],
                                                 oz + d.step * (double)nf[2], (T)0, (T)1, u,
@@ -381,7 +387,7 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
           double nx, ny, nz;
           T mul, lx;
           oq_scaled_propose_t<T>(J, ox, oy, oz, nf, pf, nx, ny, nz, mul, lx);
-          nacc += oq_try_move<NOCC, T, Real, B>(J, S, SP, C, pos, Ai, WT, wl, e, nx, ny, nz, lx,
+          nacc += oq_try_move_s<NOCC, T, Real, B>(J, S, SP, C, pos, 1, Ai, 1, e, nx, ny, nz, lx,
                                                 mul, u, logdet);
         }
       }
@@ -394,8 +400,8 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
     double see = 0.0, sen = 0.0, slp = 0.0, sg2 = 0.0;
     if (live)
       for (int e = lane; e < NE; e += P)
-        oq_eloc_electron<NOCC, T, Real, B>(J, S, SP, C, pos + wl, (size_t)WT, Ai + wl,
-                                           (size_t)WT, e, see, sen, slp, sg2);
+        oq_eloc_electron<NOCC, T, Real, B>(J, S, SP, C, pos, 1, Ai, 1, e, see,
+                                           sen, slp, sg2);
     if (P > 1) {
       see = oq_lanes_sum(see, P);
       sen = oq_lanes_sum(sen, P);
@@ -435,7 +441,7 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
     double* dst = d.walkers + (size_t)w0 * 3 * NE;
     for (int q = tid; q < cnt * 3 * NE; q += NT) {
       const int wq = q / (3 * NE), k = q - wq * 3 * NE;
-      dst[q] = pos[k * WT + wq];
+      dst[q] = pos0[wq * PP + k];
     }
   }
   if (tid == 0) atomicAdd(d.busy_ns, oq_globaltimer() - t_start);

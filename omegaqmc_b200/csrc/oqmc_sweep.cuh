@@ -1096,16 +1096,17 @@ struct OqSweepArgs {
 // lanes, the nucleus-electron distances and the gamma table.
 inline size_t oq_sweep_tile_bytes(int nocc, int natm, int wt, size_t real, int j3_cache,
                                   int j3_len) {
-  return (size_t)6 * nocc * wt * 8 + (((size_t)2 * nocc * nocc * wt * real + 15) & ~(size_t)15) +
-         (j3_cache ? (size_t)2 * nocc * natm * wt * 8 + (size_t)j3_len * 8 : 0);
+  return (size_t)(6 * nocc + 1) * wt * 8 +
+         (((size_t)(2 * nocc * nocc + 1) * wt * real + 15) & ~(size_t)15) +
+         (j3_cache ? (size_t)(2 * nocc * natm + 1) * wt * 8 + (size_t)j3_len * 8 : 0);
 }
 
 // This lane's share of the change of J3 when electron e moves to n (terms
 // t = lane, lane + P, ... of the nucleus-electron list).  rI holds the
-// walker's nucleus-electron distances [I][j], stride rs.
+// walker's nucleus-electron distances [I][j].
 template <int NE, typename T>
-__device__ __forceinline__ T oq_j3_delta_lane(const OqSystem& S, const double* pos, int ps,
-                                              const double* rI, int rs, int e, int lane, int P,
+__device__ __forceinline__ T oq_j3_delta_lane(const OqSystem& S, const double* pos,
+                                              const double* rI, int e, int lane, int P,
                                               double ox, double oy, double oz, double nx,
                                               double ny, double nz) {
   const int nI = S.j3_nI, nE = S.j3_nE, bsz = (nI + 1) * (nI + 1) * (nE + 1);
@@ -1114,13 +1115,13 @@ __device__ __forceinline__ T oq_j3_delta_lane(const OqSystem& S, const double* p
   for (int t = lane; t < S.natm * NE; t += P) {
     const int I = t / NE, j = t - I * NE, ty = S.j3_type[I], blk = (e ^ j) & 1;
     if (j == e || ty < 0 || !S.j3_on[ty][blk]) continue;
-    const T r2 = (T)rI[t * rs];
+    const T r2 = (T)rI[t];
     if (!(r2 < L)) continue;
-    const T r1o = (T)rI[(I * NE + e) * rs];
+    const T r1o = (T)rI[I * NE + e];
     const double ax = nx - S.nuc[I][0], ay = ny - S.nuc[I][1], az = nz - S.nuc[I][2];
     const T r1n = sqrt((T)(ax * ax + ay * ay + az * az));
     const double* g = S.j3_gamma + (size_t)(2 * ty + blk) * bsz;
-    const double xj = pos[(3 * j) * ps], yj = pos[(3 * j + 1) * ps], zj = pos[(3 * j + 2) * ps];
+    const double xj = pos[3 * j], yj = pos[3 * j + 1], zj = pos[3 * j + 2];
     if (r1n < L) {
       const double dx = nx - xj, dy = ny - yj, dz = nz - zj;
       acc += oq_j3_u_n<T>(g, nI, nE, L, sqrt((T)(dx * dx + dy * dy + dz * dz)), r1n, r2);
@@ -1137,7 +1138,7 @@ __device__ __forceinline__ T oq_j3_delta_lane(const OqSystem& S, const double* p
 // congruent to lane modulo P; the terms of oq_jastrow_delta) and of the
 // MIN_DIST_THRESHOLD test.
 template <int NE, typename T>
-__device__ __forceinline__ T oq_jastrow_part(const OqSystem& S, const double* pos, int ps, int e,
+__device__ __forceinline__ T oq_jastrow_part(const OqSystem& S, const double* pos, int e,
                                              int lane, int P, double ox, double oy, double oz,
                                              double nx, double ny, double nz, bool& valid) {
   const double thr2 = 1e-4 * 1e-4;
@@ -1145,7 +1146,7 @@ __device__ __forceinline__ T oq_jastrow_part(const OqSystem& S, const double* po
   valid = true;
   for (int j = lane; j < NE; j += P) {
     if (j == e) continue;
-    const double xj = pos[(3 * j) * ps], yj = pos[(3 * j + 1) * ps], zj = pos[(3 * j + 2) * ps];
+    const double xj = pos[3 * j], yj = pos[3 * j + 1], zj = pos[3 * j + 2];
     const double ax = nx - xj, ay = ny - yj, az = nz - zj;
     const double bx = ox - xj, by = oy - yj, bz = oz - zj;
     const double rn2 = ax * ax + ay * ay + az * az;
@@ -1196,7 +1197,7 @@ __device__ __forceinline__ V oq_group_sum(V v, int P) {
 template <int NOCC, typename T, typename Real, class B>
 __device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const OqSystem& S,
                                               const OqSplit& SP, const Real* C, double* pos,
-                                              Real* Ai, double* rI, int WT, int lane, int P,
+                                              Real* Ai, double* rI, int lane, int P,
                                               bool live, uint32_t w, uint32_t gstep, double step,
                                               const OqScaledF& pf, double& logdet) {
   constexpr int NE = 2 * NOCC;
@@ -1218,7 +1219,7 @@ __device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const OqSyst
       uint32_t ub;
       oq_move_normals(a.seed, w, gstep, (uint32_t)e, nf, ub);
       u = oq_uniform<T>(ub);
-      const double ox = pos[(3 * e) * WT], oy = pos[(3 * e + 1) * WT], oz = pos[(3 * e + 2) * WT];
+      const double ox = pos[3 * e], oy = pos[3 * e + 1], oz = pos[3 * e + 2];
       if (a.proposal == 0) {
         nx = ox + step * (double)nf[0];
         ny = oy + step * (double)nf[1];
@@ -1241,25 +1242,25 @@ __device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const OqSyst
       T bv[NOCC];
 #pragma unroll
       for (int m = 0; m < NOCC; ++m) bv[m] = __shfl_sync(0xffffffffu, v[m], q, P);
-      const double ox = pos[(3 * ee) * WT], oy = pos[(3 * ee + 1) * WT],
-                   oz = pos[(3 * ee + 2) * WT];
+      const double ox = pos[3 * ee], oy = pos[3 * ee + 1],
+                   oz = pos[3 * ee + 2];
       bool valid;
       T dJ;
       if (sizeof(T) == 8) {
-        dJ = oq_jastrow_part<NE, T>(S, pos, WT, ee, lane, P, ox, oy, oz, bx, by, bz, valid);
+        dJ = oq_jastrow_part<NE, T>(S, pos, ee, lane, P, ox, oy, oz, bx, by, bz, valid);
         if (OQ_HAS_J3(S))
-          dJ += oq_j3_delta_lane<NE, T>(S, pos, WT, rI, WT, ee, lane, P, ox, oy, oz, bx, by, bz);
+          dJ += oq_j3_delta_lane<NE, T>(S, pos, rI, ee, lane, P, ox, oy, oz, bx, by, bz);
         dJ = oq_group_sum(dJ, P);
         valid = ((__ballot_sync(0xffffffffu, !valid) >> gshift) & gbits) == 0u;
       } else {
-        dJ = oq_jastrow_delta<NE, T>(S, S, pos, WT, ee, ox, oy, oz, bx, by, bz, valid);
+        dJ = oq_jastrow_delta<NE, T>(S, S, pos, 1, ee, ox, oy, oz, bx, by, bz, valid);
       }
-      Real* As = Ai + (size_t)s * NN * WT;
+      Real* As = Ai + s * NN;
       T R = (T)0;
       T coli[NOCC];
 #pragma unroll
       for (int k = 0; k < NOCC; ++k) {
-        coli[k] = (T)As[(k * NOCC + i) * WT];
+        coli[k] = (T)As[k * NOCC + i];
         R += bv[k] * coli[k];
       }
       const bool acc = live && oq_accept<T>(R, dJ, blx, bmul, bu, valid);
@@ -1270,23 +1271,23 @@ __device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const OqSyst
         for (int j = lane; j < NOCC; j += P) {
           T wj = (T)0;
 #pragma unroll
-          for (int m = 0; m < NOCC; ++m) wj += bv[m] * (T)As[(m * NOCC + j) * WT];
+          for (int m = 0; m < NOCC; ++m) wj += bv[m] * (T)As[m * NOCC + j];
           const T f = (wj - (j == i ? (T)1 : (T)0)) * rinv;
 #pragma unroll
           for (int k = 0; k < NOCC; ++k) {
-            Real& ref = As[(k * NOCC + j) * WT];
+            Real& ref = As[k * NOCC + j];
             ref = (Real)((T)ref - coli[k] * f);
           }
         }
         if (lane == 0) {
-          pos[(3 * ee) * WT] = bx;
-          pos[(3 * ee + 1) * WT] = by;
-          pos[(3 * ee + 2) * WT] = bz;
+          pos[3 * ee] = bx;
+          pos[3 * ee + 1] = by;
+          pos[3 * ee + 2] = bz;
         }
         if (sizeof(T) == 8 && OQ_HAS_J3(S))
           for (int I = lane; I < S.natm; I += P) {
             const double ax = bx - S.nuc[I][0], ay = by - S.nuc[I][1], az = bz - S.nuc[I][2];
-            rI[(I * NE + ee) * WT] = sqrt(ax * ax + ay * ay + az * az);
+            rI[I * NE + ee] = sqrt(ax * ax + ay * ay + az * az);
           }
         ++nacc;
         det *= fabs((double)R);
@@ -1306,7 +1307,7 @@ __device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const OqSyst
 // Three-body part of the local energy of electron e: terms t = q, q + Q, ...
 // of the nucleus-electron list (the terms of oq_j3_vgl_electron).
 template <int NE, typename T>
-__device__ __forceinline__ void oq_j3_vgl_part(const OqSystem& S, const double* pos, int ps,
+__device__ __forceinline__ void oq_j3_vgl_part(const OqSystem& S, const double* pos,
                                                int e, int q, int Q, double x, double y, double z,
                                                T& gx, T& gy, T& gz, T& lp) {
   const int nI = S.j3_nI, nE = S.j3_nE, bsz = (nI + 1) * (nI + 1) * (nE + 1);
@@ -1317,7 +1318,7 @@ __device__ __forceinline__ void oq_j3_vgl_part(const OqSystem& S, const double* 
     const T ax = (T)(x - S.nuc[I][0]), ay = (T)(y - S.nuc[I][1]), az = (T)(z - S.nuc[I][2]);
     const T r1 = sqrt(ax * ax + ay * ay + az * az);
     if (!(r1 < L)) continue;
-    const double xj = pos[(3 * j) * ps], yj = pos[(3 * j + 1) * ps], zj = pos[(3 * j + 2) * ps];
+    const double xj = pos[3 * j], yj = pos[3 * j + 1], zj = pos[3 * j + 2];
     const T bx = (T)(xj - S.nuc[I][0]), by = (T)(yj - S.nuc[I][1]), bz = (T)(zj - S.nuc[I][2]);
     const T r2 = sqrt(bx * bx + by * by + bz * bz);
     if (!(r2 < L)) continue;
@@ -1352,12 +1353,17 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
   p += ((size_t)nbf * NOCC * sizeof(Real) + 15) & ~(size_t)15;
   const int P = a.lanes, WT = blockDim.x / P, tid = threadIdx.x;
   const int lane = tid & (P - 1), wl = tid / P, W = a.W;
-  double* pos0 = reinterpret_cast<double*>(p);          // [3 NE][WT]
-  p += (size_t)3 * NE * WT * 8;
-  Real* Ai0 = reinterpret_cast<Real*>(p);               // [2 NN][WT]
-  p += ((size_t)2 * NN * WT * sizeof(Real) + 15) & ~(size_t)15;
-  double* rI0 = reinterpret_cast<double*>(p);           // [natm][NE][WT], three-body terms only
-  double* gam = rI0 + (size_t)natm * NE * WT;
+  // a walker's state is contiguous (every index below is an immediate offset),
+  // with odd pitches so that the walkers of a warp fall on different banks;
+  // walker-minor, two thirds of the shared-memory wavefronts were conflicts
+  constexpr int PP = 3 * NE + 1, AP = 2 * NN + 1;
+  double* pos0 = reinterpret_cast<double*>(p);          // [WT][PP]
+  p += (size_t)PP * WT * 8;
+  Real* Ai0 = reinterpret_cast<Real*>(p);               // [WT][AP]
+  p += ((size_t)AP * WT * sizeof(Real) + 15) & ~(size_t)15;
+  double* rI0 = reinterpret_cast<double*>(p);           // [WT][natm NE + 1], three-body only
+  const int RP = natm * NE + 1;
+  double* gam = rI0 + (size_t)RP * WT;
   const int w0 = blockIdx.x * WT, cnt = min(WT, W - w0);
   oq_load_system(&S, gsys);
   {
@@ -1369,12 +1375,12 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
     const double* x = a.X + (size_t)w0 * 3 * NE;
     for (int q = tid; q < cnt * 3 * NE; q += blockDim.x) {
       const int j = q / (3 * NE), k = q - j * 3 * NE;
-      pos0[k * WT + j] = x[q];
+      pos0[j * PP + k] = x[q];
     }
     const Real* gA = reinterpret_cast<const Real*>(a.ainv);
     for (int q = tid; q < 2 * NN * WT; q += blockDim.x) {
       const int k = q / WT, j = q - k * WT;
-      if (j < cnt) Ai0[q] = gA[(size_t)k * W + w0 + j];
+      if (j < cnt) Ai0[j * AP + k] = gA[(size_t)k * W + w0 + j];
     }
     for (int i = tid; i < a.j3_len; i += blockDim.x) gam[i] = gsys->j3_gamma[i];
   }
@@ -1384,31 +1390,29 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
     if (tid == 0 && a.j3_len) S.j3_gamma = gam;
     for (int q = tid; q < natm * NE * cnt; q += blockDim.x) {
       const int j = q % cnt, t = q / cnt, I = t / NE, e = t - I * NE;
-      const double dx = pos0[(3 * e) * WT + j] - S.nuc[I][0],
-                   dy = pos0[(3 * e + 1) * WT + j] - S.nuc[I][1],
-                   dz = pos0[(3 * e + 2) * WT + j] - S.nuc[I][2];
-      rI0[t * WT + j] = sqrt(dx * dx + dy * dy + dz * dz);
+      const double dx = pos0[j * PP + 3 * e] - S.nuc[I][0],
+                   dy = pos0[j * PP + 3 * e + 1] - S.nuc[I][1],
+                   dz = pos0[j * PP + 3 * e + 2] - S.nuc[I][2];
+      rI0[j * RP + t] = sqrt(dx * dx + dy * dy + dz * dz);
     }
     __syncthreads();
   }
   const bool live = wl < cnt;
   const uint32_t w = (uint32_t)(w0 + wl);
-  double* pos = pos0 + wl;
-  Real* Ai = Ai0 + wl;
-  double* rI = rI0 + wl;
+  double* pos = pos0 + wl * PP;
+  Real* Ai = Ai0 + wl * AP;
+  double* rI = rI0 + wl * RP;
   const double step = a.step_dev ? *a.step_dev : a.step;
   const OqScaledF pf = oq_scaled_f(step, a.scale_r0, a.scale_fmin);
   double logdet = live ? a.logdet[w] : 0.0;
   const int n_meas = a.measure_every > 0 ? a.n_sweeps / a.measure_every : 0;
-  // lanes of one electron in the local energy: Q lanes share its pair terms
-  int PE = 1;
-  while (PE < P && PE < NE) PE <<= 1;
-  const int Q = P / PE, le = lane & (PE - 1), lq = lane / PE;
+  // local energy: PE electrons at a time, Q lanes share an electron's three-body terms
+  const int PE = min(P, NE), Q = P / PE, le = lane % PE, lq = lane / PE;
   int nacc = 0, meas = 0;
   for (int t = 0; t < a.n_sweeps; ++t) {
     const uint32_t gstep = (uint32_t)(a.step_base + t);
     if (P > 1) {
-      nacc += oq_sweep_lanes<NOCC, T, Real, B>(a, S, SP, C, pos, Ai, rI, WT, lane, P, live, w,
+      nacc += oq_sweep_lanes<NOCC, T, Real, B>(a, S, SP, C, pos, Ai, rI, lane, P, live, w,
                                                gstep, step, pf, logdet);
     } else if (live) {
       for (int e = 0; e < NE; ++e) {
@@ -1416,8 +1420,8 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
         uint32_t ub;
         oq_move_normals(a.seed, w, gstep, (uint32_t)e, nf, ub);
         const T u = oq_uniform<T>(ub);
-        const double ox = pos[(3 * e) * WT], oy = pos[(3 * e + 1) * WT],
-                     oz = pos[(3 * e + 2) * WT];
+        const double ox = pos[3 * e], oy = pos[3 * e + 1],
+                     oz = pos[3 * e + 2];
         double nx, ny, nz;
         T mul = (T)1, lx = (T)0;
         if (a.proposal == 0) {
@@ -1427,7 +1431,7 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
         } else {
           oq_scaled_propose_t<T>(S, ox, oy, oz, nf, pf, nx, ny, nz, mul, lx);
         }
-        nacc += oq_try_move_s<NOCC, T, Real, B>(S, S, SP, C, pos, WT, Ai, WT, e, nx, ny, nz, lx,
+        nacc += oq_try_move_s<NOCC, T, Real, B>(S, S, SP, C, pos, 1, Ai, 1, e, nx, ny, nz, lx,
                                                 mul, u, logdet);
       }
     }
@@ -1439,32 +1443,34 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
     if (sizeof(T) == 4) {
       if (live && lq == 0)
         for (int e = le; e < NE; e += PE)
-          oq_eloc_electron<NOCC, T, Real, B>(S, S, SP, C, pos, (size_t)WT, Ai, (size_t)WT, e, see,
+          oq_eloc_electron<NOCC, T, Real, B>(S, S, SP, C, pos, 1, Ai, 1, e, see,
                                              sen, slp, sg2);
     } else {
       // one electron per lane; its three-body terms split over Q lanes
       for (int e0 = 0; e0 < NE; e0 += PE) {
         const bool mine_e = live && e0 + le < NE;
         const int e = mine_e ? e0 + le : 0, s = e & 1, i = e >> 1;
-        const double xe = pos[(3 * e) * WT], ye = pos[(3 * e + 1) * WT],
-                     ze = pos[(3 * e + 2) * WT];
+        const double xe = pos[3 * e], ye = pos[3 * e + 1],
+                     ze = pos[3 * e + 2];
         T jx = (T)0, jy = (T)0, jz = (T)0, jl = (T)0;
         if (OQ_HAS_J3(S)) {
-          if (mine_e) oq_j3_vgl_part<NE, T>(S, pos, WT, e, lq, Q, xe, ye, ze, jx, jy, jz, jl);
-          for (int o = PE; o < P; o <<= 1) {
-            jx += __shfl_xor_sync(0xffffffffu, jx, o);
-            jy += __shfl_xor_sync(0xffffffffu, jy, o);
-            jz += __shfl_xor_sync(0xffffffffu, jz, o);
-            jl += __shfl_xor_sync(0xffffffffu, jl, o);
+          T gx = (T)0, gy = (T)0, gz = (T)0, gl = (T)0;
+          if (mine_e && lq < Q)
+            oq_j3_vgl_part<NE, T>(S, pos, e, lq, Q, xe, ye, ze, gx, gy, gz, gl);
+          for (int k = 0; k < Q; ++k) {
+            jx += __shfl_sync(0xffffffffu, gx, le + k * PE, P);
+            jy += __shfl_sync(0xffffffffu, gy, le + k * PE, P);
+            jz += __shfl_sync(0xffffffffu, gz, le + k * PE, P);
+            jl += __shfl_sync(0xffffffffu, gl, le + k * PE, P);
           }
         }
         if (mine_e && lq == 0) {
           T ac[NOCC];
 #pragma unroll
-          for (int m = 0; m < NOCC; ++m) ac[m] = (T)Ai[((s * NOCC + m) * NOCC + i) * WT];
+          for (int m = 0; m < NOCC; ++m) ac[m] = (T)Ai[(s * NOCC + m) * NOCC + i];
           T gx, gy, gz, lp;
           B::template mo_vgl_contract<T, Real>(S, SP, C, xe, ye, ze, ac, gx, gy, gz, lp);
-          oq_jastrow_vgl_coulomb<NE, T>(S, S, pos, (size_t)WT, e, xe, ye, ze, jx, jy, jz, jl, see,
+          oq_jastrow_vgl_coulomb<NE, T>(S, S, pos, 1, e, xe, ye, ze, jx, jy, jz, jl, see,
                                         sen, false);
           const double sx = (double)gx, sy = (double)gy, sz = (double)gz;
           const double Gx = sx + (double)jx, Gy = sy + (double)jy, Gz = sz + (double)jz;
@@ -1508,17 +1514,17 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
     double* x = a.X + (size_t)w0 * 3 * NE;
     for (int q = tid; q < cnt * 3 * NE; q += blockDim.x) {
       const int j = q / (3 * NE), k = q - j * 3 * NE;
-      x[q] = pos0[k * WT + j];
+      x[q] = pos0[j * PP + k];
     }
     Real* gA = reinterpret_cast<Real*>(a.ainv);
     for (int q = tid; q < 2 * NN * WT; q += blockDim.x) {
       const int k = q / WT, j = q - k * WT;
-      if (j < cnt) gA[(size_t)k * W + w0 + j] = Ai0[q];
+      if (j < cnt) gA[(size_t)k * W + w0 + j] = Ai0[j * AP + k];
     }
     if (a.pos)
       for (int q = tid; q < 3 * NE * WT; q += blockDim.x) {
         const int k = q / WT, j = q - k * WT;
-        if (j < cnt) a.pos[(size_t)k * W + w0 + j] = pos0[q];
+        if (j < cnt) a.pos[(size_t)k * W + w0 + j] = pos0[j * PP + k];
       }
   }
   if (live && lane == 0) a.logdet[w] = logdet;
