@@ -682,7 +682,7 @@ int oqmc_set_mlp_groups(oqmc_ctx* ctx, int groups) {
   return OQ_OK;
 }
 
-// Jastrow-parameter derivatives, one thread per walker, FP64: d ln|psi|/dp
+// Jastrow-parameter derivatives, FP64: d ln|psi|/dp
 // and dE_L/dp for p = (J2 like a, like b, unlike a, unlike b, J1 a_I, b_I per
 // atom), from the positions and the full gradient G of ln|psi| (oqmc_eval).
 // For u = a r/(1+b r): du/da = r/den, du/db = -a r^2/den^2; u' = a/den^2,
@@ -699,72 +699,79 @@ __device__ __forceinline__ void oq_pade_dp(double a, double b, double r, double 
   dL[1] = dupp1 + 2.0 * dup[1] / r;
 }
 
-// B-spline parameters: P_q is coefficient q+1 and coefficient 0 is
-// P_1 - 2 dr cusp, so a term at distance r in knot interval i touches the
-// parameters of coefficients i..i+3 (and P_1 through coefficient 0).
-__device__ __forceinline__ void oq_bs_param_add(const OqSystem& S, const double* c, int n,
-                                                double dinv, double rcut, double r, double gd,
-                                                bool half, double* dl, double* de) {
-  if (!(r < rcut)) return;
-  double t;
-  const int i = oq_bs_index<double>(r * dinv, n, t);
-  const double t2 = t * t, t3 = t2 * t, s6 = 1.0 / 6.0;
-  const double w[4] = {s6 * (-t3 + 3 * t2 - 3 * t + 1), s6 * (3 * t3 - 6 * t2 + 4),
-                       s6 * (-3 * t3 + 3 * t2 + 3 * t + 1), s6 * t3};
-  const double w1[4] = {s6 * dinv * (-3 * t2 + 6 * t - 3), s6 * dinv * (9 * t2 - 12 * t),
-                        s6 * dinv * (-9 * t2 + 6 * t + 3), s6 * dinv * 3 * t2};
-  const double w2[4] = {s6 * dinv * dinv * (-6 * t + 6), s6 * dinv * dinv * (18 * t - 12),
-                        s6 * dinv * dinv * (-18 * t + 6), s6 * dinv * dinv * 6 * t};
-  (void)c;
-  for (int k = 0; k < 4; ++k) {
-    const int idx = i + k;
-    const int q = idx == 0 ? 1 : idx - 1;      // coefficient 0 depends on P_1
-    if (q < 0 || q >= n) continue;
-    const double dL = w2[k] + 2.0 * w1[k] / r;
-    dl[q] += w[k];
-    de[q] -= half ? 0.5 * (dL + 2.0 * w1[k] * gd) : dL + w1[k] * gd;
-  }
+// One warp per walker.  Every parameter belongs to one lane (or is summed over
+// the lanes by shuffles), so nothing is added to global memory: with one
+// thread per walker each three-body term read and wrote the derivatives of
+// all its gammas there (walker_derivatives of H2O with three-body orders 2 and
+// 2, 2,048 walkers: 4,492 us in all, 1,320 now with the fixed-order three-body
+// polynomials of the evaluation, most of it host time).
+#define OQ_PD_WARPS 4
+// doubles of one listed three-body term: see oq_pd_j3
+#define OQ_PD_GEO 16
+
+__device__ __forceinline__ double oq_warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
 }
 
-__device__ void oq_param_derivs_bspline(const OqSystem& S, const double* x, const double* g,
-                                        int n_e, double* dl, double* de) {
-  int base = 4 + 2 * S.natm;
-  if (S.has_bs2) {
-    for (int i = 0; i < n_e; ++i)
-      for (int j = i + 1; j < n_e; ++j) {
-        const double dx = x[3 * i] - x[3 * j], dy = x[3 * i + 1] - x[3 * j + 1],
-                     dz = x[3 * i + 2] - x[3 * j + 2];
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        const double gd = ((g[3 * i] - g[3 * j]) * dx + (g[3 * i + 1] - g[3 * j + 1]) * dy +
-                           (g[3 * i + 2] - g[3 * j + 2]) * dz) / r;
-        const bool like = (i & 1) == (j & 1);
-        if (like)
-          oq_bs_param_add(S, S.bs2_like, S.bs2_n_like, S.bs2_dinv_like, S.bs2_rcut, r, gd, false,
-                          dl + base, de + base);
-        else
-          oq_bs_param_add(S, S.bs2_unlike, S.bs2_n_unlike, S.bs2_dinv_unlike, S.bs2_rcut, r, gd,
-                          false, dl + base + S.bs2_n_like, de + base + S.bs2_n_like);
-      }
-    base += S.bs2_n_like + S.bs2_n_unlike;
+// Pair p = 0, 1, ... of the list (0,1), (0,2), (1,2), (0,3), ...: i < j.
+__device__ __forceinline__ void oq_pair_of(int p, int& i, int& j) {
+  j = (int)((1.0f + sqrtf(1.0f + 8.0f * (float)p)) * 0.5f);
+  while (j * (j - 1) / 2 > p) --j;
+  while (j * (j + 1) / 2 <= p) ++j;
+  i = p - j * (j - 1) / 2;
+}
+
+// Weight of coefficient k (value, first and second derivative) in the spline
+// at r, see oq_bs_val; false when its knots do not reach r.
+__device__ __forceinline__ bool oq_bs_weight(double r, double dinv, int n, int k, double& w,
+                                             double& w1, double& w2) {
+  double t;
+  const int i = oq_bs_index<double>(r * dinv, n, t);
+  const double t2 = t * t, t3 = t2 * t, s6 = 1.0 / 6.0, s61 = s6 * dinv, s62 = s61 * dinv;
+  switch (k - i) {
+    case 0:
+      w = s6 * (-t3 + 3 * t2 - 3 * t + 1); w1 = s61 * (-3 * t2 + 6 * t - 3); w2 = s62 * (-6 * t + 6);
+      break;
+    case 1:
+      w = s6 * (3 * t3 - 6 * t2 + 4); w1 = s61 * (9 * t2 - 12 * t); w2 = s62 * (18 * t - 12);
+      break;
+    case 2:
+      w = s6 * (-3 * t3 + 3 * t2 + 3 * t + 1); w1 = s61 * (-9 * t2 + 6 * t + 3);
+      w2 = s62 * (-18 * t + 6);
+      break;
+    case 3:
+      w = s6 * t3; w1 = s61 * 3 * t2; w2 = s62 * 6 * t;
+      break;
+    default:
+      return false;
   }
-  if (S.has_bs1) {
-    int tbase[OQ_MAX_BST];
-    for (int t = 0, b = base; t < OQ_MAX_BST; ++t) {
-      tbase[t] = b;
-      b += S.bs1_n[t];
-    }
-    for (int I = 0; I < S.natm; ++I) {
-      const int ty = S.bs1_type[I];
-      if (ty < 0) continue;
-      for (int e = 0; e < n_e; ++e) {
-        const double dx = x[3 * e] - S.nuc[I][0], dy = x[3 * e + 1] - S.nuc[I][1],
-                     dz = x[3 * e + 2] - S.nuc[I][2];
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        const double gd = (g[3 * e] * dx + g[3 * e + 1] * dy + g[3 * e + 2] * dz) / r;
-        oq_bs_param_add(S, S.bs1_c[ty], S.bs1_n[ty], S.bs1_dinv[ty], S.bs1_rcut[ty], r, gd, true,
-                        dl + tbase[ty], de + tbase[ty]);
+  return true;
+}
+
+// B-spline parameters of one block (n parameters, at dl, de): P_q is
+// coefficient q + 1, and coefficient 0 is P_1 - 2 dr cusp, so it adds to P_1.
+// Lane q sums its parameter over the cnt listed terms (r, gd) at list, in
+// list order; half: the one-body form.
+__device__ __forceinline__ void oq_pd_bspline(const double* list, int cnt, int n, double dinv,
+                                              double rcut, bool half, int lane, double* dl,
+                                              double* de) {
+  for (int q = lane; q < n; q += 32) {
+    double sl = 0.0, se = 0.0;
+    for (int t = 0; t < cnt; ++t) {
+      const double r = list[2 * t], gd = list[2 * t + 1];
+      if (!(r < rcut)) continue;
+      for (int idx = q + 1; idx >= 0; idx = (q == 1 && idx == 2) ? 0 : -1) {
+        double w, w1, w2;
+        if (!oq_bs_weight(r, dinv, n, idx, w, w1, w2)) continue;
+        const double dL = w2 + 2.0 * w1 / r;
+        sl += w;
+        se -= half ? 0.5 * (dL + 2.0 * w1 * gd) : dL + w1 * gd;
       }
     }
+    dl[q] = sl;
+    de[q] = se;
   }
 }
 
@@ -774,103 +781,135 @@ __host__ __device__ static inline int j3_unique(const OqSystem& S) {
   return (S.j3_nI + 1) * (S.j3_nI + 2) / 2 * (S.j3_nE + 1);
 }
 
-__device__ __forceinline__ double oq_ipow(double x, int k) {
-  double v = 1.0;
-  for (int i = 0; i < k; ++i) v *= x;
-  return v;
-}
-
-// phi = r1^l r2^m r12^n (+ r1^m r2^l r12^n for l != m) and its partials
-// with electron 1 moving: phi, d/dr1, d/dr12, d2/dr1^2, d2/dr12^2, d2/dr1dr12.
-__device__ __forceinline__ void oq_j3_basis(int l, int m, int n, double r1, double r2, double r12,
-                                            double f[6]) {
-  for (int k = 0; k < 6; ++k) f[k] = 0.0;
-  const double e0 = oq_ipow(r12, n), e1 = n >= 1 ? n * oq_ipow(r12, n - 1) : 0.0,
-               e2 = n >= 2 ? n * (n - 1) * oq_ipow(r12, n - 2) : 0.0;
-  for (int pass = 0; pass < (l != m ? 2 : 1); ++pass) {
-    const int a = pass ? m : l, b = pass ? l : m;
-    const double p0 = oq_ipow(r1, a), p1 = a >= 1 ? a * oq_ipow(r1, a - 1) : 0.0,
-                 p2 = a >= 2 ? a * (a - 1) * oq_ipow(r1, a - 2) : 0.0, q = oq_ipow(r2, b);
-    f[0] += p0 * q * e0;
-    f[1] += p1 * q * e0;
-    f[2] += p0 * q * e1;
-    f[3] += p2 * q * e0;
-    f[4] += p0 * q * e2;
-    f[5] += p1 * q * e1;
-  }
+// x^k and its first and second derivatives; x2, x1, x0 = x^(k-2), x^(k-1), x^k.
+__device__ __forceinline__ void oq_pow_d(double x, int k, double& p0, double& p1, double& p2) {
+  double x2 = 0.0, x1 = k >= 1 ? 1.0 : 0.0, x0 = 1.0;
+  if (k >= 2) x2 = 1.0;
+  for (int i = 2; i < k; ++i) x2 *= x;
+  if (k >= 2) x1 = x2 * x;
+  if (k >= 1) x0 = x1 * x;
+  p0 = x0;
+  p1 = k * x1;
+  p2 = k * (k - 1) * x2;
 }
 
 // d log|psi| / d gamma and d E_L / d gamma of the three-body Jastrow for the
 // unique gammas of every present block (types in order, like then unlike),
 // starting at raw slot `base`.  J3 = -sum u is linear in the gammas, so each
 // gamma's derivative is the J3 value, gradient and Laplacian with that
-// gamma's monomial in place of the polynomial.
-__device__ void oq_param_derivs_j3(const OqSystem& S, const double* x, const double* g, int n_e,
-                                   int base, double* dl, double* de) {
-  const int NG = j3_unique(S);
+// gamma's monomial (r1^l r2^m + r1^m r2^l for l != m) r12^n in place of the
+// polynomial.  For 32 pairs and one nucleus at a time the lanes form the
+// geometry of a term each and list the terms inside the cutoff in shared
+// memory; then every lane goes through the list with its own monomial.
+__device__ void oq_pd_j3(const OqSystem& S, const double* x, const double* g, int n_e, int base,
+                         int lane, double* geo, double* dl, double* de) {
+  const int NG = j3_unique(S), np = n_e * (n_e - 1) / 2;
   const double L = S.j3_L;
-  int boff[OQ_MAX_BST][2];
-  for (int t = 0, o = base; t < OQ_MAX_BST; ++t)
-    for (int b = 0; b < 2; ++b) {
-      boff[t][b] = S.j3_on[t][b] ? o : -1;
-      if (S.j3_on[t][b]) o += NG;
-    }
-  for (int I = 0; I < S.natm; ++I) {
-    const int ty = S.j3_type[I];
-    if (ty < 0) continue;
-    for (int i = 0; i < n_e; ++i)
-      for (int j = i + 1; j < n_e; ++j) {
-        const int blk = (i ^ j) & 1;
-        const int off = boff[ty][blk];
-        if (off < 0) continue;
-        double di[3], dj[3], dij[3];
-        for (int c = 0; c < 3; ++c) {
-          di[c] = x[3 * i + c] - S.nuc[I][c];
-          dj[c] = x[3 * j + c] - S.nuc[I][c];
-          dij[c] = x[3 * i + c] - x[3 * j + c];
-        }
-        const double ri = sqrt(di[0] * di[0] + di[1] * di[1] + di[2] * di[2]);
-        const double rj = sqrt(dj[0] * dj[0] + dj[1] * dj[1] + dj[2] * dj[2]);
-        if (!(ri < L) || !(rj < L)) continue;
-        const double r12 = sqrt(dij[0] * dij[0] + dij[1] * dij[1] + dij[2] * dij[2]);
-        // G_a . e_aI and G_a . e_ab for the two electrons, and the cosines
-        double gi1 = 0, gie = 0, gj1 = 0, gje = 0, ci = 0, cj = 0;
-        for (int c = 0; c < 3; ++c) {
-          const double ei = di[c] / ri, ej = dj[c] / rj, e = dij[c] / r12;
-          gi1 += g[3 * i + c] * ei;
-          gie += g[3 * i + c] * e;
-          gj1 += g[3 * j + c] * ej;
-          gje -= g[3 * j + c] * e;
-          ci += ei * e;
-          cj -= ej * e;
-        }
-        // envelope (r_1I - L)^3 (r_2I - L)^3 in each electron's frame
-        const double si = ri - L, sj = rj - L;
-        const double E = si * si * si * sj * sj * sj;
-        const double Ei1 = 3.0 * si * si * sj * sj * sj, Ei11 = 6.0 * si * sj * sj * sj;
-        const double Ej1 = 3.0 * sj * sj * si * si * si, Ej11 = 6.0 * sj * si * si * si;
-        int u = 0;
-        for (int m = 0; m <= S.j3_nI; ++m)
-          for (int l = m; l <= S.j3_nI; ++l)
-            for (int n = 0; n <= S.j3_nE; ++n, ++u) {
-              double fi[6], fj[6];
-              oq_j3_basis(l, m, n, ri, rj, r12, fi);
-              oq_j3_basis(l, m, n, rj, ri, r12, fj);
-              // partials of f = phi * E with each electron as particle 1
-              const double a1 = fi[1] * E + fi[0] * Ei1, ae = fi[2] * E;
-              const double a11 = fi[3] * E + 2.0 * fi[1] * Ei1 + fi[0] * Ei11, aee = fi[4] * E;
-              const double a1e = fi[5] * E + fi[2] * Ei1;
-              const double b1 = fj[1] * E + fj[0] * Ej1, be = fj[2] * E;
-              const double b11 = fj[3] * E + 2.0 * fj[1] * Ej1 + fj[0] * Ej11, bee = fj[4] * E;
-              const double b1e = fj[5] * E + fj[2] * Ej1;
-              // J3 = -sum f: d lap and G . dG of both electrons
-              const double dlap_i = -(a11 + 2.0 * a1 / ri + aee + 2.0 * ae / r12 + 2.0 * a1e * ci);
-              const double dlap_j = -(b11 + 2.0 * b1 / rj + bee + 2.0 * be / r12 + 2.0 * b1e * cj);
-              const double gdg = -(a1 * gi1 + ae * gie) - (b1 * gj1 + be * gje);
-              dl[off + u] -= fi[0] * E;
-              de[off + u] -= 0.5 * (dlap_i + dlap_j + 2.0 * gdg);
-            }
+  for (int ty = 0, off = base; ty < OQ_MAX_BST; ++ty) {
+    if (!S.j3_on[ty][0] && !S.j3_on[ty][1]) continue;
+    for (int u0 = 0; u0 < NG; u0 += 32) {
+      // this lane's monomial
+      int l = 0, m = 0, n = 0;
+      {
+        int u = u0 + lane < NG ? u0 + lane : 0;
+        while (u >= (S.j3_nI + 1 - m) * (S.j3_nE + 1)) u -= (S.j3_nI + 1 - m++) * (S.j3_nE + 1);
+        l = m + u / (S.j3_nE + 1);
+        n = u % (S.j3_nE + 1);
       }
+      double sl[2] = {0.0, 0.0}, se[2] = {0.0, 0.0};
+      for (int I = 0; I < S.natm; ++I) {
+        if (S.j3_type[I] != ty) continue;
+        for (int p0 = 0; p0 < np; p0 += 32) {
+          int i = 0, j = 1;
+          bool in = p0 + lane < np;
+          if (in) oq_pair_of(p0 + lane, i, j);
+          const int blk = (i ^ j) & 1;
+          double di[3], dj[3], dij[3];
+          for (int c = 0; c < 3; ++c) {
+            di[c] = x[3 * i + c] - S.nuc[I][c];
+            dj[c] = x[3 * j + c] - S.nuc[I][c];
+            dij[c] = x[3 * i + c] - x[3 * j + c];
+          }
+          const double ri = sqrt(di[0] * di[0] + di[1] * di[1] + di[2] * di[2]);
+          const double rj = sqrt(dj[0] * dj[0] + dj[1] * dj[1] + dj[2] * dj[2]);
+          in = in && S.j3_on[ty][blk] && ri < L && rj < L;
+          const unsigned list = __ballot_sync(0xffffffffu, in);
+          const unsigned likes = __ballot_sync(0xffffffffu, in && blk == 0);
+          if (list == 0u) continue;
+          if (in) {
+            const double r12 = sqrt(dij[0] * dij[0] + dij[1] * dij[1] + dij[2] * dij[2]);
+            // G_a . e_aI and G_a . e_ab for the two electrons, and the cosines
+            double gi1 = 0, gie = 0, gj1 = 0, gje = 0, ci = 0, cj = 0;
+            for (int c = 0; c < 3; ++c) {
+              const double ei = di[c] / ri, ej = dj[c] / rj, e = dij[c] / r12;
+              gi1 += g[3 * i + c] * ei;
+              gie += g[3 * i + c] * e;
+              gj1 += g[3 * j + c] * ej;
+              gje -= g[3 * j + c] * e;
+              ci += ei * e;
+              cj -= ej * e;
+            }
+            const double si = ri - L, sj = rj - L;
+            double* q = geo + lane * OQ_PD_GEO;
+            q[0] = ri; q[1] = rj; q[2] = r12;
+            // envelope (r_1I - L)^3 (r_2I - L)^3 and its derivatives over it
+            q[3] = si * si * si * sj * sj * sj;
+            q[4] = 3.0 * si * si * sj * sj * sj; q[5] = 6.0 * si * sj * sj * sj;
+            q[6] = 3.0 * sj * sj * si * si * si; q[7] = 6.0 * sj * si * si * si;
+            q[8] = gi1; q[9] = gj1; q[10] = gie + gje;
+            q[11] = ci; q[12] = cj;
+            q[13] = 2.0 / ri; q[14] = 2.0 / rj; q[15] = 2.0 / r12;
+          }
+          __syncwarp();
+          for (unsigned todo = list; todo; todo &= todo - 1) {
+            const int t = __ffs(todo) - 1;
+            const double* q = geo + t * OQ_PD_GEO;
+            const double a = q[0], b = q[1], r12 = q[2], E = q[3];
+            double A, A1, A2, D, D1, D2, e0, e1, e2;
+            oq_pow_d(a, l, A, A1, A2);
+            oq_pow_d(b, m, D, D1, D2);
+            oq_pow_d(r12, n, e0, e1, e2);
+            double f = A * D, f1 = A1 * D, f11 = A2 * D, g1 = A * D1, g11 = A * D2;
+            if (l != m) {
+              oq_pow_d(a, m, A, A1, A2);
+              oq_pow_d(b, l, D, D1, D2);
+              f += A * D; f1 += A1 * D; f11 += A2 * D; g1 += A * D1; g11 += A * D2;
+            }
+            // partials of (monomial x envelope) with each electron as particle 1
+            const double Ei1 = q[4], Ej1 = q[6];
+            const double v = f * e0 * E, ae = f * e1 * E, aee = f * e2 * E;
+            const double a1 = e0 * (f1 * E + f * Ei1), b1 = e0 * (g1 * E + f * Ej1);
+            const double a11 = e0 * (f11 * E + 2.0 * f1 * Ei1 + f * q[5]);
+            const double b11 = e0 * (g11 * E + 2.0 * g1 * Ej1 + f * q[7]);
+            const double a1e = e1 * (f1 * E + f * Ei1), b1e = e1 * (g1 * E + f * Ej1);
+            // J3 = -sum f: d lap and G . dG of both electrons
+            const double lap = a11 + a1 * q[13] + b11 + b1 * q[14] + 2.0 * (aee + ae * q[15]) +
+                               2.0 * (a1e * q[11] + b1e * q[12]);
+            const double gdg = a1 * q[8] + b1 * q[9] + ae * q[10];
+            const int blk_t = (likes >> t) & 1u ? 0 : 1;
+            const double dE = 0.5 * lap + gdg;
+            sl[0] -= blk_t ? 0.0 : v;
+            sl[1] -= blk_t ? v : 0.0;
+            se[0] += blk_t ? 0.0 : dE;
+            se[1] += blk_t ? dE : 0.0;
+          }
+          __syncwarp();
+        }
+      }
+      if (u0 + lane < NG) {
+        int o = off + u0 + lane;
+        if (S.j3_on[ty][0]) {
+          dl[o] = sl[0];
+          de[o] = se[0];
+          o += NG;
+        }
+        if (S.j3_on[ty][1]) {
+          dl[o] = sl[1];
+          de[o] = se[1];
+        }
+      }
+    }
+    off += NG * (S.j3_on[ty][0] + S.j3_on[ty][1]);
   }
 }
 
@@ -884,63 +923,142 @@ static int param_count_of(const OqSystem& S) {
   return n;
 }
 
-__global__ void k_param_derivs(const OqSystem* __restrict__ gsys, const double* __restrict__ X,
-                               const double* __restrict__ G, int W, int n_e,
-                               double* __restrict__ dlog, double* __restrict__ del) {
-  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+// Shared memory of one warp: positions and gradient [3 n_e] each, the distance
+// and gradient-projection list (r, gd) of the electron pairs or of one atom's
+// electrons, and the listed three-body terms.
+static size_t param_derivs_smem(const OqSystem& S) {
+  const size_t np = (size_t)S.n_e * (S.n_e - 1) / 2;
+  return sizeof(double) * (6 * (size_t)S.n_e + 2 * (np > (size_t)S.n_e ? np : S.n_e) +
+                           (S.has_j3 ? 32 * OQ_PD_GEO : 0));
+}
+
+__global__ void __launch_bounds__(32 * OQ_PD_WARPS)
+k_param_derivs(const OqSystem* __restrict__ gsys, const double* __restrict__ X,
+               const double* __restrict__ G, int W, int n_e, int n_raw, int warp_bytes,
+               double* __restrict__ dlog, double* __restrict__ del) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int w = blockIdx.x * OQ_PD_WARPS + warp;
   if (w >= W) return;
   const OqSystem& S = *gsys;
-  int n_raw = 4 + 2 * S.natm;
-  if (S.has_bs2) n_raw += S.bs2_n_like + S.bs2_n_unlike;
-  if (S.has_bs1)
-    for (int t = 0; t < OQ_MAX_BST; ++t) n_raw += S.bs1_n[t];
-  const int j3_base = n_raw;
-  if (S.has_j3)
-    for (int t = 0; t < OQ_MAX_BST; ++t) n_raw += j3_unique(S) * (S.j3_on[t][0] + S.j3_on[t][1]);
-  const double* x = X + (size_t)w * n_e * 3;
-  const double* g = G + (size_t)w * n_e * 3;
+  const int np = n_e * (n_e - 1) / 2, natm = S.natm;
+  double* x = reinterpret_cast<double*>(smem + (size_t)warp * warp_bytes);
+  double* g = x + 3 * n_e;
+  double* list = g + 3 * n_e;                    // pairs like first, then unlike
+  double* geo = list + 2 * max(np, n_e);
+  for (int k = lane; k < 3 * n_e; k += 32) {
+    x[k] = X[(size_t)w * n_e * 3 + k];
+    g[k] = G[(size_t)w * n_e * 3 + k];
+  }
   double* dl = dlog + (size_t)w * n_raw;
   double* de = del + (size_t)w * n_raw;
-  for (int k = 0; k < n_raw; ++k) { dl[k] = 0.0; de[k] = 0.0; }
-  if (S.has_j2) {
-    double al[4] = {0, 0, 0, 0}, ae[4] = {0, 0, 0, 0};
-    for (int i = 0; i < n_e; ++i)
-      for (int j = i + 1; j < n_e; ++j) {
-        const double dx = x[3 * i] - x[3 * j], dy = x[3 * i + 1] - x[3 * j + 1],
-                     dz = x[3 * i + 2] - x[3 * j + 2];
-        const double r = sqrt(dx * dx + dy * dy + dz * dz);
-        const double gd = ((g[3 * i] - g[3 * j]) * dx + (g[3 * i + 1] - g[3 * j + 1]) * dy +
-                           (g[3 * i + 2] - g[3 * j + 2]) * dz) / r;
-        const int o = ((i & 1) == (j & 1)) ? 0 : 2;
-        double du[2], dup[2], dL[2];
-        oq_pade_dp(S.j2[o], S.j2[o + 1], r, du, dup, dL);
-        for (int q = 0; q < 2; ++q) {
-          al[o + q] += du[q];
-          ae[o + q] -= dL[q] + dup[q] * gd;
-        }
+  __syncwarp();
+  // electron pairs: two sets, like then unlike, in pair order
+  const int h = n_e / 2, nlike = h * (h - 1);
+  double al[4] = {0, 0, 0, 0}, ae[4] = {0, 0, 0, 0};
+  int cl = 0, cu = 0;
+  for (int p0 = 0; p0 < np; p0 += 32) {
+    int i = 0, j = 1;
+    const bool in = p0 + lane < np;
+    if (in) oq_pair_of(p0 + lane, i, j);
+    const double dx = x[3 * i] - x[3 * j], dy = x[3 * i + 1] - x[3 * j + 1],
+                 dz = x[3 * i + 2] - x[3 * j + 2];
+    const double r = sqrt(dx * dx + dy * dy + dz * dz);
+    const double gd = ((g[3 * i] - g[3 * j]) * dx + (g[3 * i + 1] - g[3 * j + 1]) * dy +
+                       (g[3 * i + 2] - g[3 * j + 2]) * dz) / r;
+    const int blk = (i ^ j) & 1;
+    if (S.has_j2 && in) {
+      double du[2], dup[2], dL[2];
+      oq_pade_dp(S.j2[2 * blk], S.j2[2 * blk + 1], r, du, dup, dL);
+      for (int q = 0; q < 2; ++q) {
+        const double e = dL[q] + dup[q] * gd;
+        al[q] += blk ? 0.0 : du[q];
+        al[2 + q] += blk ? du[q] : 0.0;
+        ae[q] -= blk ? 0.0 : e;
+        ae[2 + q] -= blk ? e : 0.0;
       }
-    for (int k = 0; k < 4; ++k) { dl[k] = al[k]; de[k] = ae[k]; }
+    }
+    const unsigned lk = __ballot_sync(0xffffffffu, in && !blk);
+    const unsigned un = __ballot_sync(0xffffffffu, in && blk);
+    const unsigned below = (1u << lane) - 1u;
+    if (in) {
+      const int at = blk ? nlike + cu + __popc(un & below) : cl + __popc(lk & below);
+      list[2 * at] = r;
+      list[2 * at + 1] = gd;
+    }
+    cl += __popc(lk);
+    cu += __popc(un);
   }
-  if (S.has_bs2 || S.has_bs1) oq_param_derivs_bspline(S, x, g, n_e, dl, de);
-  if (S.has_j3) oq_param_derivs_j3(S, x, g, n_e, j3_base, dl, de);
-  if (S.has_j1) {
-    for (int I = 0; I < S.natm; ++I) {
-      double sl0 = 0, sl1 = 0, se0 = 0, se1 = 0;
-      for (int e = 0; e < n_e; ++e) {
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const double sl = oq_warp_sum(al[k]), se = oq_warp_sum(ae[k]);
+    if (lane == k) {
+      dl[k] = sl;
+      de[k] = se;
+    }
+  }
+  __syncwarp();
+  int base = 4 + 2 * natm;
+  if (S.has_bs2) {
+    oq_pd_bspline(list, cl, S.bs2_n_like, S.bs2_dinv_like, S.bs2_rcut, false, lane, dl + base,
+                  de + base);
+    base += S.bs2_n_like;
+    oq_pd_bspline(list + 2 * nlike, cu, S.bs2_n_unlike, S.bs2_dinv_unlike, S.bs2_rcut, false,
+                  lane, dl + base, de + base);
+    base += S.bs2_n_unlike;
+  }
+  // electron-nucleus terms, one atom at a time; a B-spline block collects the
+  // atoms of its element, so it is summed into place
+  const int bs1_base = base;
+  if (S.has_bs1) {
+    for (int t = 0; t < OQ_MAX_BST; ++t) base += S.bs1_n[t];
+    for (int k = bs1_base + lane; k < base; k += 32) dl[k] = de[k] = 0.0;
+  }
+  for (int I = 0; I < natm; ++I) {
+    const int ty = S.has_bs1 ? S.bs1_type[I] : -1;
+    double sl[2] = {0.0, 0.0}, se[2] = {0.0, 0.0};
+    if (S.has_j1 || ty >= 0) {
+      __syncwarp();
+      if (lane < n_e) {
+        const int e = lane;                       // n_e <= 32
         const double dx = x[3 * e] - S.nuc[I][0], dy = x[3 * e + 1] - S.nuc[I][1],
                      dz = x[3 * e + 2] - S.nuc[I][2];
         const double r = sqrt(dx * dx + dy * dy + dz * dz);
         const double gd = (g[3 * e] * dx + g[3 * e + 1] * dy + g[3 * e + 2] * dz) / r;
-        double du[2], dup[2], dL[2];
-        oq_pade_dp(S.j1a[I], S.j1b[I], r, du, dup, dL);
-        sl0 += du[0]; sl1 += du[1];
-        se0 -= 0.5 * (dL[0] + 2.0 * dup[0] * gd);
-        se1 -= 0.5 * (dL[1] + 2.0 * dup[1] * gd);
+        list[2 * e] = r;
+        list[2 * e + 1] = gd;
+        if (S.has_j1) {
+          double du[2], dup[2], dL[2];
+          oq_pade_dp(S.j1a[I], S.j1b[I], r, du, dup, dL);
+          for (int q = 0; q < 2; ++q) {
+            sl[q] = du[q];
+            se[q] = -0.5 * (dL[q] + 2.0 * dup[q] * gd);
+          }
+        }
       }
-      dl[4 + 2 * I] = sl0; dl[5 + 2 * I] = sl1;
-      de[4 + 2 * I] = se0; de[5 + 2 * I] = se1;
+      __syncwarp();
+    }
+    for (int q = 0; q < 2; ++q) {
+      const double a = oq_warp_sum(sl[q]), b = oq_warp_sum(se[q]);
+      if (lane == q) {
+        dl[4 + 2 * I + q] = a;
+        de[4 + 2 * I + q] = b;
+      }
+    }
+    if (ty >= 0) {
+      int off = bs1_base;
+      for (int t = 0; t < ty; ++t) off += S.bs1_n[t];
+      // lane q owns parameter q (at most OQ_MAX_BSC of them): adds its own sum
+      double tl = 0.0, te = 0.0;
+      const int n = S.bs1_n[ty];
+      double* pl = dl + off;
+      double* pe = de + off;
+      if (lane < n) { tl = pl[lane]; te = pe[lane]; }
+      oq_pd_bspline(list, n_e, n, S.bs1_dinv[ty], S.bs1_rcut[ty], true, lane, pl, pe);
+      if (lane < n) { pl[lane] += tl; pe[lane] += te; }
     }
   }
+  if (S.has_j3) oq_pd_j3(S, x, g, n_e, base, lane, geo, dl, de);
 }
 
 int oqmc_param_count(const oqmc_ctx* ctx) { return ctx ? param_count_of(ctx->hsys) : OQ_ERR_ARG; }
@@ -951,8 +1069,13 @@ int oqmc_param_derivs(oqmc_ctx* ctx, const double* X, int W, const double* grad,
   if (W < 0 || (W > 0 && (!X || !grad || !dlogpsi || !dEL)))
     return set_err(ctx, OQ_ERR_ARG, "bad arguments%s");
   if (W == 0) return OQ_OK;
-  k_param_derivs<<<(W + 127) / 128, 128, 0, (cudaStream_t)stream>>>(ctx->d_sys, X, grad, W,
-                                                                     ctx->n_e, dlogpsi, dEL);
+  const size_t wbytes = param_derivs_smem(ctx->hsys), sm = OQ_PD_WARPS * wbytes;
+  if (sm > 48 * 1024)
+    OQ_CUDA(ctx, cudaFuncSetAttribute(k_param_derivs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sm));
+  k_param_derivs<<<(W + OQ_PD_WARPS - 1) / OQ_PD_WARPS, 32 * OQ_PD_WARPS, sm,
+                   (cudaStream_t)stream>>>(ctx->d_sys, X, grad, W, ctx->n_e,
+                                           param_count_of(ctx->hsys), (int)wbytes, dlogpsi, dEL);
   OQ_CUDA(ctx, cudaGetLastError());
   return OQ_OK;
 }

@@ -353,13 +353,13 @@ __device__ __forceinline__ T oq_j3_u(const double* __restrict__ g, int nI, int n
   return P * e * e * e;
 }
 
-// Partials of u with electron 1 as the moving particle (_eval_eeI_poly_vgl,
+// Partials of u (and, asked for, u) with electron 1 as the moving particle (_eval_eeI_poly_vgl,
 // gto.py:508-604): u1 = du/dr_1I, ue = du/dr_12, u11, uee and the mixed u1e.
 // Horner in r_12, r_2I, r_1I carrying first and second derivatives.
 template <typename T>
 __device__ __forceinline__ void oq_j3_partials(const double* __restrict__ g, int nI, int nE, T L,
                                                T r12, T r1, T r2, T& u1, T& ue, T& u11, T& uee,
-                                               T& u1e) {
+                                               T& u1e, T* u = nullptr) {
   T P = (T)0, P1 = (T)0, P11 = (T)0, Q = (T)0, Q1 = (T)0, R = (T)0;
   for (int l = nI; l >= 0; --l) {
     T a = (T)0, b = (T)0, c = (T)0;
@@ -389,6 +389,7 @@ __device__ __forceinline__ void oq_j3_partials(const double* __restrict__ g, int
   u11 = P11 * E + (T)2 * P1 * E1 + P * E11;
   uee = R * E;
   u1e = Q1 * E + Q * E1;
+  if (u) *u = P * E;
 }
 
 // The same with the orders known to the compiler for the two usual ones (2, 2
@@ -403,13 +404,13 @@ __device__ __forceinline__ T oq_j3_u_n(const double* __restrict__ g, int nI, int
 template <typename T>
 __device__ __forceinline__ void oq_j3_partials_n(const double* __restrict__ g, int nI, int nE,
                                                  T L, T r12, T r1, T r2, T& u1, T& ue, T& u11,
-                                                 T& uee, T& u1e) {
+                                                 T& uee, T& u1e, T* u = nullptr) {
   if (nI == 2 && nE == 2) {
-    oq_j3_partials<T>(g, 2, 2, L, r12, r1, r2, u1, ue, u11, uee, u1e);
+    oq_j3_partials<T>(g, 2, 2, L, r12, r1, r2, u1, ue, u11, uee, u1e, u);
   } else if (nI == 3 && nE == 3) {
-    oq_j3_partials<T>(g, 3, 3, L, r12, r1, r2, u1, ue, u11, uee, u1e);
+    oq_j3_partials<T>(g, 3, 3, L, r12, r1, r2, u1, ue, u11, uee, u1e, u);
   } else {
-    oq_j3_partials<T>(g, nI, nE, L, r12, r1, r2, u1, ue, u11, uee, u1e);
+    oq_j3_partials<T>(g, nI, nE, L, r12, r1, r2, u1, ue, u11, uee, u1e, u);
   }
 }
 

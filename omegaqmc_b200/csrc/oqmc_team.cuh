@@ -453,9 +453,40 @@ static __device__ __noinline__ void oq_team_ext(const OqSystem* gS, const double
       }
     }
   if (S.has_j3) {
-    jv -= oq_j3_electron<double>(S, pos, (size_t)ps, NE, e, e + 1, xe, ye, ze);
-    if (VGL)
-      oq_j3_vgl_electron<double>(S, pos, (size_t)ps, NE, e, xe, ye, ze, gx, gy, gz, lp);
+    const int nI = S.j3_nI, nE = S.j3_nE, bsz = (nI + 1) * (nI + 1) * (nE + 1);
+    const double L = S.j3_L;
+    for (int I = 0; I < S.natm; ++I) {
+      const int ty = S.j3_type[I];
+      if (ty < 0) continue;
+      const double ax = xe - S.nuc[I][0], ay = ye - S.nuc[I][1], az = ze - S.nuc[I][2];
+      const double r1 = sqrt(ax * ax + ay * ay + az * az);
+      if (!(r1 < L)) continue;
+      for (int j = VGL ? 0 : e + 1; j < NE; ++j) {
+        const int blk = (e ^ j) & 1;
+        if (j == e || !S.j3_on[ty][blk]) continue;
+        const double xj = pos[(3 * j) * ps], yj = pos[(3 * j + 1) * ps], zj = pos[(3 * j + 2) * ps];
+        const double bx = xj - S.nuc[I][0], by = yj - S.nuc[I][1], bz = zj - S.nuc[I][2];
+        const double r2 = sqrt(bx * bx + by * by + bz * bz);
+        if (!(r2 < L)) continue;
+        const double dx = xe - xj, dy = ye - yj, dz = ze - zj;
+        const double r12 = sqrt(dx * dx + dy * dy + dz * dz);
+        const double* g = S.j3_gamma + (size_t)(2 * ty + blk) * bsz;
+        if (!VGL) {
+          jv -= oq_j3_u_n<double>(g, nI, nE, L, r12, r1, r2);
+          continue;
+        }
+        double u1, ue, u11, uee, u1e, u;
+        oq_j3_partials_n<double>(g, nI, nE, L, r12, r1, r2, u1, ue, u11, uee, u1e, &u);
+        if (j > e) jv -= u;
+        const double i1 = 1.0 / r1, i12 = 1.0 / r12;
+        const double t1 = u1 * i1, te = ue * i12;
+        gx -= t1 * ax + te * dx;
+        gy -= t1 * ay + te * dy;
+        gz -= t1 * az + te * dz;
+        lp -= u11 + 2.0 * t1 + uee + 2.0 * te +
+              2.0 * u1e * (ax * dx + ay * dy + az * dz) * (i1 * i12);
+      }
+    }
   }
   v[0] += jv; v[1] += gx; v[2] += gy; v[3] += gz; v[4] += lp;
 }
