@@ -348,6 +348,15 @@ int oqmc_param_count(const oqmc_ctx* ctx);
 int oqmc_param_derivs(oqmc_ctx* ctx, const double* walkers, int W, const double* grad,
                       double* dlogpsi, double* dEL, void* stream);
 
+/* The same in the caller's parameters: map is a device matrix (count, n_flat),
+ * row-major, and dlogpsi, dEL (W, n_flat) receive the raw derivatives times it
+ * (zero entries are left out, so a raw derivative that is not finite reaches
+ * only the parameters it belongs to).  e_loc (W) receives the local energies
+ * of eparts, oqmc_eval's (W, 4) output.  No counterpart in the reference. */
+int oqmc_param_derivs_mapped(oqmc_ctx* ctx, const double* walkers, int W, const double* grad,
+                             const double* eparts, const double* map, int n_flat, double* e_loc,
+                             double* dlogpsi, double* dEL, void* stream);
+
 /* ------------------------------------------------------------------------
  * Batched sampling: several molecules (contexts) of different electron and
  * basis counts share one persistent launch.  No counterpart in the

@@ -147,6 +147,8 @@ _SIGS = [
     ("oqmc_set_mlp_proposal", c_int, [c_void_p, c_void_p]),
     ("oqmc_set_mlp_groups", c_int, [c_void_p, c_int]),
     ("oqmc_param_count", c_int, [c_void_p]),
+    ("oqmc_param_derivs_mapped", c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
+                                         c_int, c_void_p, c_void_p, c_void_p, c_void_p]),
     ("oqmc_param_derivs", c_int, [c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p,
                                   c_void_p]),
 ]

@@ -925,17 +925,28 @@ static int param_count_of(const OqSystem& S) {
 
 // Shared memory of one warp: positions and gradient [3 n_e] each, the distance
 // and gradient-projection list (r, gd) of the electron pairs or of one atom's
-// electrons, and the listed three-body terms.
+// electrons, the raw derivatives, and the listed three-body terms.
 static size_t param_derivs_smem(const OqSystem& S) {
   const size_t np = (size_t)S.n_e * (S.n_e - 1) / 2;
   return sizeof(double) * (6 * (size_t)S.n_e + 2 * (np > (size_t)S.n_e ? np : S.n_e) +
-                           (S.has_j3 ? 32 * OQ_PD_GEO : 0));
+                           2 * (size_t)param_count_of(S) + (S.has_j3 ? 32 * OQ_PD_GEO : 0));
 }
+
+// Where the derivatives go: the raw ones to dlog, del (W, n_raw) when map is
+// null, else their products with map (n_raw, n_flat), zeros left out, to
+// dlog, del (W, n_flat).  e_loc (W), when set, receives eparts[., 3].
+struct OqPdOut {
+  double *dlog, *del;
+  const double* map;
+  int n_flat, pad;
+  const double* eparts;
+  double* e_loc;
+};
 
 __global__ void __launch_bounds__(32 * OQ_PD_WARPS)
 k_param_derivs(const OqSystem* __restrict__ gsys, const double* __restrict__ X,
                const double* __restrict__ G, int W, int n_e, int n_raw, int warp_bytes,
-               double* __restrict__ dlog, double* __restrict__ del) {
+               OqPdOut out) {
   extern __shared__ __align__(16) unsigned char smem[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int w = blockIdx.x * OQ_PD_WARPS + warp;
@@ -945,13 +956,13 @@ k_param_derivs(const OqSystem* __restrict__ gsys, const double* __restrict__ X,
   double* x = reinterpret_cast<double*>(smem + (size_t)warp * warp_bytes);
   double* g = x + 3 * n_e;
   double* list = g + 3 * n_e;                    // pairs like first, then unlike
-  double* geo = list + 2 * max(np, n_e);
+  double* dl = list + 2 * max(np, n_e);
+  double* de = dl + n_raw;
+  double* geo = de + n_raw;
   for (int k = lane; k < 3 * n_e; k += 32) {
     x[k] = X[(size_t)w * n_e * 3 + k];
     g[k] = G[(size_t)w * n_e * 3 + k];
   }
-  double* dl = dlog + (size_t)w * n_raw;
-  double* de = del + (size_t)w * n_raw;
   __syncwarp();
   // electron pairs: two sets, like then unlike, in pair order
   const int h = n_e / 2, nlike = h * (h - 1);
@@ -1059,9 +1070,43 @@ k_param_derivs(const OqSystem* __restrict__ gsys, const double* __restrict__ X,
     }
   }
   if (S.has_j3) oq_pd_j3(S, x, g, n_e, base, lane, geo, dl, de);
+  __syncwarp();
+  if (lane == 0 && out.e_loc) out.e_loc[w] = out.eparts[(size_t)w * 4 + 3];
+  if (!out.map) {
+    for (int k = lane; k < n_raw; k += 32) {
+      out.dlog[(size_t)w * n_raw + k] = dl[k];
+      out.del[(size_t)w * n_raw + k] = de[k];
+    }
+    return;
+  }
+  for (int p = lane; p < out.n_flat; p += 32) {
+    double sl = 0.0, se = 0.0;
+    for (int k = 0; k < n_raw; ++k) {
+      const double m = out.map[(size_t)k * out.n_flat + p];
+      if (m != 0.0) {
+        sl += m * dl[k];
+        se += m * de[k];
+      }
+    }
+    out.dlog[(size_t)w * out.n_flat + p] = sl;
+    out.del[(size_t)w * out.n_flat + p] = se;
+  }
 }
 
 int oqmc_param_count(const oqmc_ctx* ctx) { return ctx ? param_count_of(ctx->hsys) : OQ_ERR_ARG; }
+
+static int launch_param_derivs(oqmc_ctx* ctx, const double* X, int W, const double* grad,
+                               const OqPdOut& out, void* stream) {
+  const size_t wbytes = param_derivs_smem(ctx->hsys), sm = OQ_PD_WARPS * wbytes;
+  if (sm > 48 * 1024)
+    OQ_CUDA(ctx, cudaFuncSetAttribute(k_param_derivs, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)sm));
+  k_param_derivs<<<(W + OQ_PD_WARPS - 1) / OQ_PD_WARPS, 32 * OQ_PD_WARPS, sm,
+                   (cudaStream_t)stream>>>(ctx->d_sys, X, grad, W, ctx->n_e,
+                                           param_count_of(ctx->hsys), (int)wbytes, out);
+  OQ_CUDA(ctx, cudaGetLastError());
+  return OQ_OK;
+}
 
 int oqmc_param_derivs(oqmc_ctx* ctx, const double* X, int W, const double* grad, double* dlogpsi,
                       double* dEL, void* stream) {
@@ -1069,15 +1114,20 @@ int oqmc_param_derivs(oqmc_ctx* ctx, const double* X, int W, const double* grad,
   if (W < 0 || (W > 0 && (!X || !grad || !dlogpsi || !dEL)))
     return set_err(ctx, OQ_ERR_ARG, "bad arguments%s");
   if (W == 0) return OQ_OK;
-  const size_t wbytes = param_derivs_smem(ctx->hsys), sm = OQ_PD_WARPS * wbytes;
-  if (sm > 48 * 1024)
-    OQ_CUDA(ctx, cudaFuncSetAttribute(k_param_derivs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sm));
-  k_param_derivs<<<(W + OQ_PD_WARPS - 1) / OQ_PD_WARPS, 32 * OQ_PD_WARPS, sm,
-                   (cudaStream_t)stream>>>(ctx->d_sys, X, grad, W, ctx->n_e,
-                                           param_count_of(ctx->hsys), (int)wbytes, dlogpsi, dEL);
-  OQ_CUDA(ctx, cudaGetLastError());
-  return OQ_OK;
+  return launch_param_derivs(ctx, X, W, grad, OqPdOut{dlogpsi, dEL, nullptr, 0, 0, nullptr, nullptr},
+                             stream);
+}
+
+int oqmc_param_derivs_mapped(oqmc_ctx* ctx, const double* X, int W, const double* grad,
+                             const double* eparts, const double* map, int n_flat, double* e_loc,
+                             double* dlogpsi, double* dEL, void* stream) {
+  if (!ctx) return OQ_ERR_ARG;
+  if (W < 0 || n_flat < 1 ||
+      (W > 0 && (!X || !grad || !eparts || !map || !e_loc || !dlogpsi || !dEL)))
+    return set_err(ctx, OQ_ERR_ARG, "bad arguments%s");
+  if (W == 0) return OQ_OK;
+  return launch_param_derivs(ctx, X, W, grad, OqPdOut{dlogpsi, dEL, map, n_flat, 0, eparts, e_loc},
+                             stream);
 }
 
 // TF32 rounding as cvt.rna (nearest, ties away from zero) and BF16 (nearest even)
@@ -1429,16 +1479,6 @@ static int pick_wpb(oqmc_ctx* ctx, int wpb, int precision, size_t* sm) {
 static int launch_moves(oqmc_ctx* ctx, const OqMoveArgs& m, int wpb, size_t sm, int precision,
                         void* stream) {
   const int mixed = precision == OQ_PREC_MIXED;
-  if (ctx->move_kind == 1 && m.mode == 0) {
-    // all-electron steps: table-driven FP64 evaluation of the proposals
-    const OqLaunch La = make_launch(ctx, stream, smem_sys_c64(ctx));
-    cudaError_t err = cudaSuccess;
-#define OQ_X(N) err = oq_moves_alle_##N(La, m, mixed)
-    OQ_SWITCH(ctx->nocc, OQ_X)
-#undef OQ_X
-    OQ_CUDA(ctx, err);
-    return OQ_OK;
-  }
   const OqLaunch L = make_launch(ctx, stream, sm);
   if (ctx->mlp && m.mode == 0) {
     OqMoveArgs mm = m;
@@ -1616,21 +1656,39 @@ int oqmc_sweeps(oqmc_ctx* ctx, double* X, int W, void* state, int precision, int
     sa.sums = sums; sa.el_trace = el_trace; sa.eparts_last = eparts_last;
     return launch_sweeps(ctx, sa, wpb_asked, wpb, precision, stream);
   }
-  // all-electron steps, the learned proposal, the tensor-core local energy:
-  // moves and local energies in separate launches
-  const bool fused_moves = ctx->move_kind == 0 && !ctx->mlp;
-  OQ_CUDA(ctx, to_soa(ctx, X, st.pos, W, s));
+  OqAlleArgs aa;
+  memset(&aa, 0, sizeof(aa));
+  aa.X = X; aa.pos = st.pos; aa.ainv = st.ainv; aa.logdet = st.logdet; aa.W = W;
+  aa.step = step; aa.seed = seed; aa.step_base = step_base; aa.flags = ctx->d_flags;
+  auto alle = [&]() -> int {
+    const OqLaunch La = make_launch(ctx, stream, 0);
+    cudaError_t err = cudaSuccess;
+#define OQ_X(N) err = oq_alle_##N(La, aa, mixed)
+    OQ_SWITCH(ctx->nocc, OQ_X)
+#undef OQ_X
+    OQ_CUDA(ctx, err);
+    return OQ_OK;
+  };
+  if (ctx->move_kind == 1 && !mixed) {
+    aa.n_steps = n_sweeps; aa.measure_every = n_sweeps >= measure_every ? measure_every : 0;
+    aa.sums = sums; aa.el_trace = el_trace; aa.eparts_last = eparts_last;
+    return alle();
+  }
+  // mixed all-electron steps, the learned proposal, the tensor-core local
+  // energy: moves and local energies in separate launches
+  if (ctx->mlp) OQ_CUDA(ctx, to_soa(ctx, X, st.pos, W, s));
   OqMoveArgs m;
   memset(&m, 0, sizeof(m));
   m.pos = st.pos; m.ainv = st.ainv; m.logdet = st.logdet; m.W = W; m.mode = 0;
   m.step = step; m.seed = seed; m.flags = ctx->d_flags;
   m.proposal = ctx->proposal; m.scale_r0 = ctx->scale_r0; m.scale_fmin = ctx->scale_fmin;
   auto moves = [&](int n, int at, double* acc) -> int {
-    m.n_steps = sa.n_sweeps = n;
-    m.step_base = sa.step_base = step_base + at;
-    m.acc_sum = sa.acc_sum = acc;
-    return fused_moves ? launch_sweeps(ctx, sa, wpb_asked, wpb, precision, stream)
-                       : launch_moves(ctx, m, wpb, sm, precision, stream);
+    m.n_steps = sa.n_sweeps = aa.n_steps = n;
+    m.step_base = sa.step_base = aa.step_base = step_base + at;
+    m.acc_sum = sa.acc_sum = aa.acc_sum = acc;
+    if (ctx->move_kind == 1) return alle();
+    return ctx->mlp ? launch_moves(ctx, m, wpb, sm, precision, stream)
+                    : launch_sweeps(ctx, sa, wpb_asked, wpb, precision, stream);
   };
   OqElocArgs el;
   memset(&el, 0, sizeof(el));
@@ -1672,7 +1730,7 @@ int oqmc_sweeps(oqmc_ctx* ctx, double* X, int W, void* state, int precision, int
     int rc = moves(n_sweeps - done, done, nullptr);
     if (rc != OQ_OK) return rc;
   }
-  OQ_CUDA(ctx, to_aos(ctx, st.pos, X, W, s));
+  if (ctx->mlp) OQ_CUDA(ctx, to_aos(ctx, st.pos, X, W, s));
   return OQ_OK;
 }
 

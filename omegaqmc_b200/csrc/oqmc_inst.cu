@@ -188,28 +188,28 @@ cudaError_t OQ_FN(oq_md_local)(const OqLaunch& L, const OqMdTables& T, const OqM
   return M == 16 ? md_local_m<16>(L, T, st, a, logpsi, grad, lap) : cudaErrorInvalidValue;
 }
 
-cudaError_t OQ_FN(oq_moves_alle)(const OqLaunch& L, const OqMoveArgs& a, int mixed) {
-  const int tpb = 128, nb = (a.W + tpb - 1) / tpb;
-  cudaError_t e;
-  if (mixed) {
-    e = oq_smem_attr(k_moves_alle<OQ_N, float>, L.smem);
-    if (e != cudaSuccess) return e;
-    k_moves_alle<OQ_N, float><<<nb, tpb, L.smem, L.stream>>>(
-        L.sys, L.C64, a.pos, (float*)a.ainv, a.logdet, a.W, a.n_steps, a.step, a.seed,
-        a.step_base, a.acc_sum, L.flags);
-  } else {
-    e = oq_smem_attr(k_moves_alle<OQ_N, double>, L.smem);
-    if (e != cudaSuccess) return e;
-    k_moves_alle<OQ_N, double><<<nb, tpb, L.smem, L.stream>>>(
-        L.sys, L.C64, a.pos, (double*)a.ainv, a.logdet, a.W, a.n_steps, a.step, a.seed,
-        a.step_base, a.acc_sum, L.flags);
-  }
+template <typename Real, bool EXT>
+static cudaError_t alle(const OqLaunch& L, OqAlleArgs a) {
+  a.wb = oq_team_walkers<OQ_N>(a.W);
+  while (a.wb > 1 && L.ao_bytes + oq_alle_tile_bytes(OQ_N, a.wb) > 227 * 1024) a.wb >>= 1;
+  a.flags = L.flags;
+  const int act = a.wb * 2 * OQ_N, tpb = act < 128 ? 128 : (act + 31) / 32 * 32;
+  const size_t smem = L.ao_bytes + oq_alle_tile_bytes(OQ_N, a.wb);
+  cudaError_t e = oq_smem_attr(k_alle<OQ_N, Real, EXT>, smem);
+  if (e != cudaSuccess) return e;
+  k_alle<OQ_N, Real, EXT><<<(a.W + a.wb - 1) / a.wb, tpb, smem, L.stream>>>(L.sys, L.ao,
+                                                                           L.ao_bytes, a);
   return cudaGetLastError();
+}
+
+cudaError_t OQ_FN(oq_alle)(const OqLaunch& L, const OqAlleArgs& a, int mixed) {
+  if (mixed) return L.ext ? alle<float, true>(L, a) : alle<float, false>(L, a);
+  return L.ext ? alle<double, true>(L, a) : alle<double, false>(L, a);
 }
 
 // Per-thread local memory (bytes) of one kernel this size launches: kind 0
 // k_team (refresh), 1 k_sweeps, 2 k_eloc, 3 k_eloc_tc, 4 k_md_refresh,
-// 5 k_md_moves, 6 k_md_local (M = 8 or 16 columns), 7 k_moves_alle.
+// 5 k_md_moves, 6 k_md_local (M = 8 or 16 columns), 7 k_alle.
 template <typename K>
 static cudaError_t oq_lmem(K kernel, size_t* out) {
   cudaFuncAttributes a;
@@ -246,8 +246,8 @@ cudaError_t OQ_FN(oq_local_bytes)(int kind, int mixed, int M, size_t* out) {
       }
       return M == 16 ? md_lmem<16>(kind, out) : cudaErrorInvalidValue;
     case 7:
-      return mixed ? oq_lmem(k_moves_alle<OQ_N, float>, out)
-                   : oq_lmem(k_moves_alle<OQ_N, double>, out);
+      return mixed ? oq_lmem(k_alle<OQ_N, float, true>, out)
+                   : oq_lmem(k_alle<OQ_N, double, true>, out);
   }
   return cudaErrorInvalidValue;
 }

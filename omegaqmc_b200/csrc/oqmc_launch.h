@@ -28,7 +28,7 @@ struct OqLaunch {
                              double* logdet, int mixed);                              \
   cudaError_t oq_basin_##N(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed); \
   cudaError_t oq_sweeps_##N(const OqLaunch& L, const OqSweepArgs& a, int nthr, int mixed); \
-  cudaError_t oq_moves_alle_##N(const OqLaunch& L, const OqMoveArgs& a, int mixed);     \
+  cudaError_t oq_alle_##N(const OqLaunch& L, const OqAlleArgs& a, int mixed);           \
   cudaError_t oq_eloc_##N(const OqLaunch& L, const OqElocArgs& a, int mixed);           \
   cudaError_t oq_eloc_tc_##N(const OqLaunch& L, const OqElocArgs& a, const void* Bpack, \
                              int nbf);                                                \

@@ -103,6 +103,21 @@ __device__ __forceinline__ void oq_ao_add(const double* C, double v, double (&mv
   }
 }
 
+// The three AOs of a p function, added to each other first (the order of
+// oq_mo_val, so that the persistent kernel's refresh gives the same values).
+template <int N>
+__device__ __forceinline__ void oq_ao_add3(const double* C, double v0, double v1, double v2,
+                                           double (&mv)[N]) {
+  constexpr int NP = (N + 1) / 2 * 2;
+  const double2* c2 = reinterpret_cast<const double2*>(C);
+#pragma unroll
+  for (int m = 0; m < N; m += 2) {
+    const double2 a = c2[m / 2], b = c2[(NP + m) / 2], c = c2[(2 * NP + m) / 2];
+    mv[m] += a.x * v0 + b.x * v1 + c.x * v2;
+    if (m + 1 < N) mv[m + 1] += a.y * v0 + b.y * v1 + c.y * v2;
+  }
+}
+
 template <int N>
 __device__ __forceinline__ double oq_ao_dot(const double* C, const double (&ac)[N]) {
   const double2* c2 = reinterpret_cast<const double2*>(C);
@@ -133,6 +148,15 @@ static __device__ __noinline__ void oq_ao_special(const OqSystem* gS, int ia, in
     }
     if (word & (0x100 << k)) oq_cusp_vgl(*gS, ia, sqrt(r2), R[k], P[k], L[k]);
   }
+}
+
+static __device__ __noinline__ double oq_ao_special_value(const OqSystem* gS, int ia, int word,
+                                                          int k, double r2, double R) {
+  if (word & (0x400 << k)) {
+    double gp, gpp;
+    oq_spline_gdd(*gS, gS->s_spl[(word >> 16) + k], r2, R, gp, gpp);
+  }
+  return word & (0x100 << k) ? oq_cusp_val(*gS, ia, sqrt(r2), R) : R;
 }
 
 static __device__ __noinline__ void oq_ao_harm(const OqSystem* gS, int am, int q, double x,
@@ -178,9 +202,8 @@ __device__ __forceinline__ void oq_ao_value(const OqAo<N>& T, const OqSystem* __
         }
       }
       if (EXT && (G.x & 0xF00)) {
-        double R[2] = {R0, R1}, P[2] = {0.0, 0.0}, L[2] = {0.0, 0.0};
-        oq_ao_special(gS, ia, G.x, r2, R, P, L);
-        R0 = R[0]; R1 = R[1];
+        R0 = oq_ao_special_value(gS, ia, G.x, 0, r2, R0);
+        R1 = oq_ao_special_value(gS, ia, G.x, 1, r2, R1);
       }
       const double* C = T.C + G.w * NP;
 #pragma unroll 1
@@ -189,9 +212,7 @@ __device__ __forceinline__ void oq_ao_value(const OqAo<N>& T, const OqSystem* __
           oq_ao_add<N>(C, R0, mv);
           C += NP;
         } else if (am == 1) {
-          oq_ao_add<N>(C, R0 * dx, mv);
-          oq_ao_add<N>(C + NP, R0 * dy, mv);
-          oq_ao_add<N>(C + 2 * NP, R0 * dz, mv);
+          oq_ao_add3<N>(C, R0 * dx, R0 * dy, R0 * dz, mv);
           C += 3 * NP;
         } else if (!EXT || am == 2) {
           double Y[5], dY[5][3];
@@ -678,6 +699,244 @@ k_team(const OqSystem* __restrict__ gS, const unsigned char* __restrict__ ao, in
       ep[0] = v[2]; ep[1] = v[3]; ep[2] = ke; ep[3] = v[2] + v[3] + ke + T.h->e_nn;
     }
     if (good && (!isfinite(ke) || !isfinite(lpsi))) atomicOr(a.flags, OQ_FLAG_NAN);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// All-electron Metropolis steps, the reference's move (metropolis_move_alle
+// and metropolis_move_1w, OmegaQMC/vmc_gto.py:815-905): every electron is
+// displaced by step * N(0, 1); a proposal with an electron-electron or
+// electron-nucleus distance below 1e-4 bohr is rejected (ratio 0,
+// constants.py:23); otherwise it is accepted when u < exp(2 (ln|psi'| -
+// ln|psi|)), ln|psi| = log|det up| + log|det down| + J evaluated afresh in
+// FP64 (inverses of the proposed Slater matrices, which become the state's
+// inverses on acceptance).  Random numbers: electron e's normals from the
+// Philox block (walker, step, e, 0), u from electron 0's block.
+//
+// The tile of k_team, kept for all steps of the launch: one thread per
+// (walker, electron), the walker's state in shared memory.  A step is one
+// orbital row, one share of the pair terms and one column of an inversion per
+// thread instead of 2 N rows, all pairs and two inversions in local memory on
+// one; the FP64 local energy of a measured step follows from what is already
+// there (the mixed one has its own kernel).  Measured with a local energy
+// every step, H2O, 16,384 walkers, FP64: 295 -> 69 us per step.
+// ---------------------------------------------------------------------------
+struct OqAlleArgs {
+  double* X;               // walkers (W, n_e, 3), updated in place
+  double* pos;             // the state's positions (SoA)
+  void* ainv;
+  double* logdet;
+  int W, wb, n_steps;
+  int measure_every;       // 0: no local energies
+  double step;
+  uint64_t seed, step_base;
+  double* acc_sum;         // += accepted electron moves outside measurements, or null
+  double* sums;            // as OqSweepArgs
+  double* el_trace;
+  double* eparts_last;
+  unsigned* flags;
+};
+
+// Bytes of a tile: k_team's, the proposals and the accepted inverses, and the
+// walkers' decisions.
+constexpr size_t oq_alle_tile_bytes(int n, int wb) {
+  return oq_team_tile_bytes(n, wb) + sizeof(double) * (size_t)wb * ((size_t)6 * n + 2 * n * n) +
+         sizeof(int) * (size_t)wb;
+}
+
+template <int N, typename Real, bool EXT>
+__global__ void __launch_bounds__(OqTeam<N>::T, OqTeam<N>::MINB)
+k_alle(const OqSystem* __restrict__ gS, const unsigned char* __restrict__ ao, int ao_bytes,
+       OqAlleArgs a) {
+  constexpr int NE = 2 * N;
+  extern __shared__ __align__(16) unsigned char smem[];
+  const int wb = a.wb, W = a.W, tid = threadIdx.x;
+  const OqTile<N> tl(smem + ao_bytes, wb);
+  double* xnew = reinterpret_cast<double*>(smem + ao_bytes + oq_team_tile_bytes(N, wb));
+  double* Acur = xnew + (size_t)6 * N * wb;
+  int* decided = reinterpret_cast<int*>(Acur + (size_t)2 * N * N * wb);
+  for (int i = tid; i < ao_bytes / 16; i += blockDim.x)
+    reinterpret_cast<int4*>(smem)[i] = reinterpret_cast<const int4*>(ao)[i];
+  const int w0 = blockIdx.x * wb;
+  for (int q = tid; q < 3 * NE * wb; q += blockDim.x) {
+    const int j = q / (3 * NE), k = q - j * 3 * NE;
+    tl.pos[k * wb + j] = a.X[(size_t)min(w0 + j, W - 1) * 3 * NE + k];
+  }
+  Real* gA = reinterpret_cast<Real*>(a.ainv);
+  for (int q = tid; q < 2 * N * N * wb; q += blockDim.x) {
+    // state (s, m, j) -> tile (s, j, m): an electron's column contiguous
+    const int j = q % wb, k = q / wb, s = k / (N * N), m = (k / N) % N, c = k % N;
+    Acur[((s * N + c) * N + m) * wb + j] = (double)gA[(size_t)k * W + min(w0 + j, W - 1)];
+  }
+  __syncthreads();
+  const OqAo<N> T(smem);
+  const int wl = tid & (wb - 1), e = tid / wb, s = e & 1, i = e >> 1, w = w0 + wl;
+  const bool active = e < NE;
+  const bool live = active && w < W;
+  double* pos = tl.pos + wl;
+  double* pn = xnew + wl;
+  double* Sw = tl.S + (size_t)s * N * N * wb + wl;
+  double* Aw = Acur + (size_t)s * N * N * wb + wl;
+  double* red = tl.red + (size_t)e * 6 * wb + wl;
+  double x = 0.0, y = 0.0, z = 0.0;
+  // the walker's ln|psi| and log|det|, held by its thread of electron 0
+  double lpsi = 0.0, ld_cur = 0.0;
+  int nacc = 0, meas = 0;
+  double gx = 0.0, gy = 0.0, gz = 0.0, lap = 0.0, ee = 0.0, en = 0.0;
+  if (active) {
+    x = pos[(3 * e) * wb]; y = pos[(3 * e + 1) * wb]; z = pos[(3 * e + 2) * wb];
+    double jv = 0.0;
+    oq_team_pairs<N, false, EXT>(T, gS, pos, wb, e, x, y, z, jv, gx, gy, gz, lap, ee, en);
+    red[0] = jv;
+  }
+  __syncthreads();
+  if (live && e == 0) {
+    ld_cur = a.logdet[w];
+    double J = 0.0;
+    for (int k = 0; k < NE; ++k) J += tl.red[(size_t)k * 6 * wb + wl];
+    lpsi = ld_cur + J;
+  }
+  const int n_meas = a.measure_every > 0 ? a.n_steps / a.measure_every : 0;
+  for (int t = 0; t < a.n_steps; ++t) {
+    double nx = 0.0, ny = 0.0, nz = 0.0, u = 0.0;
+    if (active) {
+      double n3[3];
+      oq_move_randoms(a.seed, (uint32_t)w, (uint32_t)(a.step_base + t), (uint32_t)e, n3, u);
+      nx = x + a.step * n3[0];
+      ny = y + a.step * n3[1];
+      nz = z + a.step * n3[2];
+      pn[(3 * e) * wb] = nx; pn[(3 * e + 1) * wb] = ny; pn[(3 * e + 2) * wb] = nz;
+    }
+    double col[N];
+#pragma unroll
+    for (int m = 0; m < N; ++m) col[m] = 0.0;
+    if (active) {
+      oq_ao_value<N, EXT>(T, gS, nx, ny, nz, col);
+#pragma unroll
+      for (int m = 0; m < N; ++m) Sw[(i * N + m) * wb] = col[m];
+    }
+    __syncthreads();
+    if (active) {
+#pragma unroll
+      for (int r = 0; r < N; ++r) col[r] = Sw[(r * N + i) * wb];
+    }
+    double det;
+    int dst;
+    const bool ok = oq_team_invert<N, false>(col, tl, wb, wl, s, i, active, det, dst);
+    if (active) {
+      bool valid = true;
+      for (int j = e + 1; j < NE; ++j) {
+        const double dx = nx - pn[(3 * j) * wb], dy = ny - pn[(3 * j + 1) * wb],
+                     dz = nz - pn[(3 * j + 2) * wb];
+        valid = valid && (dx * dx + dy * dy + dz * dz >= 1e-8);
+      }
+      for (int I = 0; I < T.h->natm; ++I) {
+        const double dx = nx - T.atom[I].x, dy = ny - T.atom[I].y, dz = nz - T.atom[I].z;
+        valid = valid && (dx * dx + dy * dy + dz * dz >= 1e-8);
+      }
+      double jv = 0.0;
+      oq_team_pairs<N, false, EXT>(T, gS, pn, wb, e, nx, ny, nz, jv, gx, gy, gz, lap, ee, en);
+      red[0] = log(fabs(det));
+      red[wb] = jv;
+      red[2 * wb] = valid && ok ? 1.0 : 0.0;
+    }
+    __syncthreads();
+    if (active && e == 0) {
+      double ld = 0.0, J = 0.0, good = 1.0;
+      for (int k = 0; k < NE; ++k) {
+        const double* rd = tl.red + (size_t)k * 6 * wb + wl;
+        ld += rd[0];
+        J += rd[wb];
+        good *= rd[2 * wb];
+      }
+      const double lpn = ld + J;
+      bool acc = live && good != 0.0;
+      if (acc && !isfinite(lpn)) {
+        atomicOr(a.flags, OQ_FLAG_NAN);
+        acc = false;
+      }
+      // an old state with psi = 0 (log -inf) accepts any finite proposal
+      acc = acc && (!isfinite(lpsi) || log(u) < 2.0 * (lpn - lpsi));
+      if (acc) {
+        ++nacc;
+        lpsi = lpn;
+        ld_cur = ld;
+      }
+      decided[wl] = acc;
+    }
+    __syncthreads();
+    if (active && decided[wl]) {
+      x = nx; y = ny; z = nz;
+      pos[(3 * e) * wb] = x; pos[(3 * e + 1) * wb] = y; pos[(3 * e + 2) * wb] = z;
+#pragma unroll
+      for (int m = 0; m < N; ++m) Aw[(dst * N + m) * wb] = col[m];
+    }
+    if (meas == n_meas || (t + 1) % a.measure_every != 0) continue;
+    __syncthreads();
+    if (active) {
+#pragma unroll
+      for (int m = 0; m < N; ++m) col[m] = Aw[(i * N + m) * wb];
+      double jv = 0.0;
+      ee = en = 0.0;
+      oq_ao_contract<N, EXT>(T, gS, x, y, z, col, gx, gy, gz, lap);
+      lap -= gx * gx + gy * gy + gz * gz;
+      oq_team_pairs<N, true, EXT>(T, gS, pos, wb, e, x, y, z, jv, gx, gy, gz, lap, ee, en);
+      red[0] = ee; red[wb] = en; red[2 * wb] = lap;
+      red[3 * wb] = gx * gx + gy * gy + gz * gz;
+    }
+    __syncthreads();
+    if (e == 0) {
+      // whole warps reach this when wb is 32 or more; with smaller tiles the
+      // walkers of electron 0 are the first wb threads of warp 0
+      double v[4] = {0.0, 0.0, 0.0, 0.0};
+      for (int k = 0; k < NE; ++k) {
+        const double* rd = tl.red + (size_t)k * 6 * wb + wl;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] += rd[q * wb];
+      }
+      const double ke = -0.5 * (v[2] + v[3]), el = v[0] + v[1] + ke + T.h->e_nn;
+      const bool fine = live && isfinite(el);
+      if (live) {
+        if (a.el_trace) a.el_trace[(size_t)meas * W + w] = el;
+        if (a.eparts_last && meas == n_meas - 1) {
+          double* ep = a.eparts_last + (size_t)w * 4;
+          ep[0] = v[0]; ep[1] = v[1]; ep[2] = ke; ep[3] = el;
+        }
+        if (!fine) atomicOr(a.flags, OQ_FLAG_NAN);
+      }
+      double vals[7] = {fine ? v[0] : 0.0, fine ? v[1] : 0.0, fine ? ke : 0.0, fine ? el : 0.0,
+                        fine ? el * el : 0.0, live ? (double)(nacc * NE) : 0.0, fine ? 1.0 : 0.0};
+      const int span = wb < 32 ? wb : 32;
+      const unsigned mask = span == 32 ? 0xffffffffu : (1u << span) - 1u;
+#pragma unroll
+      for (int k = 0; k < 7; ++k)
+        for (int o = span >> 1; o > 0; o >>= 1) vals[k] += __shfl_xor_sync(mask, vals[k], o);
+      if ((wl & 31) == 0) {
+        double* sm = a.sums + (size_t)meas * OQ_NSUM;
+#pragma unroll
+        for (int k = 0; k < 7; ++k) atomicAdd(sm + k, vals[k]);
+      }
+    }
+    nacc = 0;
+    ++meas;
+    __syncthreads();         // the sums are read before the next step's are written
+  }
+  __syncthreads();
+  for (int q = tid; q < 3 * NE * wb; q += blockDim.x) {
+    const int j = q / (3 * NE), k = q - j * 3 * NE;
+    if (w0 + j < W) a.X[(size_t)(w0 + j) * 3 * NE + k] = tl.pos[k * wb + j];
+  }
+  for (int q = tid; q < 3 * NE * wb; q += blockDim.x) {
+    const int k = q / wb, j = q - k * wb;
+    if (w0 + j < W) a.pos[(size_t)k * W + w0 + j] = tl.pos[q];
+  }
+  for (int q = tid; q < 2 * N * N * wb; q += blockDim.x) {
+    const int j = q % wb, k = q / wb, sp = k / (N * N), m = (k / N) % N, c = k % N;
+    if (w0 + j < W) gA[(size_t)k * W + w0 + j] = (Real)Acur[((sp * N + c) * N + m) * wb + j];
+  }
+  if (live && e == 0) {
+    a.logdet[w] = ld_cur;
+    if (a.acc_sum && nacc) atomicAdd(a.acc_sum, (double)(nacc * NE));
   }
 }
 

@@ -107,21 +107,52 @@ def raw_to_flat(raw, params_corr, system):
     return out
 
 
+def _flat_map(ctx: GTOContext, params_corr):
+    """The linear map raw -> flat of ``raw_to_flat`` as a device matrix
+    (n_raw, n_flat).  It depends on the layout of ``params_corr`` (terms, keys
+    and lengths, not values) and on the context's system, and is kept on the
+    context for the layout last used."""
+    layout = tuple((term, key, int(np.size(params_corr[term][key])))
+                   for term in sorted(params_corr) for key in sorted(params_corr[term]))
+    kept = getattr(ctx, "_flat_map", None)
+    if kept is None or kept[0] != layout:
+        n_raw = int(ctx.lib.oqmc_param_count(ctx._h))
+        ctx._check(min(n_raw, 0))
+        M = raw_to_flat(np.eye(n_raw), params_corr, ctx.system)
+        # complete before any stream reads it
+        dM = torch.as_tensor(M, device=ctx.device)
+        torch.cuda.synchronize(ctx.device)
+        kept = (layout, dM)
+        ctx._flat_map = kept
+    return kept[1]
+
+
 def walker_derivatives(ctx: GTOContext, X, params_corr, stream=None):
     """(E_L (W,), d ln|psi|/dp (W, P), dE_L/dp (W, P)) in the flat parameter
-    order, for walkers X (W, n_e, 3), evaluated in FP64 on the GPU."""
+    order, for walkers X (W, n_e, 3), evaluated in FP64 on the GPU.
+
+    The map onto the flat parameters is applied on the device and the three
+    results come back in one copy."""
     X = ctx.walkers_tensor(X)
     W = X.shape[0]
-    ev = ctx.evaluate(X, want_grad=True, want_lap=False, stream=stream)
-    n_raw = int(ctx.lib.oqmc_param_count(ctx._h))
-    ctx._check(min(n_raw, 0))
-    dl = torch.empty(W, n_raw, dtype=torch.float64, device=ctx.device)
-    de = torch.empty(W, n_raw, dtype=torch.float64, device=ctx.device)
-    ctx._check(ctx.lib.oqmc_param_derivs(ctx._h, _dptr(X), W, _dptr(ev["grad"]), _dptr(dl),
-                                         _dptr(de), _stream_ptr(stream)))
-    dl_f = raw_to_flat(dl.cpu().numpy(), params_corr, ctx.system)
-    de_f = raw_to_flat(de.cpu().numpy(), params_corr, ctx.system)
-    return ev["e_loc"].cpu().numpy(), dl_f, de_f
+    M = _flat_map(ctx, params_corr)
+    P = M.shape[1]
+    with torch.cuda.stream(stream if stream is not None else torch.cuda.current_stream()):
+        buf = torch.empty(W * (1 + 2 * P), dtype=torch.float64, device=ctx.device)
+        opt = dict(dtype=torch.float64, device=ctx.device)
+        logpsi, grad, ep = (torch.empty(W, **opt), torch.empty(W, ctx.n_e, 3, **opt),
+                            torch.empty(W, 4, **opt))
+        e, dl, de = buf[:W], buf[W:W * (1 + P)], buf[W * (1 + P):]
+        ctx._check(ctx.lib.oqmc_eval(ctx._h, _dptr(X), W, _dptr(logpsi), _dptr(grad), None,
+                                     _dptr(ep), _stream_ptr(stream)))
+        if P:
+            ctx._check(ctx.lib.oqmc_param_derivs_mapped(
+                ctx._h, _dptr(X), W, _dptr(grad), _dptr(ep), _dptr(M), P, _dptr(e), _dptr(dl),
+                _dptr(de), _stream_ptr(stream)))
+        else:
+            e.copy_(ep[:, 3])
+        h = buf.cpu().numpy()
+    return h[:W], h[W:W * (1 + P)].reshape(W, P), h[W * (1 + P):].reshape(W, P)
 
 
 def build_matrices(E_L, dlogpsi, dEL):

@@ -95,3 +95,91 @@ def test_determinant_sizes_match_oracle(nocc):
 
 def test_wide_contractions_match_oracle():
     _check(_system(3, _columns), 50)
+
+
+@pytest.mark.parametrize("name,extra,W", [("H2", None, 1), ("H2O", "bspline", 5),
+                                          ("H2O_dimer", "bspline", 3), ("LiH", "j3", 2),
+                                          ("H2O", "j33", 7)])
+def test_parameter_derivatives_raw_and_mapped(name, extra, W):
+    """One warp per walker, four to a CTA: the raw derivatives against the
+    oracle (a wide and a narrow determinant, both spline blocks, three-body
+    orders 2 and 3 with more gammas than lanes), and the mapped form against
+    raw_to_flat of the raw one."""
+    import ctypes
+    import torch
+    from omegaqmc_b200.context import _dptr, _stream_ptr
+    from omegaqmc_b200.optim import raw_to_flat, walker_derivatives
+    mol = M.named_system(name)
+    pc, cfg = M.default_params_corr(mol), None
+    els = sorted(set(mol.elements))
+    if extra == "bspline":
+        pc["J2_bspline"] = {"like": np.array([0.2, 0.1, 0.05]), "unlike": np.linspace(0.4, 0.0, 9)}
+        pc["J1_bspline"] = {e: np.array([-0.1, 0.05, 0.02, 0.01]) for e in els}
+        cfg = {"J2": {"r_cut": 3.5}, "J1": {e: {"r_cut": 3.0} for e in els}}
+    elif extra:
+        k = 2 if extra == "j3" else 3
+        rng = np.random.default_rng(6)
+        pc["J3_eeI"] = {p + e: rng.normal(size={2: 8, 3: 26}[k]) * 0.01 for e in els
+                        for p in ("like+", "unlike+") if p + e != "like+" + els[0]}
+        cfg = {"J3": {"N_eI": k, "N_ee": k, "r_cut": 4.5}}
+    import warnings
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        s = build_system(M.make_mf(name), pc, None, cfg)
+    ctx = GTOContext(s)
+    X = ctx.walkers_tensor(seeded_walkers(s, W, 0.9, 7))
+    grad = ctx.evaluate(X)["grad"]
+    n = ctx.lib.oqmc_param_count(ctx._h)
+    dl = torch.full((W, n), np.nan, dtype=torch.float64, device="cuda")
+    de = dl.clone()
+    ctx._check(ctx.lib.oqmc_param_derivs(ctx._h, _dptr(X), W, _dptr(grad), _dptr(dl), _dptr(de),
+                                         _stream_ptr(None)))
+    rl, re_ = O.param_derivatives(s, X.cpu().numpy())
+    assert np.max(np.abs(dl.cpu().numpy() - rl) / (np.abs(rl).max(axis=0) + 1.0)) < 1e-10
+    assert np.max(np.abs(de.cpu().numpy() - re_) / (np.abs(re_).max(axis=0) + 1.0)) < 1e-9
+    e, fl, fe = walker_derivatives(ctx, X, pc)
+    ml, me = raw_to_flat(dl.cpu().numpy(), pc, s), raw_to_flat(de.cpu().numpy(), pc, s)
+    # the same products summed in another order
+    assert np.max(np.abs(fl - ml) / (np.abs(ml).max(axis=0) + 1.0)) < 1e-13
+    assert np.max(np.abs(fe - me) / (np.abs(me).max(axis=0) + 1.0)) < 1e-13
+    assert e.shape == (W,) and fl.shape == fe.shape == ml.shape
+    assert ctx.lib.oqmc_param_derivs_mapped(ctx._h, _dptr(X), W, _dptr(grad), None, None, 0, None,
+                                            None, None, ctypes.c_void_p(0)) == -1
+
+
+@pytest.mark.parametrize("name,prec,sizes", [("H2", "fp64", (1, 70, 40000)),
+                                             ("LiH", "fp64", (2, 33, 5000)),
+                                             ("H2O", "fp64", (3, 65, 20001)),
+                                             ("H2O", "mixed", (3, 500)),
+                                             ("H2O_dimer", "fp64", (1, 17))])
+def test_all_electron_steps_do_not_depend_on_the_tile(name, prec, sizes):
+    """A walker's chain depends on its index and the seed, not on the tile it
+    shares: the first walkers of ensembles whose tiles differ (one warp up to
+    full CTAs, partial last tiles) agree, and the last local energies and
+    log|det| match the oracle at the final walkers."""
+    import torch
+    mf = M.make_mf(name)
+    s = build_system(mf, M.default_params_corr(mf.mol))
+    X = seeded_walkers(s, max(sizes), 0.8, 5)
+    runs = []
+    for W in sizes:
+        ctx = GTOContext(s)
+        ctx.set_move_kind(1)
+        ens = WalkerEnsemble(ctx, X[:W], prec, seed=4, refresh_every=10**9)
+        ep = torch.zeros(W, 4, dtype=torch.float64, device="cuda")
+        sums = ens.run(6, 0.12, measure_every=2, eparts_last=ep)
+        assert torch.all(sums[:, 6] == W) and torch.all(sums[:, 5] % s.n_e == 0)
+        assert abs(float(sums[-1, 3]) - float(ep[:, 3].sum())) < 1e-9 * float(ep[:, 3].abs().sum())
+        m = min(W, 100)
+        o = O.evaluate(s, ens.X[:m].cpu().numpy())
+        sc = 0.5 * (np.sum(np.abs(o["lap"]), axis=1) + np.sum(o["grad"] ** 2, axis=(1, 2))) + 1.0
+        err = np.abs(ep[:m, 3].cpu().numpy() - o["e_loc"]) / (np.abs(o["e_loc"]) + sc)
+        assert np.max(err) < (1e-10 if prec == "fp64" else 2e-3)
+        ld = ens.logdet()[:m].cpu().numpy()
+        assert np.max(np.abs(ld - O.log_slater(s, ens.X[:m].cpu().numpy())) / (np.abs(ld) + 1)) < TOL
+        ens.run(1, 0.12)                       # a step after the last measurement
+        assert ctx.flags() == 0
+        runs.append(ens.X)
+    for a, b in zip(runs, runs[1:]):
+        assert torch.equal(a, b[: a.shape[0]])
+    assert not torch.equal(runs[-1], torch.as_tensor(X, device="cuda"))
