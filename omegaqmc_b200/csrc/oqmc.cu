@@ -106,7 +106,7 @@ static bool nocc_supported(int n) {
 static OqLaunch make_launch(const oqmc_ctx* ctx, void* stream, size_t smem) {
   OqLaunch L;
   L.sys = ctx->d_sys; L.split = ctx->d_split; L.C64 = ctx->d_C64; L.C32 = ctx->d_C32;
-  L.ao = ctx->d_ao; L.ao_bytes = ctx->ao_bytes; L.ext = ctx->ao_ext;
+  L.ao = ctx->d_ao; L.ao_bytes = ctx->ao_bytes; L.ext = ctx->ao_ext; L.Ct = ctx->d_Ct;
   L.flags = ctx->d_flags; L.stream = (cudaStream_t)stream; L.smem = smem;
   return L;
 }
@@ -493,8 +493,14 @@ extern "C" int oqmc_create(oqmc_ctx** out, const oqmc_system_desc* d) {
   const std::vector<unsigned char> ao = pack_ao(S, d->C);
   ctx->ao_bytes = (int)ao.size();
   ctx->ao_ext = reinterpret_cast<const OqAoHead*>(ao.data())->ext;
-  e = (e == cudaSuccess) ? cudaMalloc(&ctx->d_ao, ao.size()) : e;
+  std::vector<double> Ct((size_t)d->nbf * d->nocc);
+  for (int a = 0; a < d->nbf; ++a)
+    for (int m = 0; m < d->nocc; ++m) Ct[(size_t)m * d->nbf + a] = d->C[(size_t)a * d->nocc + m];
+  e = (e == cudaSuccess) ? cudaMalloc(&ctx->d_ao, ao.size() + sizeof(double) * Ct.size()) : e;
   e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_ao, ao.data(), ao.size(), cudaMemcpyHostToDevice) : e;
+  ctx->d_Ct = reinterpret_cast<double*>(ctx->d_ao + ao.size());
+  e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_Ct, Ct.data(), sizeof(double) * Ct.size(),
+                                      cudaMemcpyHostToDevice) : e;
   e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_sys, &S, sizeof(OqSystem), cudaMemcpyHostToDevice) : e;
   e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_split, &ctx->hsplit, sizeof(OqSplit), cudaMemcpyHostToDevice) : e;
   e = (e == cudaSuccess) ? cudaMemcpy(ctx->d_C64, d->C, sizeof(double) * c32.size(), cudaMemcpyHostToDevice) : e;

@@ -27,6 +27,7 @@ struct oqmc_ctx {
   double* d_C64;
   float* d_C32;
   unsigned char* d_ao;     // packed tables of the FP64 evaluation (OqAoHead ...)
+  double* d_Ct;            // MO coefficients, one orbital after the other (in d_ao's block)
   int ao_bytes, ao_ext;    // ao_ext: OqAoHead::ext
   unsigned* d_flags;
   double* d_j3;            // three-body Jastrow gamma blocks (or null)

@@ -27,9 +27,11 @@ template <int MODE, typename Real, bool EXT>
 static cudaError_t team_ext(const OqLaunch& L, OqTeamArgs a) {
   a.wb = oq_team_walkers<OQ_N>(a.W);
   a.flags = L.flags;
+  a.Ct = L.Ct;
   // at least 128 threads, so that a small tile copies the system tables fast
   const int act = a.wb * 2 * OQ_N, tpb = act < 128 ? 128 : (act + 31) / 32 * 32;
-  const size_t smem = L.ao_bytes + oq_team_tile_bytes(OQ_N, a.wb);
+  const size_t smem = L.ao_bytes + oq_team_tile_bytes(OQ_N, a.wb) +
+                      (MODE == OQ_TEAM_EVAL ? sizeof(double) * 8 * OQ_N * OQ_N : 0);
   cudaError_t e = oq_smem_attr(k_team<OQ_N, MODE, Real, EXT>, smem);
   if (e != cudaSuccess) return e;
   k_team<OQ_N, MODE, Real, EXT><<<(a.W + a.wb - 1) / a.wb, tpb, smem, L.stream>>>(L.sys, L.ao,

@@ -14,6 +14,7 @@ struct OqLaunch {
   const float* C32;
   const unsigned char* ao;   // packed tables of the FP64 evaluation (oqmc_team.cuh)
   int ao_bytes, ext;
+  const double* Ct;          // MO coefficients, orbital by orbital
   unsigned* flags;
   cudaStream_t stream;
   size_t smem;

@@ -14,7 +14,7 @@
 // an N-th of the chain, keeps one matrix column of N doubles in registers,
 // and costs one barrier per elimination step.  Measured per call (thread per
 // walker -> this): H2O, 1 walker 281 -> 25 us (launch and host time); N2,
-// 4,097 walkers 855 -> 47 us; (H2O)2, 16,384 walkers 1,653 -> 222 us (FP64
+// 4,097 walkers 855 -> 60 us; (H2O)2, 16,384 walkers 1,653 -> 240 us (FP64
 // pipe 38% busy, issue slots 54%); log|psi| of 65,536 H2O walkers 181 -> 94
 // us.
 #pragma once
@@ -344,6 +344,8 @@ struct OqTile {
     red = f + (size_t)4 * N * wb;
     piv = reinterpret_cast<int*>(red + (size_t)12 * N * wb);
   }
+  // k_team's evaluation only: oq_walker_by_orbital's [2 N][N][4]
+  __device__ double* orb(int wb) const { return reinterpret_cast<double*>(piv + 4 * wb); }
 };
 
 // Gauss-Jordan inversion of both N x N Slater matrices of every walker of
@@ -569,6 +571,105 @@ __device__ __forceinline__ void oq_team_pairs(const OqAo<N>& T, const OqSystem* 
   }
 }
 
+// Gradient and Laplacian at x of the orbital whose coefficients are C.
+static __device__ __noinline__ void oq_orbital_vgl(const OqSystem* gS, const double* C, double x,
+                                                   double y, double z, double* out) {
+  double mv[1], mg[1][3], ml[1];
+  oq_mo_vgl<1>(*gS, C, x, y, z, mv, mg, ml);
+  out[0] = mg[0][0]; out[1] = mg[0][1]; out[2] = mg[0][2]; out[3] = ml[0];
+}
+
+// Gradient and Laplacian of log|psi| of every electron of one walker of the
+// tile, orbital by orbital: a thread per (electron, orbital), then a thread
+// per electron for the contraction with its inverse column and the pair
+// terms, each sum in one fixed order.  See k_team for its use.  orb: [NE][N][4].
+// Every thread of the CTA calls this.
+template <int N, bool EXT>
+static __device__ __noinline__ void oq_walker_by_orbital(const OqSystem* gS, const double* Ct,
+                                                         const double* pos, const double* A,
+                                                         int ps, double* orb, double* red,
+                                                         double* grad, double* lap) {
+  constexpr int NE = 2 * N;
+  for (int t = threadIdx.x; t < NE * N; t += blockDim.x) {
+    const int e = t / N, m = t - e * N;
+    oq_orbital_vgl(gS, Ct + (size_t)m * gS->nbf, pos[(3 * e) * ps], pos[(3 * e + 1) * ps],
+                   pos[(3 * e + 2) * ps], orb + t * 4);
+  }
+  __syncthreads();
+  const int e = threadIdx.x;
+  if (e < NE) {
+    const OqSystem& S = *gS;
+    const double x = pos[(3 * e) * ps], y = pos[(3 * e + 1) * ps], z = pos[(3 * e + 2) * ps];
+    double gx = 0.0, gy = 0.0, gz = 0.0, lp = 0.0;
+    for (int m = 0; m < N; ++m) {
+      const double am = A[(size_t)(((e & 1) * N + (e >> 1)) * N + m) * ps];
+      const double* o = orb + (e * N + m) * 4;
+      gx += am * o[0]; gy += am * o[1]; gz += am * o[2];
+      lp += am * o[3];
+    }
+    lp -= gx * gx + gy * gy + gz * gz;
+    if (S.has_j2) {
+      for (int j = 0; j < NE; ++j) {
+        if (j == e) continue;
+        const double dx = x - pos[(3 * j) * ps], dy = y - pos[(3 * j + 1) * ps],
+                     dz = z - pos[(3 * j + 2) * ps];
+        const double r = sqrt(dx * dx + dy * dy + dz * dz);
+        const int o = ((e & 1) == (j & 1)) ? 0 : 2;
+        double upr, l;
+        oq_pade_vgl(S.j2[o], S.j2[o + 1], r, upr, l);
+        gx += upr * dx; gy += upr * dy; gz += upr * dz; lp += l;
+      }
+    }
+    if (EXT && S.has_bs2) {
+      for (int j = 0; j < NE; ++j) {
+        if (j == e) continue;
+        const double dx = x - pos[(3 * j) * ps], dy = y - pos[(3 * j + 1) * ps],
+                     dz = z - pos[(3 * j + 2) * ps];
+        const double r = sqrt(dx * dx + dy * dy + dz * dz);
+        const bool like = (e & 1) == (j & 1);
+        double upr, l;
+        oq_bs_vgl<double>(like ? S.bs2_like : S.bs2_unlike, like ? S.bs2_n_like : S.bs2_n_unlike,
+                          like ? S.bs2_dinv_like : S.bs2_dinv_unlike, S.bs2_rcut, r, 1.0 / r,
+                          upr, l);
+        gx += upr * dx; gy += upr * dy; gz += upr * dz; lp += l;
+      }
+    }
+    if (S.has_j1) {
+      for (int I = 0; I < S.natm; ++I) {
+        const double dx = x - S.nuc[I][0], dy = y - S.nuc[I][1], dz = z - S.nuc[I][2];
+        const double r = sqrt(dx * dx + dy * dy + dz * dz);
+        double upr, l;
+        oq_pade_vgl(S.j1a[I], S.j1b[I], r, upr, l);
+        gx += upr * dx; gy += upr * dy; gz += upr * dz; lp += l;
+      }
+    }
+    if (EXT && S.has_bs1) {
+      for (int I = 0; I < S.natm; ++I) {
+        const int ty = S.bs1_type[I];
+        if (ty < 0) continue;
+        const double dx = x - S.nuc[I][0], dy = y - S.nuc[I][1], dz = z - S.nuc[I][2];
+        const double r = sqrt(dx * dx + dy * dy + dz * dz);
+        double upr, l;
+        oq_bs_vgl<double>(S.bs1_c[ty], S.bs1_n[ty], S.bs1_dinv[ty], S.bs1_rcut[ty], r, 1.0 / r,
+                          upr, l);
+        gx += upr * dx; gy += upr * dy; gz += upr * dz; lp += l;
+      }
+    }
+    if (EXT && S.has_j3)
+      oq_j3_vgl_electron<double>(S, pos, (size_t)ps, NE, e, x, y, z, gx, gy, gz, lp);
+    red[(size_t)(e * 6 + 4) * ps] = lp;
+    orb[e * N * 4] = gx; orb[e * N * 4 + 1] = gy; orb[e * N * 4 + 2] = gz;
+    if (grad) { grad[3 * e] = gx; grad[3 * e + 1] = gy; grad[3 * e + 2] = gz; }
+    if (lap) lap[e] = lp;
+  }
+  __syncthreads();
+  if (e < NE) {
+    const double* o = orb + e * N * 4;
+    red[(size_t)(e * 6 + 5) * ps] = o[0] * o[0] + o[1] * o[1] + o[2] * o[2];
+  }
+  __syncthreads();
+}
+
 // What the tile kernel computes.
 enum { OQ_TEAM_EVAL = 0, OQ_TEAM_LOGPSI = 1, OQ_TEAM_REFRESH = 2 };
 
@@ -580,6 +681,7 @@ struct OqTeamArgs {
   double* lap;          // (W, n_e) or null
   double* eparts;       // (W, 4) or null
   void* ainv;           // REFRESH: [2 N N][W] Real
+  const double* Ct;     // EVAL: MO coefficients (N, nbf), for oq_walker_by_orbital
   unsigned* flags;
 };
 
@@ -671,23 +773,51 @@ k_team(const OqSystem* __restrict__ gS, const unsigned char* __restrict__ ao, in
     }
   }
   // sums over the electrons of a walker
+  double* rd0 = tl.red + (size_t)e * 6 * wb + wl;
   if (active) {
-    double* rd = tl.red + (size_t)e * 6 * wb + wl;
-    rd[0] = ok ? log(fabs(det)) : -INFINITY;
-    if (MODE != OQ_TEAM_REFRESH) rd[wb] = jv;
+    rd0[0] = ok ? log(fabs(det)) : -INFINITY;
+    if (MODE != OQ_TEAM_REFRESH) rd0[wb] = jv;
     if (MODE == OQ_TEAM_EVAL) {
-      rd[2 * wb] = ee; rd[3 * wb] = en; rd[4 * wb] = lap; rd[5 * wb] = g2;
+      rd0[2 * wb] = ee; rd0[3 * wb] = en; rd0[4 * wb] = lap; rd0[5 * wb] = g2;
     }
   }
   __syncthreads();
-  if (!live || e != 0) return;
   double v[6] = {0, 0, 0, 0, 0, 0};
   constexpr int NV = MODE == OQ_TEAM_REFRESH ? 1 : (MODE == OQ_TEAM_LOGPSI ? 2 : 6);
-  for (int k = 0; k < NE; ++k) {
-    const double* rd = tl.red + (size_t)k * 6 * wb + wl;
+  if (live && e == 0)
+    for (int k = 0; k < NE; ++k) {
+      const double* rd = tl.red + (size_t)k * 6 * wb + wl;
 #pragma unroll
-    for (int q = 0; q < NV; ++q) v[q] += rd[q * wb];
+      for (int q = 0; q < NV; ++q) v[q] += rd[q * wb];
+    }
+  if (MODE == OQ_TEAM_EVAL) {
+    // Next to a node of the determinant the sums of Laplacians and of squared
+    // gradients, each of order 1/d^2 at distance d, cancel to the kinetic
+    // energy, of order 1/d, and their rounding is what is left of its last
+    // digits.  Such walkers (some in 10^5 of a random set) are evaluated
+    // orbital by orbital instead, in one fixed order of summation, so that
+    // their kinetic energies do not depend on how a tile splits the work.
+    const bool close = live && e == 0 && v[5] > 2e5 * fabs(v[4] + v[5]);
+    if (__syncthreads_or(close)) {
+      if (active && e == 0) tl.piv[wl] = close;
+      __syncthreads();
+      for (int j = 0; j < wb; ++j)
+        if (tl.piv[j])
+          oq_walker_by_orbital<N, EXT>(
+              gS, a.Ct, tl.pos + j, tl.S + j, wb, tl.orb(wb), tl.red + j,
+              a.grad ? a.grad + (size_t)(w0 + j) * NE * 3 : nullptr,
+              a.lap ? a.lap + (size_t)(w0 + j) * NE : nullptr);
+      if (close) {
+        v[4] = v[5] = 0.0;
+        for (int k = 0; k < NE; ++k) {
+          const double* rd = tl.red + (size_t)k * 6 * wb + wl;
+          v[4] += rd[4 * wb];
+          v[5] += rd[5 * wb];
+        }
+      }
+    }
   }
+  if (!live || e != 0) return;
   const bool good = v[0] > -INFINITY;
   const double lpsi = v[0] + v[1];
   a.logpsi[w] = good ? lpsi : -INFINITY;
