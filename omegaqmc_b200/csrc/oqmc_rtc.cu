@@ -419,7 +419,9 @@ struct Gen {
 // The basis policy of one system as a struct named `name`.
 std::string generate_basis(const OqSystem& S, const OqSplit& SP, const double* C, int nocc,
                            const std::string& name) {
-  std::string src = "struct " + name + " {\n";
+  std::string src = "struct " + name + " {\n  static constexpr int natm = " +
+                    std::to_string(S.natm) + ", has_j1 = " + std::to_string(S.has_j1) +
+                    ", has_j2 = " + std::to_string(S.has_j2) + ";\n";
   {
     Gen g{S, SP, C, nocc, ""};
     g.body(false);
