@@ -41,22 +41,6 @@ struct OqJas {
   double j2[4];
 };
 
-// The same constants with what the generator knows of the molecule B belongs
-// to fixed at compile time: the loops over nuclei unroll, and absent Padé
-// terms leave no test behind.
-template <class B>
-struct OqJasOf {
-  static constexpr int natm = B::natm, has_j1 = B::has_j1, has_j2 = B::has_j2;
-  double e_nn;
-  const double (&nuc)[OQ_MAX_NUC][3];
-  const double (&Z)[OQ_MAX_NUC];
-  const double (&j1a)[OQ_MAX_NUC];
-  const double (&j1b)[OQ_MAX_NUC];
-  const double (&j2)[4];
-  __device__ explicit OqJasOf(const OqJas& j)
-      : e_nn(j.e_nn), nuc(j.nuc), Z(j.Z), j1a(j.j1a), j1b(j.j1b), j2(j.j2) {}
-};
-
 // One system of the batch (device copy; filled by the host).
 struct OqBatchSys {
   const OqSystem* sys;      // system tables (global memory)
@@ -321,7 +305,7 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
                                               const OqJas& jas, int w0, uint64_t step0,
                                               uint64_t slot0, unsigned char* smem) {
   constexpr int NE = 2 * NOCC;
-  const OqJasOf<B> J(jas);
+  const OqJasOf<B> J(jas.nuc, jas.e_nn);
   const int NT = blockDim.x, tid = threadIdx.x, WT = d.wt;
   const int P = NT / WT, lane = tid & (P - 1), wl = tid / P;
   constexpr int PP = 3 * NE + 1, AP = 2 * NOCC * NOCC + 1;

@@ -416,12 +416,24 @@ struct Gen {
   }
 };
 
+// A member function name(i) of the policy that returns v[i]: with an index known
+// to the compiler a literal of the type it is converted to, so the kernels'
+// (float)Z[I] costs no conversion.
+std::string const_table(const std::string& name, const double* v, int n) {
+  std::string e = Gen::num(v[n - 1]);
+  for (int i = n - 2; i >= 0; --i)
+    e = "i == " + std::to_string(i) + " ? " + Gen::num(v[i]) + " : " + e;
+  return "  __device__ static constexpr double " + name + "(int i) { return " + e + "; }\n";
+}
+
 // The basis policy of one system as a struct named `name`.
 std::string generate_basis(const OqSystem& S, const OqSplit& SP, const double* C, int nocc,
                            const std::string& name) {
   std::string src = "struct " + name + " {\n  static constexpr int natm = " +
                     std::to_string(S.natm) + ", has_j1 = " + std::to_string(S.has_j1) +
-                    ", has_j2 = " + std::to_string(S.has_j2) + ";\n";
+                    ", has_j2 = " + std::to_string(S.has_j2) + ";\n" +
+                    const_table("Z", S.Z, S.natm) + const_table("j1a", S.j1a, S.natm) +
+                    const_table("j1b", S.j1b, S.natm) + const_table("j2", S.j2, 4);
   {
     Gen g{S, SP, C, nocc, ""};
     g.body(false);

@@ -261,8 +261,11 @@ __device__ __forceinline__ void oq_mo_vgl_t(const OqSystem& S, const OqSplit& SP
 // OqBasisTable reads the system tables (any molecule); a per-system policy
 // generated at run time (oqmc_specialize) has the same two members with the
 // exponents and coefficients compiled in.
+// Generated policies also carry the molecule's charges and Padé constants
+// (see OqJasOf); natm = 0 says that this one does not.
 template <int NOCC>
 struct OqBasisTable {
+  static constexpr int natm = 0;
   template <typename T, typename TC>
   __device__ static __forceinline__ void mo_val(const OqSystem& S, const OqSplit& SP,
                                                 const TC* __restrict__ C, double x, double y,
@@ -290,6 +293,36 @@ struct OqBasisTable {
       lp += ac[m] * ml[m];
     }
   }
+};
+
+// Nuclei and Jastrow constants of the molecule a generated policy B belongs to,
+// in the form the move and local-energy code reads them.  What the generator
+// knows is fixed at compile time: the loops over nuclei unroll, absent Padé
+// terms leave no test behind, and the constants become literals of the working
+// precision (an FP64 constant converted where it is used costs a slot of the
+// conversion unit per pair).  The coordinates stay in memory, where an FP64
+// operation can take them as an operand.
+template <class B>
+struct OqJasOf {
+  static constexpr int natm = B::natm, has_j1 = B::has_j1, has_j2 = B::has_j2;
+  struct Zs { __device__ constexpr double operator[](int i) const { return B::Z(i); } } Z;
+  struct A1 { __device__ constexpr double operator[](int i) const { return B::j1a(i); } } j1a;
+  struct B1 { __device__ constexpr double operator[](int i) const { return B::j1b(i); } } j1b;
+  struct J2 { __device__ constexpr double operator[](int i) const { return B::j2(i); } } j2;
+  const double (&nuc)[OQ_MAX_NUC][3];
+  double e_nn;
+  __device__ OqJasOf(const double (&n)[OQ_MAX_NUC][3], double e) : nuc(n), e_nn(e) {}
+};
+// The same for a table-driven policy: the system tables themselves.
+template <class B, bool GENERATED = (B::natm > 0)>
+struct OqJasSel {
+  typedef OqJasOf<B> type;
+  __device__ static type of(const OqSystem& S) { return type(S.nuc, S.e_nn); }
+};
+template <class B>
+struct OqJasSel<B, false> {
+  typedef const OqSystem& type;
+  __device__ static type of(const OqSystem& S) { return S; }
 };
 
 // ---------------------------------------------------------------------------
@@ -893,7 +926,8 @@ k_eloc(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
   double ee = 0.0, en = 0.0, lp_tot = 0.0, g2 = 0.0;
   if (live) {
     double gx, gy, gz, le;
-    oq_eloc_electron_out<NOCC, T, Real, B>(S, S, SP, C, a.pos + w, (size_t)W,
+    typename OqJasSel<B>::type J = OqJasSel<B>::of(S);
+    oq_eloc_electron_out<NOCC, T, Real, B>(J, S, SP, C, a.pos + w, (size_t)W,
                                            reinterpret_cast<const Real*>(a.ainv) + w,
                                            (size_t)W, e, ee, en, lp_tot, g2, gx, gy, gz, le);
     if (a.grad) {
@@ -1042,8 +1076,9 @@ __device__ __forceinline__ T oq_j3_delta_lane(const OqSystem& S, const double* p
 // This lane's share of the Padé and B-spline change (pairs j and nuclei I
 // congruent to lane modulo P; the terms of oq_jastrow_delta) and of the
 // MIN_DIST_THRESHOLD test.
-template <int NE, typename T>
-__device__ __forceinline__ T oq_jastrow_part(const OqSystem& S, const double* pos, int e,
+template <int NE, typename T, class SJ>
+__device__ __forceinline__ T oq_jastrow_part(const SJ& J, const OqSystem& S, const double* pos,
+                                             int e,
                                              int lane, int P, double ox, double oy, double oz,
                                              double nx, double ny, double nz, bool& valid) {
   const double thr2 = 1e-4 * 1e-4;
@@ -1058,9 +1093,9 @@ __device__ __forceinline__ T oq_jastrow_part(const OqSystem& S, const double* po
     valid = valid && (rn2 >= thr2);
     const T rn2t = (T)rn2, ro2t = (T)(bx * bx + by * by + bz * bz);
     const bool like = (e & 1) == (j & 1);
-    if (S.has_j2) {
+    if (J.has_j2) {
       const int o = like ? 0 : 2;
-      dJ += oq_pade_diff((T)S.j2[o], (T)S.j2[o + 1], rn2t * oq_rsqrt(rn2t),
+      dJ += oq_pade_diff((T)J.j2[o], (T)J.j2[o + 1], rn2t * oq_rsqrt(rn2t),
                          ro2t * oq_rsqrt(ro2t));
     }
     if (OQ_HAS_BS2(S)) {
@@ -1072,14 +1107,14 @@ __device__ __forceinline__ T oq_jastrow_part(const OqSystem& S, const double* po
     }
   }
   // the nuclei go to the lanes that the pairs load least
-  for (int I = P - 1 - lane; I < S.natm; I += P) {
-    const double ax = nx - S.nuc[I][0], ay = ny - S.nuc[I][1], az = nz - S.nuc[I][2];
+  for (int I = P - 1 - lane; I < J.natm; I += P) {
+    const double ax = nx - J.nuc[I][0], ay = ny - J.nuc[I][1], az = nz - J.nuc[I][2];
     const double rn2 = ax * ax + ay * ay + az * az;
     valid = valid && (rn2 >= thr2);
-    const double bx = ox - S.nuc[I][0], by = oy - S.nuc[I][1], bz = oz - S.nuc[I][2];
+    const double bx = ox - J.nuc[I][0], by = oy - J.nuc[I][1], bz = oz - J.nuc[I][2];
     const T rn2t = (T)rn2, ro2t = (T)(bx * bx + by * by + bz * bz);
-    if (S.has_j1)
-      dJ += oq_pade_diff((T)S.j1a[I], (T)S.j1b[I], rn2t * oq_rsqrt(rn2t), ro2t * oq_rsqrt(ro2t));
+    if (J.has_j1)
+      dJ += oq_pade_diff((T)J.j1a[I], (T)J.j1b[I], rn2t * oq_rsqrt(rn2t), ro2t * oq_rsqrt(ro2t));
     if (OQ_HAS_BS1(S) && S.bs1_type[I] >= 0) {
       const int ty = S.bs1_type[I];
       const T dinv = (T)S.bs1_dinv[ty], rc = (T)S.bs1_rcut[ty];
@@ -1099,8 +1134,8 @@ __device__ __forceinline__ V oq_group_sum(V v, int P) {
 // One sweep of a walker on its P lanes; returns the accepted moves (the same
 // on every lane).  All lanes of the warp call it; walkers beyond the tile
 // (live = false) never accept.
-template <int NOCC, typename T, typename Real, class B>
-__device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const OqSystem& S,
+template <int NOCC, typename T, typename Real, class B, class SJ>
+__device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const SJ& J, const OqSystem& S,
                                               const OqSplit& SP, const Real* C, double* pos,
                                               Real* Ai, double* rI, int lane, int P,
                                               bool live, uint32_t w, uint32_t gstep, double step,
@@ -1130,7 +1165,7 @@ __device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const OqSyst
         ny = oy + step * (double)nf[1];
         nz = oz + step * (double)nf[2];
       } else {
-        oq_scaled_propose_t<T>(S, ox, oy, oz, nf, pf, nx, ny, nz, mul, lx);
+        oq_scaled_propose_t<T>(J, ox, oy, oz, nf, pf, nx, ny, nz, mul, lx);
       }
       B::template mo_val<T, Real>(S, SP, C, nx, ny, nz, v);
     }
@@ -1152,13 +1187,13 @@ __device__ __forceinline__ int oq_sweep_lanes(const OqSweepArgs& a, const OqSyst
       bool valid;
       T dJ;
       if (sizeof(T) == 8) {
-        dJ = oq_jastrow_part<NE, T>(S, pos, ee, lane, P, ox, oy, oz, bx, by, bz, valid);
+        dJ = oq_jastrow_part<NE, T>(J, S, pos, ee, lane, P, ox, oy, oz, bx, by, bz, valid);
         if (OQ_HAS_J3(S))
           dJ += oq_j3_delta_lane<NE, T>(S, pos, rI, ee, lane, P, ox, oy, oz, bx, by, bz);
         dJ = oq_group_sum(dJ, P);
         valid = ((__ballot_sync(0xffffffffu, !valid) >> gshift) & gbits) == 0u;
       } else {
-        dJ = oq_jastrow_delta<NE, T>(S, S, pos, 1, ee, ox, oy, oz, bx, by, bz, valid);
+        dJ = oq_jastrow_delta<NE, T>(J, S, pos, 1, ee, ox, oy, oz, bx, by, bz, valid);
       }
       Real* As = Ai + s * NN;
       T R = (T)0;
@@ -1307,6 +1342,7 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
   double* pos = pos0 + wl * PP;
   Real* Ai = Ai0 + wl * AP;
   double* rI = rI0 + wl * RP;
+  typename OqJasSel<B>::type J = OqJasSel<B>::of(S);
   const double step = a.step_dev ? *a.step_dev : a.step;
   const OqScaledF pf = oq_scaled_f(step, a.scale_r0, a.scale_fmin);
   double logdet = live ? a.logdet[w] : 0.0;
@@ -1317,7 +1353,7 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
   for (int t = 0; t < a.n_sweeps; ++t) {
     const uint32_t gstep = (uint32_t)(a.step_base + t);
     if (P > 1) {
-      nacc += oq_sweep_lanes<NOCC, T, Real, B>(a, S, SP, C, pos, Ai, rI, lane, P, live, w,
+      nacc += oq_sweep_lanes<NOCC, T, Real, B>(a, J, S, SP, C, pos, Ai, rI, lane, P, live, w,
                                                gstep, step, pf, logdet);
     } else if (live) {
       for (int e = 0; e < NE; ++e) {
@@ -1334,9 +1370,9 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
           ny = oy + step * (double)nf[1];
           nz = oz + step * (double)nf[2];
         } else {
-          oq_scaled_propose_t<T>(S, ox, oy, oz, nf, pf, nx, ny, nz, mul, lx);
+          oq_scaled_propose_t<T>(J, ox, oy, oz, nf, pf, nx, ny, nz, mul, lx);
         }
-        nacc += oq_try_move_s<NOCC, T, Real, B>(S, S, SP, C, pos, 1, Ai, 1, e, nx, ny, nz, lx,
+        nacc += oq_try_move_s<NOCC, T, Real, B>(J, S, SP, C, pos, 1, Ai, 1, e, nx, ny, nz, lx,
                                                 mul, u, logdet);
       }
     }
@@ -1348,7 +1384,7 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
     if (sizeof(T) == 4) {
       if (live && lq == 0)
         for (int e = le; e < NE; e += PE)
-          oq_eloc_electron<NOCC, T, Real, B>(S, S, SP, C, pos, 1, Ai, 1, e, see,
+          oq_eloc_electron<NOCC, T, Real, B>(J, S, SP, C, pos, 1, Ai, 1, e, see,
                                              sen, slp, sg2);
     } else {
       // one electron per lane; its three-body terms split over Q lanes
@@ -1375,7 +1411,7 @@ k_sweeps(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
           for (int m = 0; m < NOCC; ++m) ac[m] = (T)Ai[(s * NOCC + m) * NOCC + i];
           T gx, gy, gz, lp;
           B::template mo_vgl_contract<T, Real>(S, SP, C, xe, ye, ze, ac, gx, gy, gz, lp);
-          oq_jastrow_vgl_coulomb<NE, T>(S, S, pos, 1, e, xe, ye, ze, jx, jy, jz, jl, see,
+          oq_jastrow_vgl_coulomb<NE, T>(J, S, pos, 1, e, xe, ye, ze, jx, jy, jz, jl, see,
                                         sen, false);
           const double sx = (double)gx, sy = (double)gy, sz = (double)gz;
           const double Gx = sx + (double)jx, Gy = sy + (double)jy, Gz = sz + (double)jz;
