@@ -5,7 +5,7 @@
 // walkers of one system is processed start to finish by one CTA:
 //   1. its positions are read from the system's (W, n_e, 3) walker array
 //      (one contiguous block, coalesced) into shared memory, walker-minor;
-//   2. the Slater inverses are rebuilt in FP64 (MO values from the tables,
+//   2. the Slater inverses are rebuilt in FP64 (generated orbital code,
 //      Gauss-Jordan with partial pivoting), stored in shared memory as Real;
 //   3. n_sweeps single-electron sweeps run with the walkers' state resident
 //      in shared memory (threads 0..WT-1, one walker each), and every
@@ -331,8 +331,8 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
   const int w = w0 + wl;
   double logdet = 0.0;
   {
-    // FP64 refresh of the spin blocks: both on the walker's
-    // thread when P = 1, spin s on lane s otherwise
+    // FP64 refresh of the spin blocks, with the generated orbitals: both on the
+    // walker's thread when P = 1, spin s on lane s otherwise
     bool ok = true;
     if (live && lane < 2) {
       for (int s = (P == 1 ? 0 : lane); s < (P == 1 ? 2 : lane + 1); ++s) {
@@ -340,8 +340,8 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
         for (int i = 0; i < NOCC; ++i) {
           const int e = 2 * i + s;
           double mv[NOCC];
-          oq_mo_val<NOCC>(S, d.C64, pos[3 * e], pos[3 * e + 1],
-                          pos[3 * e + 2], mv);
+          B::template mo_val<double, double>(S, SP, d.C64, pos[3 * e], pos[3 * e + 1],
+                                             pos[3 * e + 2], mv);
 #pragma unroll
           for (int m = 0; m < NOCC; ++m) Sm[i][m] = mv[m];
         }

@@ -104,7 +104,7 @@ __device__ __forceinline__ void oq_ao_add(const double* C, double v, double (&mv
 }
 
 // The three AOs of a p function, added to each other first (the order of
-// oq_mo_val, so that the persistent kernel's refresh gives the same values).
+// oq_mo_val).
 template <int N>
 __device__ __forceinline__ void oq_ao_add3(const double* C, double v0, double v1, double v2,
                                            double (&mv)[N]) {
