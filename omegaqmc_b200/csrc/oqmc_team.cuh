@@ -43,11 +43,13 @@ constexpr size_t oq_team_tile_bytes(int n, int wb) {
 
 // Walkers per tile for W walkers: the largest tile (whole warps of one
 // electron, conflict-free shared memory) unless that leaves SMs idle; then
-// halved until there are four tiles per SM or a tile is one warp.
+// halved until there are four tiles per SM, or, once a tile has no more than
+// 128 threads (below that threads would idle), one per SM or a tile is a warp.
 template <int N>
 inline int oq_team_walkers(int W) {
+  constexpr int NE = OqTeam<N>::NE;
   int wb = OqTeam<N>::WB;
-  while (wb > 1 && wb * OqTeam<N>::NE > 32 && (W + wb - 1) / wb < 4 * 148) wb >>= 1;
+  while (wb > 1 && wb * NE > 32 && (W + wb - 1) / wb < (wb * NE > 128 ? 4 * 148 : 148)) wb >>= 1;
   return wb;
 }
 
