@@ -6,8 +6,8 @@ then the local energy of every walker is evaluated and reduced.  A full FP64
 LU refresh of each inverse runs every 50 sweeps inside the timed region.
 Default path: one fused persistent launch per 50 sweeps (refresh, moves,
 local energies; the batched entry points with one molecule), the timed
-launches replayed from a CUDA graph; --path split runs the separate move and
-local-energy kernels through oqmc_sweeps.
+launches replayed from a CUDA graph; --path split runs oqmc_sweeps (moves and
+local energies of 50 sweeps in one launch) and the refresh between its calls.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
                     [--precision mixed|fp64] [--system H2O] [--walkers 65536]
@@ -99,7 +99,8 @@ def parse():
                          "per-output errors)")
     ap.add_argument("--path", default="persistent", choices=["persistent", "split"],
                     help="persistent: one fused launch per 50 sweeps (refresh, moves, E_L) "
-                         "under a CUDA graph; split: separate move / local-energy kernels")
+                         "under a CUDA graph; split: oqmc_sweeps (moves and E_L of 50 sweeps "
+                         "in one launch, refresh in its own)")
     ap.add_argument("--quick", action="store_true",
                     help="profiling mode: no equilibration, comparison, e2e or CPU legs")
     ap.add_argument("--generic", action="store_true",
@@ -308,8 +309,8 @@ def kappa_spread(series, parts):
 
 
 def sweep_launches(ens, n_sweeps, measure_every=1):
-    """Kernels that ``ens.run(n_sweeps)`` launches from the ensemble's current
-    refresh phase (the chunking of WalkerEnsemble.run): per oqmc_sweeps call a
+    """Kernels that ``ens.run(n_sweeps)`` launches with the learned proposal from
+    the ensemble's current refresh phase (the chunking of WalkerEnsemble.run): per oqmc_sweeps call a
     layout conversion in and one out, per measurement a move kernel and a
     local-energy kernel (one more move kernel for sweeps after the last
     measurement of a call), per FP64 refresh a conversion and the refresh
@@ -322,6 +323,29 @@ def sweep_launches(ens, n_sweeps, measure_every=1):
             chunk = min(chunk, n_sweeps - done)
         m = chunk // measure_every
         n += 2 + 2 * m + (1 if chunk > m * measure_every else 0)
+        done += chunk
+        since += chunk
+        if since >= ens.refresh_every:
+            n += 2
+            since = 0
+    return n
+
+
+def fused_launches(ens, n_sweeps, measure_every=1, tensor_core_energy=False):
+    """Kernels that ``ens.run(n_sweeps)`` launches where the sweeps are fused
+    (single-electron sweeps and FP64 all-electron steps): one per oqmc_sweeps
+    call, or with the tensor-core local energy a sweep and an energy kernel
+    per measurement (one more sweep kernel for sweeps after the last
+    measurement of a call); per FP64 refresh a conversion and the refresh
+    kernel."""
+    since, n, done = ens.since_refresh, 0, 0
+    while done < n_sweeps:
+        chunk = min(n_sweeps - done, ens.refresh_every - since)
+        if measure_every > 1:
+            chunk = max(measure_every, chunk - chunk % measure_every)
+            chunk = min(chunk, n_sweeps - done)
+        m = chunk // measure_every
+        n += 2 * m + (1 if chunk > m * measure_every else 0) if tensor_core_energy else 1
         done += chunk
         since += chunk
         if since >= ens.refresh_every:
@@ -429,7 +453,7 @@ def run_ours(a):
     sums = torch.zeros(K, NSUM, dtype=torch.float64, device=dev)
     ev0 = torch.cuda.Event(enable_timing=True)
     ev1 = torch.cuda.Event(enable_timing=True)
-    n_launch = sweep_launches(ens, K)
+    n_launch = fused_launches(ens, K, 1, a.eloc == "tc" and a.precision == "mixed")
     if world > 1:
         dist.barrier()
     torch.cuda.synchronize()
@@ -570,7 +594,7 @@ def run_ours(a):
         "roofline": {"bound": "fp64" if peak_kind == 0 else "fp32",
                      "achieved": achieved / 1e12, "peak": rate / 1e12, "unit": "TFLOP/s",
                      "frac": achieved / rate if rate else None, "traffic": traffic,
-                     "kernel": "k_moves+k_eloc (one 50-sweep oqmc_sweeps call)",
+                     "kernel": "k_sweeps (one 50-sweep oqmc_sweeps call)",
                      "kernel_ms_per_launch": sweep_ms,
                      "refresh_ms_per_launch": refresh_ms,
                      "flops_per_walker_sweep": work["flops"],
@@ -1389,7 +1413,7 @@ def run_alle(a):
     sums = torch.zeros(K, NSUM, dtype=torch.float64, device=dev)
     ev0 = torch.cuda.Event(enable_timing=True)
     ev1 = torch.cuda.Event(enable_timing=True)
-    n_launch = sweep_launches(ens, K)
+    n_launch = fused_launches(ens, K)
     if world > 1:
         dist.barrier()
     torch.cuda.synchronize()

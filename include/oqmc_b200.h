@@ -244,8 +244,8 @@ int oqmc_basin(oqmc_ctx* ctx, double* walkers, int W, void* state, int precision
  * per-thread local memory than the device's current stack limit
  * (cudaLimitStackSize) returns OQ_ERR_UNSUPPORTED instead of letting the
  * driver grow its local-memory reservation: at the default 1 KiB this
- * refuses all-electron steps and multi-determinant trials until an
- * allocating call has raised the limit.  All calls share the array: calls
+ * refuses multi-determinant trials until an allocating call has raised the
+ * limit.  All calls share the array: calls
  * that overlap on the GPU race, so serialise them. */
 int oqmc_sweeps_noalloc(oqmc_ctx* ctx, double* walkers, int W, int precision,
                         int n_sweeps, int measure_every, double step,
@@ -269,9 +269,7 @@ int oqmc_set_proposal(oqmc_ctx* ctx, int kind, double r0, double fmin_frac);
  * to single-electron sweeps only; the learned proposal, multi-determinant
  * trials and oqmc_batch_bind refuse kind 1.  The accepted-move sum counts
  * electron moves in both kinds: an accepted all-electron step adds n_e.
- * The all-electron kernel's per-thread stack exceeds the default local-memory
- * reservation, so oqmc_sweeps_noalloc refuses kind 1 on a device whose stack
- * limit has not been raised (see there). */
+ * FP64 steps and their local energies run in one launch per call. */
 int oqmc_set_move_kind(oqmc_ctx* ctx, int kind);
 /* Multi-determinant trial (the `trial` dict of get_psi_fun /
  * get_vmc_gto_func, OmegaQMC/psi/gto.py:846-863, 1312-1488):

@@ -1,7 +1,13 @@
 // Learned proposal network: training-data features, inference, training
 // (forward + backward on the tensor cores) and the Adam update.
 //
-// Training step of one CTA (128 rows, thread t = row t = TMEM lane t):
+// Training step of one CTA (128 rows, row t = TMEM lane t, two threads per row:
+// t for columns 0-63 of every epilogue and t + 128 for the rest, and in the
+// loss threads 128-255 fetch the first transposed weights; a CTA is a chain of
+// nine MMA steps with short epilogues, four warps of them waited on each
+// other's stores, so the chain is shortened by splitting the epilogues and by
+// loading W^T behind the previous step's MMAs: backward() of 8,192 rows, 102.6
+// -> 93.1 us with its two host reads):
 //   forward   X0 -> H1 -> H2 -> H3 -> out (4 MMA chains into TMEM columns
 //             [0,128)), keeping H_l^T (features x rows, K-major) in shared
 //             memory for the weight gradients and the ReLU masks in
@@ -14,7 +20,7 @@
 //             dZ_{l-1} = dH_{l-1} * ReLU'(Z_{l-1}) overwrites H_{l-1}^T in
 //             place once its MMA has read it; bias gradients are the row sums
 //             of dZ^T.  Gradients are added to the global FP32 buffer with
-//             atomics (one add per parameter per CTA).
+//             atomics (one add per parameter per CTA, two per bias).
 // Every MMA operand is BF16 (as the oracle emulates), every accumulation
 // FP32.  Waits on the MMA mbarrier are bounded; a timeout sets
 // OQ_FLAG_TIMEOUT, stops the CTA's work and frees its TMEM.
@@ -49,11 +55,11 @@
 
 static_assert(TR_SMEM <= 232448, "training tile exceeds shared memory");
 
-// Sum of row n (128 BF16 values) of a [rows x 128] K-major buffer.
-__device__ __forceinline__ float oq_mlp_rowsum(const unsigned char* buf, int n) {
+// Sum of 64 values (half h) of row n of a [rows x 128] K-major buffer.
+__device__ __forceinline__ float oq_mlp_rowsum(const unsigned char* buf, int n, int h) {
   float s = 0.0f;
-#pragma unroll 4
-  for (int c = 0; c < 16; ++c) {
+#pragma unroll
+  for (int c = 8 * h; c < 8 * h + 8; ++c) {
     const uint4 q = *reinterpret_cast<const uint4*>(buf + (((n >> 3) * 16 + c) << 7) + ((n & 7) << 4));
     s += oq_bf16_lo(q.x) + oq_bf16_hi(q.x) + oq_bf16_lo(q.y) + oq_bf16_hi(q.y) +
          oq_bf16_lo(q.z) + oq_bf16_hi(q.z) + oq_bf16_lo(q.w) + oq_bf16_hi(q.w);
@@ -61,35 +67,35 @@ __device__ __forceinline__ float oq_mlp_rowsum(const unsigned char* buf, int n) 
   return s;
 }
 
-// dZ = dH (TMEM row r) * ReLU mask; BF16 into act (KC = 16, may be null) and
-// transposed into ht.
+// dZ = dH (TMEM row r) * ReLU mask, columns c_begin .. c_begin + 63; BF16 into
+// act (KC = 16, may be null) and transposed into ht.
 __device__ __forceinline__ void oq_mlp_dz_epilogue(uint32_t trow, const uint32_t* mask,
-                                                   unsigned char* act, int r, unsigned char* ht) {
-#pragma unroll 1
-  for (int c0 = 0; c0 < OQ_MLP_H; c0 += 16) {
-    float v[16];
-    oq_tmem_ld16(trow + (uint32_t)c0, v);
+                                                   unsigned char* act, int r, unsigned char* ht,
+                                                   int c_begin) {
+  uint32_t raw[64];
+#pragma unroll
+  for (int q = 0; q < 4; ++q)
+    oq_tmem_ld16_nw(trow + (uint32_t)(c_begin + 16 * q), raw + 16 * q);
+  oq_tmem_wait_ld();
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const int c0 = c_begin + 16 * q;
     const uint32_t mb = mask[c0 >> 5] >> (c0 & 16);
+    float v[16];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) v[j] = ((mb >> j) & 1u) ? v[j] : 0.0f;
+    for (int j = 0; j < 16; ++j)
+      v[j] = ((mb >> j) & 1u) ? __uint_as_float(raw[16 * q + j]) : 0.0f;
     if (act) oq_mlp_store_row16(act, r, c0, 16, v);
-#pragma unroll
-    for (int j = 0; j < 16; j += 2) {
-      const uint32_t p = oq_bf16x2(v[j], v[j + 1]);
-      *reinterpret_cast<unsigned short*>(ht + oq_kmajor_off2(c0 + j, r, 16)) =
-          (unsigned short)(p & 0xFFFFu);
-      *reinterpret_cast<unsigned short*>(ht + oq_kmajor_off2(c0 + j + 1, r, 16)) =
-          (unsigned short)(p >> 16);
-    }
+    oq_mlp_store_col16(ht, r, c0, v);
   }
 }
 
-// Read ncol columns of TMEM row r (a weight-gradient row) and add them to
-// grad[base + col * stride].
-__device__ __forceinline__ void oq_mlp_flush_grad(uint32_t trow, int ncol, float* grad,
-                                                  int base, int stride) {
+// Read columns [c_begin, c_end) (multiples of 16) of TMEM row r (a
+// weight-gradient row) and add them to grad[base + col * stride].
+__device__ __forceinline__ void oq_mlp_flush_grad(uint32_t trow, int c_begin, int c_end,
+                                                  float* grad, int base, int stride) {
 #pragma unroll 1
-  for (int c0 = 0; c0 < ncol; c0 += 16) {
+  for (int c0 = c_begin; c0 < c_end; c0 += 16) {
     float v[16];
     oq_tmem_ld16(trow + (uint32_t)c0, v);
 #pragma unroll
@@ -97,7 +103,7 @@ __device__ __forceinline__ void oq_mlp_flush_grad(uint32_t trow, int ncol, float
   }
 }
 
-__global__ void __launch_bounds__(128, 1)
+__global__ void __launch_bounds__(256, 1)
 k_mlp_train(const unsigned short* __restrict__ feat, const float* __restrict__ target, int R,
             float scale, const unsigned short* __restrict__ wbf,
             const unsigned short* __restrict__ wtbf, const float* __restrict__ theta,
@@ -109,16 +115,21 @@ k_mlp_train(const unsigned short* __restrict__ feat, const float* __restrict__ t
   unsigned char* ht2 = smem + TR_HT2;
   unsigned char* ht3 = smem + TR_HT3;
   unsigned char* wreg = smem + TR_W;
+  // backward operands over the forward weights: W4^T (12 KB) at 0, dZ4^T (12 KB)
+  // at 32 KB, W3^T (32 KB) at 48 KB, W2^T over W4^T
   unsigned char* z4t = wreg + 32768;
+  unsigned char* w3t = wreg + 49152;
   float* bias = reinterpret_cast<float*>(smem + TR_BIAS);
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + TR_BAR);
   uint32_t* slot = reinterpret_cast<uint32_t*>(smem + TR_BAR + 8);
-  const int t = threadIdx.x, warp = t >> 5;
-  const int row = blockIdx.x * 128 + t;
+  // two threads per row: threads 128-255 (the same TMEM lane quarters) take
+  // columns 64-127 of every epilogue
+  const int t = threadIdx.x & 127, h = threadIdx.x >> 7, warp = threadIdx.x >> 5;
+  const int row = blockIdx.x * 128 + t, ch = 64 * h;
   const bool valid = row < R;
   if (warp == 0) oq_tmem_alloc(slot, 256);
-  if (t == 0) oq_mbar_init(bar, 1);
-  {
+  if (threadIdx.x == 0) oq_mbar_init(bar, 1);
+  if (h == 0) {
     uint4 q[4] = {};
     if (valid) {
       const uint4* s = reinterpret_cast<const uint4*>(feat + (size_t)row * OQ_MLP_K0);
@@ -126,9 +137,9 @@ k_mlp_train(const unsigned short* __restrict__ feat, const float* __restrict__ t
     }
     for (int c = 0; c < 4; ++c)
       *reinterpret_cast<uint4*>(act + (((t >> 3) * 4 + c) << 7) + ((t & 7) << 4)) = q[c];
-    const unsigned short* h = reinterpret_cast<const unsigned short*>(q);
+    const unsigned short* f = reinterpret_cast<const unsigned short*>(q);
     for (int k = 0; k < OQ_MLP_K0; ++k)
-      *reinterpret_cast<unsigned short*>(ht0 + oq_kmajor_off2(k, t, 16)) = h[k];
+      *reinterpret_cast<unsigned short*>(ht0 + oq_kmajor_off2(k, t, 16)) = f[k];
   }
   float dtg[3] = {0.0f, 0.0f, 0.0f};
   if (valid) {
@@ -142,7 +153,7 @@ k_mlp_train(const unsigned short* __restrict__ feat, const float* __restrict__ t
   __syncthreads();
   oq_tc_fence_after();
   const uint32_t tmem = *slot;
-  const uint32_t lane = (uint32_t)(warp * 32) << 16;
+  const uint32_t lane = (uint32_t)((warp & 3) * 32) << 16;
   const uint32_t t1 = tmem + lane, t2 = tmem + 128 + lane;
   OqMlpSync sy{bar, 0u};
   uint32_t mask[12];
@@ -151,26 +162,29 @@ k_mlp_train(const unsigned short* __restrict__ feat, const float* __restrict__ t
   unsigned char* hts[3] = {ht1, ht2, ht3};
   bool ok = oq_mlp_forward_tile(act, wreg, bias, tmem, sy, out, hts, mask);
   if (ok) {
-    float g[OQ_MLP_NOUT];
-    double nl = 0.0;
-    if (valid) {
-      nl = oq_mix_nll_grad(out, dtg, scale, g);
+    if (h == 0) {
+      float g[OQ_MLP_NOUT];
+      double nl = 0.0;
+      if (valid) {
+        nl = oq_mix_nll_grad(out, dtg, scale, g);
+      } else {
+        for (int j = 0; j < OQ_MLP_NOUT; ++j) g[j] = 0.0f;
+      }
+      double s = nl;
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if ((t & 31) == 0 && loss_sum) atomicAdd(loss_sum, s);
+      // dZ4 (rows x 48) and its transpose
+      for (int c0 = 0; c0 < OQ_MLP_NOUT; c0 += 16) {
+        oq_mlp_store_row16(act, t, c0, 6, g + c0);
+        oq_mlp_store_col16(z4t, t, c0, g + c0);
+      }
     } else {
-      for (int j = 0; j < OQ_MLP_NOUT; ++j) g[j] = 0.0f;
+      // meanwhile W4^T and W3^T over the forward weights
+      oq_mlp_load_kmajor_part(wreg, wtbf + OQ_MLP_OFF_W4, OQ_MLP_H, OQ_MLP_NOUT, t, 128);
+      oq_mlp_load_kmajor_part(w3t, wtbf + OQ_MLP_OFF_W3, OQ_MLP_H, OQ_MLP_H, t, 128);
     }
-    double s = nl;
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((t & 31) == 0 && loss_sum) atomicAdd(loss_sum, s);
-    // dZ4 (rows x 48) and its transpose; W4^T into the weight region
-    for (int c0 = 0; c0 < OQ_MLP_NOUT; c0 += 16) oq_mlp_store_row16(act, t, c0, 6, g + c0);
-    for (int j = 0; j < OQ_MLP_NOUT; j += 2) {
-      const uint32_t p = oq_bf16x2(g[j], g[j + 1]);
-      *reinterpret_cast<unsigned short*>(z4t + oq_kmajor_off2(j, t, 16)) = (unsigned short)(p & 0xFFFFu);
-      *reinterpret_cast<unsigned short*>(z4t + oq_kmajor_off2(j + 1, t, 16)) = (unsigned short)(p >> 16);
-    }
-    oq_mlp_load_kmajor(wreg, wtbf + OQ_MLP_OFF_W4, OQ_MLP_H, OQ_MLP_NOUT);
     oq_mlp_pre_issue();
-    if (t == 0) {
+    if (threadIdx.x == 0) {
       const uint32_t a0 = oq_smem_addr(act), b0 = oq_smem_addr(wreg);
       for (int ks = 0; ks < OQ_MLP_NOUT / 16; ++ks)
         oq_mma_bf16(tmem, oq_desc_kmajor(a0 + ks * 256u, 128u, 6u * 128u),
@@ -186,53 +200,42 @@ k_mlp_train(const unsigned short* __restrict__ feat, const float* __restrict__ t
     ok = oq_mlp_wait(sy);
   }
   if (ok) {
-    if (t < OQ_MLP_NOUT) {
-      // row t of dZ4^T, 128 rows of the tile
-      float sb = 0.0f;
-      for (int c = 0; c < 16; ++c) {
-        const uint4 q = *reinterpret_cast<const uint4*>(z4t + (((t >> 3) * 16 + c) << 7) + ((t & 7) << 4));
-        sb += oq_bf16_lo(q.x) + oq_bf16_hi(q.x) + oq_bf16_lo(q.y) + oq_bf16_hi(q.y) +
-              oq_bf16_lo(q.z) + oq_bf16_hi(q.z) + oq_bf16_lo(q.w) + oq_bf16_hi(q.w);
-      }
-      atomicAdd(grad + OQ_MLP_OFF_B4 + t, sb);
-    }
-    oq_mlp_flush_grad(t2, OQ_MLP_NOUT, grad, OQ_MLP_OFF_W4 + t, OQ_MLP_H);   // dW4[n][t]
-    oq_mlp_dz_epilogue(t1, mask + 8, act, t, ht3);                          // dZ3
-    oq_tc_fence_before();
-    __syncthreads();
-    oq_mlp_load_kmajor(wreg, wtbf + OQ_MLP_OFF_W3, OQ_MLP_H, OQ_MLP_H);
+    if (t < OQ_MLP_NOUT) atomicAdd(grad + OQ_MLP_OFF_B4 + t, oq_mlp_rowsum(z4t, t, h));
+    oq_mlp_flush_grad(t2, 32 * h, h ? OQ_MLP_NOUT : 32, grad, OQ_MLP_OFF_W4 + t,
+                      OQ_MLP_H);                                              // dW4[n][t]
+    oq_mlp_dz_epilogue(t1, mask + 8, act, t, ht3, ch);                        // dZ3
     oq_mlp_pre_issue();
-    if (t == 0) {
-      oq_mlp_mma(tmem, act, wreg, OQ_MLP_H, OQ_MLP_H, nullptr);
+    if (threadIdx.x == 0) {
+      oq_mlp_mma(tmem, act, w3t, OQ_MLP_H, OQ_MLP_H, nullptr);
       oq_mlp_mma(tmem + 128, ht2, ht3, OQ_MLP_H, OQ_MLP_H, bar);
     }
+    // W2^T over W4^T and dZ4^T, which the finished MMAs have read, while
+    // these run
+    oq_mlp_load_kmajor(wreg, wtbf + OQ_MLP_OFF_W2, OQ_MLP_H, OQ_MLP_H);
     ok = oq_mlp_wait(sy);
   }
   if (ok) {
-    atomicAdd(grad + OQ_MLP_OFF_B3 + t, oq_mlp_rowsum(ht3, t));
-    oq_mlp_flush_grad(t2, OQ_MLP_H, grad, OQ_MLP_OFF_W3 + t, OQ_MLP_H);
-    oq_mlp_dz_epilogue(t1, mask + 4, act, t, ht2);                          // dZ2
-    oq_tc_fence_before();
-    __syncthreads();
-    oq_mlp_load_kmajor(wreg, wtbf + OQ_MLP_OFF_W2, OQ_MLP_H, OQ_MLP_H);
+    atomicAdd(grad + OQ_MLP_OFF_B3 + t, oq_mlp_rowsum(ht3, t, h));
+    oq_mlp_flush_grad(t2, ch, ch + 64, grad, OQ_MLP_OFF_W3 + t, OQ_MLP_H);
+    oq_mlp_dz_epilogue(t1, mask + 4, act, t, ht2, ch);                        // dZ2
     oq_mlp_pre_issue();
-    if (t == 0) {
+    if (threadIdx.x == 0) {
       oq_mlp_mma(tmem, act, wreg, OQ_MLP_H, OQ_MLP_H, nullptr);
       oq_mlp_mma(tmem + 128, ht1, ht2, OQ_MLP_H, OQ_MLP_H, bar);
     }
     ok = oq_mlp_wait(sy);
   }
   if (ok) {
-    atomicAdd(grad + OQ_MLP_OFF_B2 + t, oq_mlp_rowsum(ht2, t));
-    oq_mlp_flush_grad(t2, OQ_MLP_H, grad, OQ_MLP_OFF_W2 + t, OQ_MLP_H);
-    oq_mlp_dz_epilogue(t1, mask, nullptr, t, ht1);                          // dZ1^T
+    atomicAdd(grad + OQ_MLP_OFF_B2 + t, oq_mlp_rowsum(ht2, t, h));
+    oq_mlp_flush_grad(t2, ch, ch + 64, grad, OQ_MLP_OFF_W2 + t, OQ_MLP_H);
+    oq_mlp_dz_epilogue(t1, mask, nullptr, t, ht1, ch);                        // dZ1^T
     oq_mlp_pre_issue();
-    if (t == 0) oq_mlp_mma(tmem, ht1, ht0, OQ_MLP_K0, OQ_MLP_H, bar);       // dW1 [128 x 32]
+    if (threadIdx.x == 0) oq_mlp_mma(tmem, ht1, ht0, OQ_MLP_K0, OQ_MLP_H, bar);  // dW1 [128 x 32]
     ok = oq_mlp_wait(sy);
   }
   if (ok) {
-    atomicAdd(grad + OQ_MLP_OFF_B1 + t, oq_mlp_rowsum(ht1, t));
-    oq_mlp_flush_grad(t1, OQ_MLP_K0, grad, OQ_MLP_OFF_W1 + t * OQ_MLP_K0, 1);
+    atomicAdd(grad + OQ_MLP_OFF_B1 + t, oq_mlp_rowsum(ht1, t, h));
+    oq_mlp_flush_grad(t1, 16 * h, 16 * h + 16, grad, OQ_MLP_OFF_W1 + t * OQ_MLP_K0, 1);
   }
   oq_tc_fence_before();
   __syncthreads();
@@ -241,7 +244,7 @@ k_mlp_train(const unsigned short* __restrict__ feat, const float* __restrict__ t
     if (!ok) oq_mbar_wait(bar, sy.phase ^ 1u);   // let an outstanding MMA drain
     oq_tmem_dealloc(tmem, 256);
   }
-  if (!ok && t == 0) atomicOr(flags, OQ_FLAG_TIMEOUT);
+  if (!ok && threadIdx.x == 0) atomicOr(flags, OQ_FLAG_TIMEOUT);
 }
 
 __global__ void __launch_bounds__(128, 1)
@@ -391,7 +394,7 @@ static int train_kernel(oqmc_mlp* m, const unsigned short* feat, const float* ta
                                      TR_SMEM));
     attr = true;
   }
-  k_mlp_train<<<(R + 127) / 128, 128, TR_SMEM, s>>>(feat, target, R, 1.0f / (float)R, m->wbf,
+  k_mlp_train<<<(R + 127) / 128, 256, TR_SMEM, s>>>(feat, target, R, 1.0f / (float)R, m->wbf,
                                                     m->wtbf, m->theta, grad, loss, m->d_flags);
   OQ_MCUDA(m, cudaGetLastError());
   return OQ_OK;

@@ -51,16 +51,21 @@ __device__ __forceinline__ float oq_bf16_lo(uint32_t v) { return __uint_as_float
 __device__ __forceinline__ float oq_bf16_hi(uint32_t v) { return __uint_as_float(v & 0xFFFF0000u); }
 
 // Copy a row-major BF16 matrix [N][K] from global memory into the canonical
-// K-major layout (16-byte chunks; K a multiple of 8).
-__device__ __forceinline__ void oq_mlp_load_kmajor(unsigned char* dst,
-                                                   const unsigned short* __restrict__ src,
-                                                   int N, int K) {
+// K-major layout (16-byte chunks; K a multiple of 8): thread tid of nt.
+__device__ __forceinline__ void oq_mlp_load_kmajor_part(unsigned char* dst,
+                                                        const unsigned short* __restrict__ src,
+                                                        int N, int K, int tid, int nt) {
   const int KC = K / 8;
   const uint4* s4 = reinterpret_cast<const uint4*>(src);
-  for (int i = threadIdx.x; i < N * KC; i += blockDim.x) {
+  for (int i = tid; i < N * KC; i += nt) {
     const int n = i / KC, c = i - n * KC;
     *reinterpret_cast<uint4*>(dst + (((n >> 3) * KC + c) << 7) + ((n & 7) << 4)) = s4[i];
   }
+}
+__device__ __forceinline__ void oq_mlp_load_kmajor(unsigned char* dst,
+                                                   const unsigned short* __restrict__ src,
+                                                   int N, int K) {
+  oq_mlp_load_kmajor_part(dst, src, N, K, threadIdx.x, blockDim.x);
 }
 
 // Store 16 FP32 values (columns c0..c0+15 of row r) as BF16 into a K-major
@@ -76,6 +81,23 @@ __device__ __forceinline__ void oq_mlp_store_row16(unsigned char* buf, int r, in
   unsigned char* p = buf + (((r >> 3) * KC + c) << 7) + ((r & 7) << 4);
   *reinterpret_cast<uint4*>(p) = a;
   *reinterpret_cast<uint4*>(p + 128) = b;
+}
+
+// Store the same 16 values transposed: row r's entry of rows c0..c0+15 of a
+// [features x 128 rows] buffer (KC = 16).  Neighbouring rows share 4-byte
+// words, so lane pairs exchange one packed word per two features and each
+// stores one feature's word (half the stores of 2-byte writes).  All lanes of
+// the warp call this.
+__device__ __forceinline__ void oq_mlp_store_col16(unsigned char* ht, int r, int c0,
+                                                   const float v[16]) {
+  const int odd = r & 1;
+#pragma unroll
+  for (int j = 0; j < 16; j += 2) {
+    const uint32_t p = oq_bf16x2(v[j], v[j + 1]);
+    const uint32_t q = __shfl_xor_sync(0xffffffffu, p, 1);
+    *reinterpret_cast<uint32_t*>(ht + oq_kmajor_off2(c0 + j + odd, r & ~1, 16)) =
+        odd ? __byte_perm(q, p, 0x7632) : __byte_perm(p, q, 0x5410);
+  }
 }
 
 // Issue D[128 x N] = A[128 x K] B[N x K]^T (both K-major canonical, BF16)
@@ -145,14 +167,7 @@ __device__ __forceinline__ void oq_mlp_hidden_epilogue(uint32_t tmem_row, const 
       oq_mlp_store_row16(act, r, c0, 16, v);
       if (mask) mask[c0 >> 5] |= mbits << (c0 & 16);
       if (ht) {
-#pragma unroll
-        for (int j = 0; j < 16; j += 2) {
-          const uint32_t p = oq_bf16x2(v[j], v[j + 1]);
-          *reinterpret_cast<unsigned short*>(ht + oq_kmajor_off2(c0 + j, r, 16)) =
-              (unsigned short)(p & 0xFFFFu);
-          *reinterpret_cast<unsigned short*>(ht + oq_kmajor_off2(c0 + j + 1, r, 16)) =
-              (unsigned short)(p >> 16);
-        }
+        oq_mlp_store_col16(ht, r, c0, v);
       }
     }
   }
@@ -200,7 +215,7 @@ __device__ __forceinline__ void oq_mlp_load_weights(unsigned char* wreg,
 // KC = 4); leaves row r's 48 outputs in `out` of thread r (r < 128).
 // With 256 threads, threads 128-255 (warps 4-7, the same TMEM lane quarters
 // as warps 0-3) write columns 64-127 of every hidden layer and threads
-// 0-127 columns 0-63.  `ht`/`mask` (training, 128 threads) receive the
+// 0-127 columns 0-63.  `ht`/`mask` (training) receive the
 // transposed hidden activations and ReLU masks of layers 1..3.  Returns
 // false when an MMA wait timed out (uniform over the CTA).
 __device__ __forceinline__ bool oq_mlp_forward_tile(unsigned char* act, const unsigned char* wreg,

@@ -77,8 +77,8 @@ extern "C" int oqmc_sweeps_noalloc(oqmc_ctx* ctx, double* walkers, int W, int pr
   if (W == 0 || n_sweeps == 0) return OQ_OK;
   // a kernel whose per-thread local memory exceeds the device's current
   // stack limit makes the driver grow its local-memory reservation at launch,
-  // which is a device allocation (the all-electron step and the
-  // multi-determinant kernels need more than the default 1 KiB)
+  // which is a device allocation (the multi-determinant kernels need more
+  // than the default 1 KiB)
   size_t lmem = 0, limit = 0;
   const int lrc = oq_ctx_sweep_local_bytes(ctx, precision, &lmem);
   if (lrc != OQ_OK) return lrc;
