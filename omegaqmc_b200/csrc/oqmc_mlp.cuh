@@ -450,11 +450,14 @@ __device__ __forceinline__ void oq_mix_sample_f(const float out[OQ_MLP_NOUT], fl
 __device__ __forceinline__ double oq_mix_nll_grad(const float out[OQ_MLP_NOUT], const float d[3],
                                                   float scale, float g[OQ_MLP_NOUT]) {
   double amax = -1e300;
+#pragma unroll
   for (int c = 0; c < OQ_MLP_NMIX; ++c) amax = fmax(amax, (double)out[c]);
   double zs = 0.0;
+#pragma unroll
   for (int c = 0; c < OQ_MLP_NMIX; ++c) zs += exp((double)out[c] - amax);
   const double lz = amax + log(zs);
   double L[OQ_MLP_NMIX], sg[OQ_MLP_NMIX], r2[OQ_MLP_NMIX], lmax = -1e300;
+#pragma unroll
   for (int c = 0; c < OQ_MLP_NMIX; ++c) {
     sg[c] = OQ_MLP_SIGMIN + oq_softplus((double)out[32 + c]);
     const double ex = d[0] - out[8 + 3 * c], ey = d[1] - out[9 + 3 * c], ez = d[2] - out[10 + 3 * c];
@@ -463,9 +466,12 @@ __device__ __forceinline__ double oq_mix_nll_grad(const float out[OQ_MLP_NOUT], 
     lmax = fmax(lmax, L[c]);
   }
   double s = 0.0;
+#pragma unroll
   for (int c = 0; c < OQ_MLP_NMIX; ++c) s += exp(L[c] - lmax);
   const double lq = lmax + log(s);
+#pragma unroll
   for (int j = 0; j < OQ_MLP_NOUT; ++j) g[j] = 0.0f;
+#pragma unroll
   for (int c = 0; c < OQ_MLP_NMIX; ++c) {
     const double gam = exp(L[c] - lq);
     const double w = exp((double)out[c] - lz);

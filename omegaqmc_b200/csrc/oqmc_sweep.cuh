@@ -1,11 +1,10 @@
 // Single-electron Metropolis sweeps with Sherman-Morrison inverse updates.
 //
-// One thread per walker.  A CTA copies the system tables and its walkers'
-// state (positions, the two inverse Slater matrices) into shared memory
-// once, runs n_sweeps sweeps without touching HBM except to reduce the
-// local energy of each measured sweep, and writes the state back at the end.
-// Shared-memory walker arrays are walker-minor so that a warp's 32 walkers
-// read 32 consecutive words.
+// A CTA copies the system tables and its walkers' state (positions, the two
+// inverse Slater matrices) into shared memory once, runs all sweeps of a call
+// without touching HBM except to reduce the local energy of each measured
+// sweep, and writes the state back at the end.  One to 32 threads of a warp
+// share a walker (k_sweeps); a walker's state is contiguous, at an odd pitch.
 //
 // A sweep moves every electron once (Gaussian proposal of width `step`,
 // exact Metropolis acceptance |R|^2 exp(2 dJ) with R the determinant ratio
