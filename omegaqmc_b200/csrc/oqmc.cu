@@ -127,10 +127,80 @@ static void compute_split(oqmc_ctx* ctx) {
 
 // Record an error on a context (used by entry points in other files).
 
+// Lanes per walker of the sweeps: as many as there are electrons (all orbital
+// rows of a sweep at once; 32 with three-body terms in FP64, which fill them),
+// halved while the threads would exceed 512 per SM.  Beyond that the register
+// file (128 per thread) is full and lanes only add shuffles.
+//
+// Three-body terms in FP32 are the exception: every lane sums all of them (the
+// order of that sum decides moves), so lanes repeat that work and pay only
+// while it hides in idle issue slots: all lanes up to a number of threads per
+// SM, one lane beyond.  Five sweeps, us, all lanes | one lane: H2O 2,048
+// walkers 3,316 | 3,459, 4,096: 3,933 | 3,459; orders (3, 3) 512 walkers 4,311
+// | 4,352, 4,096: 5,844 | 4,369; LiH
+// 8,192: 451 | 520, 16,384: 553 | 520; (H2O)2 2,048: 7,643 |
+// 11,000, 16 lanes at 4,096: 9,787 | 11,160.
+static int sweep_lanes(const oqmc_ctx* ctx, int W, int mixed) {
+  int P = 1;
+  while (P < ctx->n_e && P < 32) P <<= 1;
+  const OqSystem& S = ctx->hsys;
+  if (S.has_j3 && mixed) {
+    const int gammas = (S.j3_nI + 1) * (S.j3_nI + 1) * (S.j3_nE + 1);
+    const long long cap = 148ll * (P == 2 || P == 32 ? 512 : gammas > 27 ? 128 : 256);
+    if (P == 32 && (long long)W * P > cap) P = 16;
+    return (long long)W * P > cap ? 1 : P;
+  }
+  if (S.has_j3) P = 32;
+  while (P > 1 && (long long)W * P > 148ll * 512) P >>= 1;
+  return P;
+}
+
+// With one lane per walker, whether the moves run in k_moves instead of
+// k_sweeps.  Without compiled-in orbitals, or with three-body terms, the local
+// energy costs the fused kernel's moves registers and, at this size, nothing
+// is left to share between lanes: 65,536 walkers, us per sweep, k_sweeps |
+// k_moves and k_eloc: H2O table-driven 459 | 337 (mixed), 622 | 467 (FP64),
+// H2O with three-body terms 2,200 | 1,761 and 3,132 | 1,869.  For few orbitals
+// the launches cost more than that: LiH table-driven 85 | 112, with three-body
+// terms mixed 155 | 169, but 246 | 237 in FP64, and mixed 16,384 walkers 123 |
+// 104.
+static bool moves_by_thread(const oqmc_ctx* ctx, int W, int mixed, int lanes) {
+  if (lanes != 1 || ctx->nocc < 2) return false;
+  if (ctx->nocc < 4) return ctx->spec && ctx->hsys.has_j3 && (!mixed || W <= 148 * 256);
+  return !ctx->spec || ctx->hsys.has_j3;
+}
+
+// How the single-electron sweeps of W walkers run: lanes per walker, and
+// whether the local energies are formed in the sweep kernel too (fused) or by
+// k_eloc after each measured sweep.
+struct SweepPlan {
+  int lanes;
+  bool fused;
+};
+
+// Lanes, and where the local energies are formed.  Several lanes: in the sweep
+// kernel.  One lane: there too, except where k_moves makes the moves and in
+// FP64, where a thread's local energy lives in local memory from eight
+// orbitals on ((H2O)2, 65,536 walkers: 4,459 us per sweep fused, 2,699 with
+// k_eloc; N2, seven orbitals: 658 and 700) and where a CTA size asked for by
+// the caller leaves one thread per walker too few warps to hide it (H2O, 1,000
+// walkers: 100 and 87 us; 65,536 in CTAs of 32: 332 and 314, of 128: 224 and
+// 245).  wpb: walkers per CTA asked for (one lane then), or 0.
+static SweepPlan sweep_plan(const oqmc_ctx* ctx, int W, int mixed, int wpb) {
+  SweepPlan p;
+  p.lanes = wpb ? 1 : sweep_lanes(ctx, W, mixed);
+  const bool few = wpb && ctx->nocc >= 5 && (wpb < 128 || W < 148 * 128);
+  p.fused = p.lanes > 1 ||
+            (!moves_by_thread(ctx, W, mixed, 1) &&
+             (mixed || !ctx->spec || (ctx->nocc < 8 && !few)));
+  return p;
+}
+
 // Largest per-thread local memory (bytes) among the kernels that
-// oqmc_refresh followed by oqmc_sweeps launch for this context and precision
-// (the same dispatch as those two entry points).  Returns OQ_OK or an error.
-int oq_ctx_sweep_local_bytes(oqmc_ctx* ctx, int precision, size_t* out) {
+// oqmc_refresh followed by oqmc_sweeps launch for W walkers of this context
+// and precision (the same dispatch as those two entry points).  Returns OQ_OK
+// or an error.
+int oq_ctx_sweep_local_bytes(oqmc_ctx* ctx, int W, int precision, size_t* out) {
   const int mixed = precision == OQ_PREC_MIXED;
   size_t best = 0, v = 0;
   cudaError_t err = cudaSuccess;
@@ -154,14 +224,19 @@ int oq_ctx_sweep_local_bytes(oqmc_ctx* ctx, int precision, size_t* out) {
   } else {
     ok = take(0, 0);
     const bool alle = ctx->move_kind == 1, tc = mixed && ctx->use_tc;
+    const SweepPlan plan = sweep_plan(ctx, W, mixed, 0);
     if (ok) {
+      const int scaled = ctx->proposal == 1;
       if (alle) ok = take(7, 0);
       else if (ctx->mlp) ok = take_rtc(ctx->mlp_fn[ctx->mlp_groups == 4 ? 1 : 0]);
-      else if (ctx->spec) ok = take_rtc(oq_spec_function(ctx->spec, mixed));
-      else ok = take(1, 0);
+      else if (!moves_by_thread(ctx, W, mixed, plan.lanes))
+        ok = ctx->spec ? take_rtc(oq_spec_function(ctx->spec, mixed)) : take(1, 0);
+      else
+        ok = ctx->spec ? take_rtc(oq_spec_function(ctx->spec, 4 + 2 * scaled + mixed))
+                       : take(8 + scaled, 0);
     }
     // the fused sweeps hold the local energy themselves
-    if (ok && (alle || ctx->mlp || tc)) {
+    if (ok && (alle || ctx->mlp || tc || !plan.fused)) {
       if (tc) ok = take(3, 0);
       else if (ctx->spec) ok = take_rtc(oq_spec_function(ctx->spec, 2 + mixed));
       else ok = take(2, 0);
@@ -1482,6 +1557,8 @@ static int pick_wpb(oqmc_ctx* ctx, int wpb, int precision, size_t* sm) {
   return wpb;
 }
 
+// Launch the moves `m` describes with one thread per walker (the learned
+// proposal: its tiles): sweeps (mode 0) or basin relocations (mode 1).
 static int launch_moves(oqmc_ctx* ctx, const OqMoveArgs& m, int wpb, size_t sm, int precision,
                         void* stream) {
   const int mixed = precision == OQ_PREC_MIXED;
@@ -1497,33 +1574,27 @@ static int launch_moves(oqmc_ctx* ctx, const OqMoveArgs& m, int wpb, size_t sm, 
       return set_err(ctx, OQ_ERR_CUDA, "learned-proposal move kernel launch failed%s");
     return OQ_OK;
   }
+  if (ctx->spec && m.mode == 0) {
+    OqMoveArgs mm = m;
+    const void* C = mixed ? (const void*)ctx->d_C32 : (const void*)ctx->d_C64;
+    void* args[4] = {(void*)&L.sys, (void*)&L.split, (void*)&C, (void*)&mm};
+    if (oq_spec_launch(ctx->spec, (m.proposal == 1 ? 6 : 4) + mixed,
+                       dim3((m.W + wpb - 1) / wpb), dim3(wpb), sm, L.stream, args) != 0)
+      return set_err(ctx, OQ_ERR_CUDA, "specialised move kernel launch failed%s");
+    return OQ_OK;
+  }
   cudaError_t err = cudaSuccess;
-#define OQ_X(N) err = oq_basin_##N(L, m, wpb, mixed)
+#define OQ_X(N) err = oq_moves_##N(L, m, wpb, mixed)
   OQ_SWITCH(ctx->nocc, OQ_X)
 #undef OQ_X
   OQ_CUDA(ctx, err);
   return OQ_OK;
 }
 
-// Lanes per walker of the fused sweeps: as many as there are electrons (all
-// orbital rows of a sweep at once; 32 with three-body terms in FP64, which
-// fill them), halved while the threads would exceed 512 per SM.  Beyond that the register file (128 per thread) is full and
-// lanes only add shuffles.
-static int sweep_lanes(const oqmc_ctx* ctx, int W, int mixed) {
-  int P = 1;
-  while (P < ctx->n_e && P < 32) P <<= 1;
-  if (!mixed && ctx->hsys.has_j3) P = 32;
-  while (P > 1 && (long long)W * P > 148ll * 512) P >>= 1;
-  return P;
-}
-
-// Launch the fused sweeps `a` describes.  wpb: walkers per CTA asked for by the
-// caller (one lane per walker then), 0 for the library's choice; wpb1 is the
+// Launch the sweeps `a` describes with a.lanes lanes per walker; wpb1 is the
 // CTA size that fits with one lane.
-static int launch_sweeps(oqmc_ctx* ctx, OqSweepArgs a, int wpb, int wpb1, int precision,
-                         void* stream) {
+static int launch_sweeps(oqmc_ctx* ctx, OqSweepArgs a, int wpb1, int precision, void* stream) {
   const int mixed = precision == OQ_PREC_MIXED;
-  a.lanes = wpb ? 1 : sweep_lanes(ctx, a.W, mixed);
   int nthr = a.lanes == 1 ? wpb1 : 128;
   a.j3_cache = !mixed && a.lanes > 1 && ctx->hsys.has_j3;
   a.j3_len = a.j3_cache && ctx->j3_len <= 2048 ? ctx->j3_len : 0;
@@ -1657,10 +1728,12 @@ int oqmc_sweeps(oqmc_ctx* ctx, double* X, int W, void* state, int precision, int
   const bool tc = mixed && ctx->use_tc;
   OqSweepArgs sa = sweep_args(ctx, X, W, st);
   sa.step = step; sa.seed = seed; sa.step_base = step_base;
-  if (ctx->move_kind == 0 && !ctx->mlp && !tc) {
+  const SweepPlan plan = sweep_plan(ctx, W, mixed, wpb_asked);
+  sa.lanes = plan.lanes;
+  if (ctx->move_kind == 0 && !ctx->mlp && !tc && plan.fused) {
     sa.n_sweeps = n_sweeps; sa.measure_every = n_sweeps >= measure_every ? measure_every : 0;
     sa.sums = sums; sa.el_trace = el_trace; sa.eparts_last = eparts_last;
-    return launch_sweeps(ctx, sa, wpb_asked, wpb, precision, stream);
+    return launch_sweeps(ctx, sa, wpb, precision, stream);
   }
   OqAlleArgs aa;
   memset(&aa, 0, sizeof(aa));
@@ -1681,8 +1754,11 @@ int oqmc_sweeps(oqmc_ctx* ctx, double* X, int W, void* state, int precision, int
     return alle();
   }
   // mixed all-electron steps, the learned proposal, the tensor-core local
-  // energy: moves and local energies in separate launches
-  if (ctx->mlp) OQ_CUDA(ctx, to_soa(ctx, X, st.pos, W, s));
+  // energy, sweeps that sweep_plan does not fuse: moves and local energies in
+  // separate launches
+  const bool threads =
+      ctx->move_kind == 0 && (ctx->mlp || moves_by_thread(ctx, W, mixed, plan.lanes));
+  if (threads) OQ_CUDA(ctx, to_soa(ctx, X, st.pos, W, s));
   OqMoveArgs m;
   memset(&m, 0, sizeof(m));
   m.pos = st.pos; m.ainv = st.ainv; m.logdet = st.logdet; m.W = W; m.mode = 0;
@@ -1693,8 +1769,8 @@ int oqmc_sweeps(oqmc_ctx* ctx, double* X, int W, void* state, int precision, int
     m.step_base = sa.step_base = aa.step_base = step_base + at;
     m.acc_sum = sa.acc_sum = aa.acc_sum = acc;
     if (ctx->move_kind == 1) return alle();
-    return ctx->mlp ? launch_moves(ctx, m, wpb, sm, precision, stream)
-                    : launch_sweeps(ctx, sa, wpb_asked, wpb, precision, stream);
+    return threads ? launch_moves(ctx, m, wpb, sm, precision, stream)
+                   : launch_sweeps(ctx, sa, wpb, precision, stream);
   };
   OqElocArgs el;
   memset(&el, 0, sizeof(el));
@@ -1736,8 +1812,23 @@ int oqmc_sweeps(oqmc_ctx* ctx, double* X, int W, void* state, int precision, int
     int rc = moves(n_sweeps - done, done, nullptr);
     if (rc != OQ_OK) return rc;
   }
-  if (ctx->mlp) OQ_CUDA(ctx, to_aos(ctx, st.pos, X, W, s));
+  if (threads) OQ_CUDA(ctx, to_aos(ctx, st.pos, X, W, s));
   return OQ_OK;
+}
+
+// One step of the reference's step-size rule (_adapt_step_size,
+// OmegaQMC/vmc_gto.py:121-126) after a sweep of k_moves: with the acceptance
+// ratio acc = (*accepted) * inv_moves of the sweep just made,
+// log s <- log s + rate (acc - target).  Records the ratio in place of the
+// count and the new width in step_trace (if set).  One thread.
+__global__ void k_adapt_step(double* __restrict__ step, double* __restrict__ accepted,
+                             double inv_moves, double rate, double target,
+                             double* __restrict__ step_trace) {
+  const double acc = *accepted * inv_moves;
+  const double s = exp(log(*step) + rate * (acc - target));
+  *step = s;
+  *accepted = acc;
+  if (step_trace) *step_trace = s;
 }
 
 int oqmc_equilibrate(oqmc_ctx* ctx, double* X, int W, void* state, int precision,
@@ -1767,16 +1858,29 @@ int oqmc_equilibrate(oqmc_ctx* ctx, double* X, int W, void* state, int precision
   while (a.tick <= (double)W * ctx->n_e) a.tick *= 2.0;
   const OqLaunch Lr = make_launch(ctx, stream, 0);
   const int mixed = precision == OQ_PREC_MIXED;
+  a.lanes = sweep_plan(ctx, W, mixed, 0).lanes;
+  const bool threads = moves_by_thread(ctx, W, mixed, a.lanes);
+  OqMoveArgs m;
+  memset(&m, 0, sizeof(m));
+  m.pos = st.pos; m.ainv = st.ainv; m.logdet = st.logdet; m.W = W; m.n_steps = 1;
+  m.step_dev = step; m.seed = seed; m.flags = ctx->d_flags;
+  m.proposal = ctx->proposal; m.scale_r0 = ctx->scale_r0; m.scale_fmin = ctx->scale_fmin;
+  if (threads) OQ_CUDA(ctx, to_soa(ctx, X, st.pos, W, s));
   int since = since_refresh;
   for (int t = 0; t < n_steps; ++t) {
     const bool refresh = since + 1 >= refresh_every;
-    a.step_base = step_base + t;
-    a.acc_sum = acc_trace + t;
+    a.step_base = m.step_base = step_base + t;
+    a.acc_sum = m.acc_sum = acc_trace + t;
     a.step_trace = step_trace ? step_trace + t : nullptr;
     // the state's own positions are read by the refresh and after the call
     a.pos = refresh || t == n_steps - 1 ? st.pos : nullptr;
-    int rc = launch_sweeps(ctx, a, 0, wpb, precision, stream);
+    const int rc = threads ? launch_moves(ctx, m, wpb, sm, precision, stream)
+                           : launch_sweeps(ctx, a, wpb, precision, stream);
     if (rc != OQ_OK) return rc;
+    if (threads) {
+      k_adapt_step<<<1, 1, 0, s>>>(step, a.acc_sum, a.inv_moves, rate, target, a.step_trace);
+      OQ_CUDA(ctx, cudaGetLastError());
+    }
     ++since;
     if (refresh) {
       cudaError_t err = cudaSuccess;
@@ -1787,6 +1891,7 @@ int oqmc_equilibrate(oqmc_ctx* ctx, double* X, int W, void* state, int precision
       since = 0;
     }
   }
+  if (threads) OQ_CUDA(ctx, to_aos(ctx, st.pos, X, W, s));
   return OQ_OK;
 }
 

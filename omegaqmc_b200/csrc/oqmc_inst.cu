@@ -79,20 +79,31 @@ cudaError_t OQ_FN(oq_refresh)(const OqLaunch& L, const double* pos, int W, void*
   return mixed ? team<OQ_TEAM_REFRESH, float>(L, a) : team<OQ_TEAM_REFRESH, double>(L, a);
 }
 
-// basin relocations
-cudaError_t OQ_FN(oq_basin)(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed) {
+template <int PROP>
+static cudaError_t moves_prop(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed) {
   const int nb = (a.W + wpb - 1) / wpb;
   cudaError_t e;
   if (mixed) {
-    e = oq_smem_attr(k_moves<OQ_N, float, float, 2>, L.smem);
+    e = oq_smem_attr(k_moves<OQ_N, float, float, PROP>, L.smem);
     if (e != cudaSuccess) return e;
-    k_moves<OQ_N, float, float, 2><<<nb, wpb, L.smem, L.stream>>>(L.sys, L.split, L.C32, a);
+    k_moves<OQ_N, float, float, PROP><<<nb, wpb, L.smem, L.stream>>>(L.sys, L.split, L.C32, a);
   } else {
-    e = oq_smem_attr(k_moves<OQ_N, double, double, 2>, L.smem);
+    e = oq_smem_attr(k_moves<OQ_N, double, double, PROP>, L.smem);
     if (e != cudaSuccess) return e;
-    k_moves<OQ_N, double, double, 2><<<nb, wpb, L.smem, L.stream>>>(L.sys, L.split, L.C64, a);
+    k_moves<OQ_N, double, double, PROP><<<nb, wpb, L.smem, L.stream>>>(L.sys, L.split, L.C64, a);
   }
   return cudaGetLastError();
+}
+
+cudaError_t OQ_FN(oq_moves)(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed) {
+  if (a.mode == 1) return moves_prop<2>(L, a, wpb, mixed);
+  // table-driven, fewer than four orbitals always sweep in k_sweeps (moves_by_thread)
+#if OQ_N >= 4
+  if (a.proposal == 1) return moves_prop<1>(L, a, wpb, mixed);
+  return moves_prop<0>(L, a, wpb, mixed);
+#else
+  return cudaErrorInvalidValue;
+#endif
 }
 
 cudaError_t OQ_FN(oq_sweeps)(const OqLaunch& L, const OqSweepArgs& a, int nthr, int mixed) {
@@ -211,7 +222,8 @@ cudaError_t OQ_FN(oq_alle)(const OqLaunch& L, const OqAlleArgs& a, int mixed) {
 
 // Per-thread local memory (bytes) of one kernel this size launches: kind 0
 // k_team (refresh), 1 k_sweeps, 2 k_eloc, 3 k_eloc_tc, 4 k_md_refresh,
-// 5 k_md_moves, 6 k_md_local (M = 8 or 16 columns), 7 k_alle.
+// 5 k_md_moves, 6 k_md_local (M = 8 or 16 columns), 7 k_alle, 8 and 9 k_moves
+// (fixed-width and nucleus-scaled proposal).
 template <typename K>
 static cudaError_t oq_lmem(K kernel, size_t* out) {
   cudaFuncAttributes a;
@@ -247,6 +259,14 @@ cudaError_t OQ_FN(oq_local_bytes)(int kind, int mixed, int M, size_t* out) {
         if (M == 8) return md_lmem<8>(kind, out);
       }
       return M == 16 ? md_lmem<16>(kind, out) : cudaErrorInvalidValue;
+#if OQ_N >= 4
+    case 8:
+      return mixed ? oq_lmem(k_moves<OQ_N, float, float, 0>, out)
+                   : oq_lmem(k_moves<OQ_N, double, double, 0>, out);
+    case 9:
+      return mixed ? oq_lmem(k_moves<OQ_N, float, float, 1>, out)
+                   : oq_lmem(k_moves<OQ_N, double, double, 1>, out);
+#endif
     case 7:
       return mixed ? oq_lmem(k_alle<OQ_N, float, true>, out)
                    : oq_lmem(k_alle<OQ_N, double, true>, out);

@@ -27,7 +27,7 @@ struct OqLaunch {
   cudaError_t oq_movals_##N(const OqLaunch& L, const double* X, int W, double* out);  \
   cudaError_t oq_refresh_##N(const OqLaunch& L, const double* pos, int W, void* ainv, \
                              double* logdet, int mixed);                              \
-  cudaError_t oq_basin_##N(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed); \
+  cudaError_t oq_moves_##N(const OqLaunch& L, const OqMoveArgs& a, int wpb, int mixed); \
   cudaError_t oq_sweeps_##N(const OqLaunch& L, const OqSweepArgs& a, int nthr, int mixed); \
   cudaError_t oq_alle_##N(const OqLaunch& L, const OqAlleArgs& a, int mixed);           \
   cudaError_t oq_eloc_##N(const OqLaunch& L, const OqElocArgs& a, int mixed);           \

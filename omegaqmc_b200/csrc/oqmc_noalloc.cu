@@ -65,7 +65,7 @@ static cudaError_t scratch_address(void** out) {
 }
 
 int oq_ctx_set_error(oqmc_ctx* ctx, int code, const char* msg);
-int oq_ctx_sweep_local_bytes(oqmc_ctx* ctx, int precision, size_t* out);
+int oq_ctx_sweep_local_bytes(oqmc_ctx* ctx, int W, int precision, size_t* out);
 
 extern "C" int oqmc_sweeps_noalloc(oqmc_ctx* ctx, double* walkers, int W, int precision,
                                    int n_sweeps, int measure_every, double step,
@@ -80,7 +80,7 @@ extern "C" int oqmc_sweeps_noalloc(oqmc_ctx* ctx, double* walkers, int W, int pr
   // which is a device allocation (the multi-determinant kernels need more
   // than the default 1 KiB)
   size_t lmem = 0, limit = 0;
-  const int lrc = oq_ctx_sweep_local_bytes(ctx, precision, &lmem);
+  const int lrc = oq_ctx_sweep_local_bytes(ctx, W, precision, &lmem);
   if (lrc != OQ_OK) return lrc;
   const cudaError_t le = cudaDeviceGetLimit(&limit, cudaLimitStackSize);
   if (le != cudaSuccess) return oq_ctx_set_error(ctx, OQ_ERR_CUDA, cudaGetErrorString(le));

@@ -17,6 +17,8 @@
 #include <dlfcn.h>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -484,8 +486,10 @@ std::string oq_spec_term_defines(const std::vector<const OqSystem*>& S) {
 
 namespace {
 
-std::string generate(const OqSystem& S, const OqSplit& SP, const double* C, int nocc) {
-  return oq_spec_term_defines({&S}) + "#include \"oqmc_sweep.cuh\"\n\n" + generate_basis(S, SP, C, nocc, "OqSpecBasis");
+std::string generate(const OqSystem& S, const OqSplit& SP, const double* C, int nocc,
+                     bool term_defines = true) {
+  return (term_defines ? oq_spec_term_defines({&S}) : std::string()) +
+         "#include \"oqmc_sweep.cuh\"\n\n" + generate_basis(S, SP, C, nocc, "OqSpecBasis");
 }
 
 }  // namespace
@@ -622,40 +626,67 @@ int oq_rtc_local_bytes(void* fn) {
 }
 
 struct OqSpecModule {
-  CUmodule mod = nullptr;
-  CUfunction fn[4] = {nullptr, nullptr, nullptr, nullptr};   // fused sweeps d/f, local energy d/f
+  void* mod[2] = {nullptr, nullptr};
+  // fused sweeps d/f, local energy d/f, moves alone d/f of either proposal
+  CUfunction fn[8] = {};
 };
+
+bool oq_spec_has_moves(const OqSystem& S, int nocc) { return S.has_j3 && nocc >= 2; }
 
 int oq_spec_build(const OqSystem& S, const OqSplit& SP, const double* C, int nocc,
                   OqSpecModule** out, std::string* err) {
-  std::vector<std::string> names;
-  const char* forms[4] = {"k_sweeps<%d, double, double, OqSpecBasis>",
-                          "k_sweeps<%d, float, float, OqSpecBasis>",
-                          "k_eloc<%d, double, double, OqSpecBasis>",
-                          "k_eloc<%d, float, float, OqSpecBasis>"};
-  for (const char* f : forms) {
-    char b[128];
-    snprintf(b, sizeof b, f, nocc);
-    names.push_back(b);
+  const std::string N = std::to_string(nocc);
+  std::vector<std::string> names, moves;
+  for (const char* k : {"k_sweeps<", "k_eloc<"})
+    for (const char* t : {"double, double", "float, float"})
+      names.push_back(k + N + ", " + t + ", OqSpecBasis>");
+  for (const char* prop : {"0", "1"})
+    for (const char* t : {"double, double", "float, float"})
+      moves.push_back("k_moves<" + N + ", " + t + ", " + prop + ", OqSpecBasis>");
+  const std::string src = generate(S, SP, C, nocc);
+  // k_moves keeps the absent terms' branches: without them the compiler
+  // schedules the FP64 three-body sums worse (N2, 65,536 walkers: 4,833 us per
+  // sweep with, 5,515 without; H2O, LiH and (H2O)2 within 1.5%)
+  const std::string src2 = generate(S, SP, C, nocc, false);
+  const bool two = oq_spec_has_moves(S, nocc);
+  std::vector<char> cubin, cubin2;
+  std::vector<std::string> low, low2;
+  std::string err2;
+  int rc = 0, rc2 = 0;
+  auto second = [&] { rc2 = oq_rtc_compile(src2, moves, &cubin2, &low2, &err2); };
+  std::thread th;
+  if (two) {
+    try {                       // beside the first module, on another host thread
+      th = std::thread(second);
+    } catch (const std::system_error&) {
+      second();                 // no thread to be had
+    }
   }
-  void* mod = nullptr;
-  std::vector<void*> fns;
-  if (oq_rtc_build(generate(S, SP, C, nocc), names, &mod, &fns, err) != 0) return -1;
+  rc = oq_rtc_compile(src, names, &cubin, &low, err);
+  if (th.joinable()) th.join();
+  if (rc == 0 && rc2 != 0) *err = err2;
+  if (rc != 0 || rc2 != 0) return -1;
   OqSpecModule* m = new OqSpecModule();
-  m->mod = (CUmodule)mod;
+  std::vector<void*> fns, fns2;
+  if (oq_rtc_load(cubin, low, &m->mod[0], &fns, err) != 0 ||
+      (two && oq_rtc_load(cubin2, low2, &m->mod[1], &fns2, err) != 0)) {
+    oq_spec_destroy(m);
+    return -1;
+  }
   for (int i = 0; i < 4; ++i) m->fn[i] = (CUfunction)fns[i];
+  for (int i = 0; two && i < 4; ++i) m->fn[4 + i] = (CUfunction)fns2[i];
   *out = m;
   return 0;
 }
 
 void oq_spec_destroy(OqSpecModule* m) {
   if (!m) return;
-  if (g_api.ok && m->mod) g_api.ModuleUnload(m->mod);
+  for (void* mod : m->mod) oq_rtc_unload(mod);
   delete m;
 }
 
 void* oq_spec_function(OqSpecModule* m, int which) {
-  return (m && which >= 0 && which < 4) ? (void*)m->fn[which] : nullptr;
+  return (m && which >= 0 && which < 8) ? (void*)m->fn[which] : nullptr;
 }
 
 int oq_spec_launch(OqSpecModule* m, int which, dim3 grid, dim3 block, size_t smem,

@@ -12,11 +12,16 @@ struct OqSpecModule;
 int oq_spec_build(const OqSystem& S, const OqSplit& SP, const double* C, int nocc,
                   OqSpecModule** out, std::string* err);
 void oq_spec_destroy(OqSpecModule* m);
-// which: 0/1 = fused sweeps FP64/mixed, 2/3 = local energy FP64/mixed
+// which: 0/1 = fused sweeps FP64/mixed, 2/3 = local energy FP64/mixed, and
+// where oq_spec_has_moves, 4/5 and 6/7 = moves alone (k_moves) FP64/mixed with
+// the fixed-width and the nucleus-scaled proposal
 int oq_spec_launch(OqSpecModule* m, int which, dim3 grid, dim3 block, size_t smem,
                    cudaStream_t stream, void** args);
 // The CUfunction behind `which` (numbering as for oq_spec_launch).
 void* oq_spec_function(OqSpecModule* m, int which);
+// Whether the module holds the moves alone as well (see moves_by_thread in
+// oqmc.cu).
+bool oq_spec_has_moves(const OqSystem& S, int nocc);
 std::string oq_spec_source(const OqSystem& S, const OqSplit& SP, const double* C, int nocc);
 
 // Which optional Jastrow terms any of the systems has, as #define lines for the

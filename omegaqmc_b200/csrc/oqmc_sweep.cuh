@@ -605,10 +605,11 @@ __device__ __forceinline__ int oq_basin_propose(const OqSystem& S, const double*
 }
 
 // Metropolis moves alone, one thread per walker, state resident in shared
-// memory for the whole launch; the library launches it for basin relocations
-// (sweeps run in k_sweeps).  PROP (compile time) selects the proposal: 0 fixed-
-// width Gaussian, 1 nucleus-scaled Gaussian, 2 basin relocation.  mode 0: n_steps sweeps over all electrons with
-// Gaussian proposals (metropolis_move_1w, OmegaQMC/vmc_gto.py:841-905, as
+// memory for the whole launch: basin relocations, and the sweeps that
+// moves_by_thread (oqmc.cu) keeps out of k_sweeps.  PROP (compile time) selects
+// the proposal: 0 fixed-width Gaussian, 1 nucleus-scaled Gaussian, 2 basin
+// relocation.  mode 0: n_steps sweeps over all electrons with Gaussian
+// proposals (metropolis_move_1w, OmegaQMC/vmc_gto.py:841-905, as
 // single-electron moves).  mode 1: n_steps basin relocations: one random
 // electron proposed at N(R_J, sigma^2) around a random nucleus J, accepted
 // with the exact proposal ratio q(old)/q(new), q(x) = sum_J
