@@ -1066,9 +1066,16 @@ k_alle(const OqSystem* __restrict__ gS, const unsigned char* __restrict__ ao, in
     const int j = q % wb, k = q / wb, sp = k / (N * N), m = (k / N) % N, c = k % N;
     if (w0 + j < W) gA[(size_t)k * W + w0 + j] = (Real)Acur[((sp * N + c) * N + m) * wb + j];
   }
-  if (live && e == 0) {
-    a.logdet[w] = ld_cur;
-    if (a.acc_sum && nacc) atomicAdd(a.acc_sum, (double)(nacc * NE));
+  if (e == 0) {
+    if (live) a.logdet[w] = ld_cur;
+    if (a.acc_sum) {
+      // one addition per warp: one per walker, all to one address, took most of
+      // a mixed step of many small walkers (H2, 65,536: 137 us)
+      const int span = wb < 32 ? wb : 32;
+      const unsigned mask = span == 32 ? 0xffffffffu : (1u << span) - 1u;
+      for (int o = span >> 1; o > 0; o >>= 1) nacc += __shfl_xor_sync(mask, nacc, o);
+      if ((wl & 31) == 0 && nacc) atomicAdd(a.acc_sum, (double)(nacc * NE));
+    }
   }
 }
 

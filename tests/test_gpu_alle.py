@@ -130,3 +130,32 @@ def test_noalloc_entry_runs_all_electron_steps_once_the_stack_allows():
     torch.cuda.synchronize()
     assert torch.equal(Xa, Xb) and torch.allclose(sa, sb, rtol=1e-12, atol=1e-12)
     assert not torch.equal(Xa, X0)
+
+
+@pytest.mark.parametrize("name,W", [("H2", 65537), ("H2", 5), ("H2O", 3001), ("H2O_dimer", 333)])
+def test_mixed_steps_count_every_accepted_walker(name, W):
+    """The accepted moves of a mixed step, added per warp, are the walkers
+    that moved; and adding them does not dominate the step (an addition per
+    walker made a mixed step of 65,537 H2 walkers take four FP64 ones)."""
+    s = _sys(name)
+    times = {}
+    for prec in ("fp64", "mixed"):
+        ctx = GTOContext(s)
+        ctx.set_move_kind(1)
+        ens = WalkerEnsemble(ctx, seeded_walkers(s, W, 0.8, 4), prec, seed=21, refresh_every=10**9)
+        X0 = ens.X.clone()
+        sums = ens.run(1, 0.2)
+        moved = int(torch.any((ens.X != X0).view(W, -1), dim=1).sum())
+        assert 0 < moved and float(sums[0, 5]) == moved * s.n_e
+        best = np.inf
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            ens.run(8, 0.2)
+            b.record()
+            torch.cuda.synchronize()
+            best = min(best, a.elapsed_time(b))
+        times[prec] = best
+        assert ctx.flags() == 0
+    if W > 10**4:
+        assert times["mixed"] < 2.5 * times["fp64"], times
