@@ -183,3 +183,22 @@ def test_all_electron_steps_do_not_depend_on_the_tile(name, prec, sizes):
     for a, b in zip(runs, runs[1:]):
         assert torch.equal(a, b[: a.shape[0]])
     assert not torch.equal(runs[-1], torch.as_tensor(X, device="cuda"))
+
+
+@pytest.mark.parametrize("W", [1, 33, 4097])
+def test_f_and_g_shell_values_match_oracle(W):
+    """The value path of f and g shells (mo_values, log_psi, the refresh)
+    forms no harmonic gradients; its values are evaluate's."""
+    from helpers import golden_system
+    s, _ = golden_system("fg_shells")
+    ctx = GTOContext(s)
+    X = seeded_walkers(s, W, 0.9, 17)
+    m = min(W, 200)
+    mo = ctx.mo_values(X)[:m].cpu().numpy()
+    ref = O.mo_value(s, X[:m])
+    assert np.max(np.abs(mo - ref) / (np.abs(ref) + 1.0)) < TOL
+    lp, ev = ctx.log_psi(X).cpu().numpy(), ctx.evaluate(X)["logpsi"].cpu().numpy()
+    assert np.max(np.abs(lp - ev) / (np.abs(ev) + 1.0)) < 1e-12
+    ens = WalkerEnsemble(ctx, X, "fp64", seed=1)
+    ld = ens.logdet()[:m].cpu().numpy()
+    assert np.max(np.abs(ld - O.log_slater(s, X[:m])) / (np.abs(ld) + 1.0)) < TOL
