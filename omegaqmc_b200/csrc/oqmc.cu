@@ -783,9 +783,9 @@ __device__ __forceinline__ void oq_pade_dp(double a, double b, double r, double 
 // One warp per walker.  Every parameter belongs to one lane (or is summed over
 // the lanes by shuffles), so nothing is added to global memory: with one
 // thread per walker each three-body term read and wrote the derivatives of
-// all its gammas there (walker_derivatives of H2O with three-body orders 2 and
-// 2, 2,048 walkers: 4,492 us in all, 1,320 now with the fixed-order three-body
-// polynomials of the evaluation, most of it host time).
+// all its gammas there (H2O with three-body orders 2 and 2, 2,048 walkers:
+// 2,256 us, 58 with a warp each).  Many walkers of a few pairs each leave most
+// lanes idle and go to k_param_derivs_thread instead, see launch_param_derivs.
 #define OQ_PD_WARPS 4
 // doubles of one listed three-body term: see oq_pd_j3
 #define OQ_PD_GEO 16
@@ -1174,10 +1174,122 @@ k_param_derivs(const OqSystem* __restrict__ gsys, const double* __restrict__ X,
   }
 }
 
+// All B-spline parameters that a term at distance r touches, see
+// oq_pd_bspline: those of coefficients i..i+3 of its knot interval i, and P_1
+// through coefficient 0.
+__device__ __forceinline__ void oq_bs_param_add(int n, double dinv, double rcut, double r,
+                                                double gd, bool half, double* dl, double* de) {
+  if (!(r < rcut)) return;
+  double t;
+  const int i = oq_bs_index<double>(r * dinv, n, t);
+  for (int k = 0; k < 4; ++k) {
+    const int idx = i + k, q = idx == 0 ? 1 : idx - 1;
+    double w, w1, w2;
+    if (q < 0 || q >= n || !oq_bs_weight(r, dinv, n, idx, w, w1, w2)) continue;
+    const double dL = w2 + 2.0 * w1 / r;
+    dl[q] += w;
+    de[q] -= half ? 0.5 * (dL + 2.0 * w1 * gd) : dL + w1 * gd;
+  }
+}
+
+// The raw derivatives without three-body terms, one thread per walker.
+__global__ void __launch_bounds__(128)
+k_param_derivs_thread(const OqSystem* __restrict__ gsys, const double* __restrict__ X,
+                      const double* __restrict__ G, int W, int n_e, int n_raw,
+                      double* __restrict__ dlog, double* __restrict__ del) {
+  const int w = blockIdx.x * blockDim.x + threadIdx.x;
+  if (w >= W) return;
+  const OqSystem& S = *gsys;
+  const int natm = S.natm, bs2 = 4 + 2 * natm;
+  const int bs1 = bs2 + (S.has_bs2 ? S.bs2_n_like + S.bs2_n_unlike : 0);
+  const double* x = X + (size_t)w * n_e * 3;
+  const double* g = G + (size_t)w * n_e * 3;
+  double* dl = dlog + (size_t)w * n_raw;
+  double* de = del + (size_t)w * n_raw;
+  for (int k = 0; k < n_raw; ++k) dl[k] = de[k] = 0.0;
+  if (S.has_j2 || S.has_bs2) {
+    double al[4] = {0, 0, 0, 0}, ae[4] = {0, 0, 0, 0};
+    for (int i = 0; i < n_e; ++i)
+      for (int j = i + 1; j < n_e; ++j) {
+        const double dx = x[3 * i] - x[3 * j], dy = x[3 * i + 1] - x[3 * j + 1],
+                     dz = x[3 * i + 2] - x[3 * j + 2];
+        const double r = sqrt(dx * dx + dy * dy + dz * dz);
+        const double gd = ((g[3 * i] - g[3 * j]) * dx + (g[3 * i + 1] - g[3 * j + 1]) * dy +
+                           (g[3 * i + 2] - g[3 * j + 2]) * dz) / r;
+        const int blk = (i ^ j) & 1;
+        if (S.has_j2) {
+          double du[2], dup[2], dL[2];
+          oq_pade_dp(S.j2[2 * blk], S.j2[2 * blk + 1], r, du, dup, dL);
+          for (int q = 0; q < 2; ++q) {
+            const double e = dL[q] + dup[q] * gd;
+            al[q] += blk ? 0.0 : du[q];
+            al[2 + q] += blk ? du[q] : 0.0;
+            ae[q] -= blk ? 0.0 : e;
+            ae[2 + q] -= blk ? e : 0.0;
+          }
+        }
+        if (S.has_bs2) {
+          const int o = bs2 + (blk ? S.bs2_n_like : 0);
+          oq_bs_param_add(blk ? S.bs2_n_unlike : S.bs2_n_like,
+                          blk ? S.bs2_dinv_unlike : S.bs2_dinv_like, S.bs2_rcut, r, gd, false,
+                          dl + o, de + o);
+        }
+      }
+    for (int k = 0; k < 4; ++k) {
+      dl[k] = al[k];
+      de[k] = ae[k];
+    }
+  }
+  for (int I = 0; I < natm; ++I) {
+    const int ty = S.has_bs1 ? S.bs1_type[I] : -1;
+    if (!S.has_j1 && ty < 0) continue;
+    int o = bs1;
+    for (int t = 0; t < ty; ++t) o += S.bs1_n[t];
+    double sl[2] = {0.0, 0.0}, se[2] = {0.0, 0.0};
+    for (int e = 0; e < n_e; ++e) {
+      const double dx = x[3 * e] - S.nuc[I][0], dy = x[3 * e + 1] - S.nuc[I][1],
+                   dz = x[3 * e + 2] - S.nuc[I][2];
+      const double r = sqrt(dx * dx + dy * dy + dz * dz);
+      const double gd = (g[3 * e] * dx + g[3 * e + 1] * dy + g[3 * e + 2] * dz) / r;
+      if (S.has_j1) {
+        double du[2], dup[2], dL[2];
+        oq_pade_dp(S.j1a[I], S.j1b[I], r, du, dup, dL);
+        for (int q = 0; q < 2; ++q) {
+          sl[q] += du[q];
+          se[q] -= 0.5 * (dL[q] + 2.0 * dup[q] * gd);
+        }
+      }
+      if (ty >= 0)
+        oq_bs_param_add(S.bs1_n[ty], S.bs1_dinv[ty], S.bs1_rcut[ty], r, gd, true, dl + o, de + o);
+    }
+    for (int q = 0; q < 2; ++q) {
+      dl[4 + 2 * I + q] = sl[q];
+      de[4 + 2 * I + q] = se[q];
+    }
+  }
+}
+
 int oqmc_param_count(const oqmc_ctx* ctx) { return ctx ? param_count_of(ctx->hsys) : OQ_ERR_ARG; }
 
+// A thread per walker pays from so many walkers per pair term on, and some
+// thousands in all (raw derivatives, us, warp | thread: H2, 5 terms, 8,192
+// walkers 27 | 17, 65,536: 116 | 26; LiH, 14 terms, 6,000: 25 | 26, 16,384: 40 |
+// 26; H2O, 75 terms, 20,000: 60 | 71, 65,536: 160 | 89; N2, 119 terms, 131,072:
+// 329 | 263; with B-splines, whose weights a warp forms again for each
+// parameter, H2O 8,192: 177 | 210, 13,000: 258 | 134, H2 1,000: 18 | 25, 65,536:
+// 207 | 50).  Beyond sixteen electrons it does not: its positions no longer
+// stay in the cache ((H2O)2, 131,072 walkers: 648 | 728).
 static int launch_param_derivs(oqmc_ctx* ctx, const double* X, int W, const double* grad,
                                const OqPdOut& out, void* stream) {
+  const OqSystem& S = ctx->hsys;
+  const int terms = S.n_e * (S.n_e - 1) / 2 + S.n_e * S.natm;
+  if (!out.map && !S.has_j3 && S.n_e <= 16 && W > 4000 &&
+      W > (S.has_bs1 || S.has_bs2 ? 140 : 400) * terms) {
+    k_param_derivs_thread<<<(W + 127) / 128, 128, 0, (cudaStream_t)stream>>>(
+        ctx->d_sys, X, grad, W, ctx->n_e, param_count_of(S), out.dlog, out.del);
+    OQ_CUDA(ctx, cudaGetLastError());
+    return OQ_OK;
+  }
   const size_t wbytes = param_derivs_smem(ctx->hsys), sm = OQ_PD_WARPS * wbytes;
   if (sm > 48 * 1024)
     OQ_CUDA(ctx, cudaFuncSetAttribute(k_param_derivs, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -202,3 +202,44 @@ def test_f_and_g_shell_values_match_oracle(W):
     ens = WalkerEnsemble(ctx, X, "fp64", seed=1)
     ld = ens.logdet()[:m].cpu().numpy()
     assert np.max(np.abs(ld - O.log_slater(s, X[:m])) / (np.abs(ld) + 1.0)) < TOL
+
+
+@pytest.mark.parametrize("name,bs,W", [("H2", False, 4001), ("H2", False, 4000), ("LiH", False, 5601),
+                                       ("H2O", True, 10501), ("H2", True, 4097)])
+def test_raw_derivatives_of_many_walkers(name, bs, W):
+    """One thread per walker above 4,000 walkers and 400 per pair term (140
+    with B-splines; H2 has 5 terms, LiH 14, H2O 75): against the oracle on both
+    sides of the line, and the last walkers of a partial CTA."""
+    import torch
+    from omegaqmc_b200.context import _dptr, _stream_ptr
+    mol = M.named_system(name)
+    pc, cfg = M.default_params_corr(mol), None
+    els = sorted(set(mol.elements))
+    if bs:
+        pc["J2_bspline"] = {"like": np.array([0.2, 0.1, 0.05]), "unlike": np.linspace(0.4, 0.0, 9)}
+        pc["J1_bspline"] = {e: np.array([-0.1, 0.05, 0.02, 0.01]) for e in els}
+        cfg = {"J2": {"r_cut": 3.5}, "J1": {e: {"r_cut": 3.0} for e in els}}
+    import warnings
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        s = build_system(M.make_mf(name), pc, None, cfg)
+    ctx = GTOContext(s)
+    X = ctx.walkers_tensor(seeded_walkers(s, W, 0.9, 7))
+    grad = ctx.evaluate(X)["grad"]
+    n = ctx.lib.oqmc_param_count(ctx._h)
+    dl = torch.full((W + 1, n), np.nan, dtype=torch.float64, device="cuda")
+    de = dl.clone()
+    ctx._check(ctx.lib.oqmc_param_derivs(ctx._h, _dptr(X), W, _dptr(grad), _dptr(dl), _dptr(de),
+                                         _stream_ptr(None)))
+    assert bool(torch.isnan(dl[W]).all()) and bool(torch.isnan(de[W]).all())
+    pick = np.r_[0:40, W - 40:W]
+    rl, re_ = O.param_derivatives(s, X.cpu().numpy()[pick])
+    assert np.max(np.abs(dl.cpu().numpy()[pick] - rl) / (np.abs(rl).max(axis=0) + 1.0)) < 1e-10
+    assert np.max(np.abs(de.cpu().numpy()[pick] - re_) / (np.abs(re_).max(axis=0) + 1.0)) < 1e-9
+    # the mapped form keeps a warp per walker: the same numbers, other sums
+    from omegaqmc_b200.optim import raw_to_flat, walker_derivatives
+    e, fl, fe = walker_derivatives(ctx, X, pc)
+    ml = raw_to_flat(dl[:W].cpu().numpy(), pc, s)
+    me = raw_to_flat(de[:W].cpu().numpy(), pc, s)
+    assert np.max(np.abs(fl - ml) / (np.abs(ml).max(axis=0) + 1.0)) < 1e-12
+    assert np.max(np.abs(fe - me) / (np.abs(me).max(axis=0) + 1.0)) < 1e-12
