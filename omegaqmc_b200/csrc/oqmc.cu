@@ -1293,7 +1293,7 @@ static int launch_param_derivs(oqmc_ctx* ctx, const double* X, int W, const doub
   const size_t wbytes = param_derivs_smem(ctx->hsys), sm = OQ_PD_WARPS * wbytes;
   if (sm > 48 * 1024)
     OQ_CUDA(ctx, cudaFuncSetAttribute(k_param_derivs, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)sm));
+                                      OQ_SMEM_OPTIN));
   k_param_derivs<<<(W + OQ_PD_WARPS - 1) / OQ_PD_WARPS, 32 * OQ_PD_WARPS, sm,
                    (cudaStream_t)stream>>>(ctx->d_sys, X, grad, W, ctx->n_e,
                                            param_count_of(ctx->hsys), (int)wbytes, out);

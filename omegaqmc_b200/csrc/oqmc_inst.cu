@@ -18,7 +18,8 @@ static cudaError_t oq_smem_attr(K kernel, size_t smem) {
                                        (int)cudaSharedmemCarveoutMaxShared);
   if (e != cudaSuccess) return e;
   if (smem > 48 * 1024)
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                OQ_SMEM_OPTIN);
   return cudaSuccess;
 }
 

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include "oqmc_eloc_tc.cuh"
 #include "oqmc_multidet.cuh"
+#include "oqmc_smem.h"
 #include "oqmc_team.cuh"
 
 struct OqLaunch {

@@ -25,6 +25,7 @@
 #include <nvrtc.h>
 
 #include "oqmc_rtc.h"
+#include "oqmc_smem.h"
 #include "oqmc_rtc_src.inc"   // generated: the kernel headers as strings
 
 namespace {
@@ -592,7 +593,7 @@ int oq_rtc_launch(void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t str
   const Api& A = g_api;
   CUfunction f = (CUfunction)fn;
   if (smem > 48 * 1024 &&
-      A.FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem) !=
+      A.FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, OQ_SMEM_OPTIN) !=
           CUDA_SUCCESS)
     return -1;
   return A.LaunchKernel(f, grid.x, grid.y, grid.z, block.x, block.y, block.z, (unsigned)smem,
@@ -604,9 +605,10 @@ int oq_rtc_launch(void* fn, dim3 grid, dim3 block, size_t smem, cudaStream_t str
 int oq_rtc_occupancy(void* fn, int block, size_t smem, int* nblk) {
   const Api& A = g_api;
   CUfunction f = (CUfunction)fn;
-  if (smem > 48 * 1024 &&
-      A.FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem) !=
-          CUDA_SUCCESS) {
+  if (smem > OQ_SMEM_OPTIN ||
+      (smem > 48 * 1024 &&
+       A.FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, OQ_SMEM_OPTIN) !=
+           CUDA_SUCCESS)) {
     *nblk = 0;
     return 0;
   }
@@ -694,7 +696,7 @@ int oq_spec_launch(OqSpecModule* m, int which, dim3 grid, dim3 block, size_t sme
   const Api& A = g_api;
   CUfunction f = m->fn[which];
   if (smem > 48 * 1024 &&
-      A.FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem) !=
+      A.FuncSetAttribute(f, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, OQ_SMEM_OPTIN) !=
           CUDA_SUCCESS)
     return -1;
   return A.LaunchKernel(f, grid.x, grid.y, grid.z, block.x, block.y, block.z, (unsigned)smem,
