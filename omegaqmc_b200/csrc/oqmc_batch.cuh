@@ -331,8 +331,10 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
   const int w = w0 + wl;
   double logdet = 0.0;
   {
-    // FP64 refresh of the spin blocks, with the generated orbitals: both on the
-    // walker's thread when P = 1, spin s on lane s otherwise
+    // FP64 refresh of the spin blocks: both on the walker's thread when P = 1,
+    // spin s on lane s otherwise.  With the generated orbitals, but all their
+    // terms: the moves and local energies leave out coefficients below 1e-12 of
+    // an orbital's largest, the step that stops drift does not.
     bool ok = true;
     if (live && lane < 2) {
       for (int s = (P == 1 ? 0 : lane); s < (P == 1 ? 2 : lane + 1); ++s) {
@@ -340,8 +342,8 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
         for (int i = 0; i < NOCC; ++i) {
           const int e = 2 * i + s;
           double mv[NOCC];
-          B::template mo_val<double, double>(S, SP, d.C64, pos[3 * e], pos[3 * e + 1],
-                                             pos[3 * e + 2], mv);
+          B::template mo_val_full<double, double>(S, SP, d.C64, pos[3 * e], pos[3 * e + 1],
+                                                  pos[3 * e + 2], mv);
 #pragma unroll
           for (int m = 0; m < NOCC; ++m) Sm[i][m] = mv[m];
         }

@@ -107,6 +107,7 @@ struct Gen {
   int nocc;
   std::string o;
   bool contract = false;   // VGL contracted with an inverse column (mo_vgl_contract)
+  bool full = false;       // every coefficient but exact zeros (mo_val_full)
   std::vector<double> cmax;  // largest |C[.][m]| of each orbital
   void add(const std::string& s) { o += s; }
 
@@ -124,7 +125,7 @@ struct Gen {
         for (int k = 0; k < nocc; ++k) cmax[k] = std::max(cmax[k], std::fabs(C[mu * nocc + k]));
     }
     const double c = std::fabs(C[ao * nocc + m]);
-    return c != 0.0 && c > 1e-12 * cmax[m];
+    return c != 0.0 && (full || c > 1e-12 * cmax[m]);
   }
 
   static std::string num(double v) {
@@ -466,6 +467,17 @@ std::string generate_basis(const OqSystem& S, const OqSplit& SP, const double* C
            "  __device__ static __forceinline__ void mo_vgl_contract(const OqSystem& S,\n"
            "      const OqSplit& SP, const TC* __restrict__ C, double x, double y, double z,\n"
            "      const T* ac, T& gx, T& gy, T& gz, T& lp) {\n  (void)SP; (void)C;\n";
+    src += g.o + "  }\n";
+  }
+  {
+    Gen g{S, SP, C, nocc, ""};
+    g.full = true;
+    g.body(false);
+    src += "\n  // values with no coefficient left out: the FP64 refresh of the inverses\n"
+           "  template <typename T, typename TC>\n"
+           "  __device__ static __forceinline__ void mo_val_full(const OqSystem& S,\n"
+           "      const OqSplit& SP, const TC* __restrict__ C, double x, double y, double z,\n"
+           "      T* mv) {\n  (void)SP; (void)C;\n";
     src += g.o + "  }\n";
   }
   src += "};\n";
