@@ -205,7 +205,7 @@ int oq_ctx_sweep_local_bytes(oqmc_ctx* ctx, int W, int precision, size_t* out) {
   size_t best = 0, v = 0;
   cudaError_t err = cudaSuccess;
   auto take = [&](int kind, int M) -> bool {
-#define OQ_X(N) err = oq_local_bytes_##N(kind, mixed, M, &v)
+#define OQ_X(N) err = oq_local_bytes_##N(kind, mixed, ctx->ao_ext, M, &v)
     OQ_SWITCH(ctx->nocc, OQ_X)
 #undef OQ_X
     if (err != cudaSuccess) return false;
@@ -235,8 +235,10 @@ int oq_ctx_sweep_local_bytes(oqmc_ctx* ctx, int W, int precision, size_t* out) {
         ok = ctx->spec ? take_rtc(oq_spec_function(ctx->spec, 4 + 2 * scaled + mixed))
                        : take(8 + scaled, 0);
     }
-    // the fused sweeps hold the local energy themselves
-    if (ok && (alle || ctx->mlp || tc || !plan.fused)) {
+    // the fused sweeps and FP64 all-electron steps hold the local energy
+    // themselves
+    const bool own = alle ? mixed != 0 : ctx->mlp || tc || !plan.fused;
+    if (ok && own) {
       if (tc) ok = take(3, 0);
       else if (ctx->spec) ok = take_rtc(oq_spec_function(ctx->spec, 2 + mixed));
       else ok = take(2, 0);

@@ -224,7 +224,7 @@ cudaError_t OQ_FN(oq_alle)(const OqLaunch& L, const OqAlleArgs& a, int mixed) {
 // Per-thread local memory (bytes) of one kernel this size launches: kind 0
 // k_team (refresh), 1 k_sweeps, 2 k_eloc, 3 k_eloc_tc, 4 k_md_refresh,
 // 5 k_md_moves, 6 k_md_local (M = 8 or 16 columns), 7 k_alle, 8 and 9 k_moves
-// (fixed-width and nucleus-scaled proposal).
+// (fixed-width and nucleus-scaled proposal).  ext: OqLaunch::ext, for 0 and 7.
 template <typename K>
 static cudaError_t oq_lmem(K kernel, size_t* out) {
   cudaFuncAttributes a;
@@ -240,11 +240,19 @@ static cudaError_t md_lmem(int kind, size_t* out) {
   return oq_lmem(k_md_local<OQ_N, M>, out);
 }
 
-cudaError_t OQ_FN(oq_local_bytes)(int kind, int mixed, int M, size_t* out) {
+template <bool EXT>
+static cudaError_t tile_lmem(int kind, int mixed, size_t* out) {
+  if (kind == 0)
+    return mixed ? oq_lmem(k_team<OQ_N, OQ_TEAM_REFRESH, float, EXT>, out)
+                 : oq_lmem(k_team<OQ_N, OQ_TEAM_REFRESH, double, EXT>, out);
+  return mixed ? oq_lmem(k_alle<OQ_N, float, EXT>, out) : oq_lmem(k_alle<OQ_N, double, EXT>, out);
+}
+
+cudaError_t OQ_FN(oq_local_bytes)(int kind, int mixed, int ext, int M, size_t* out) {
   switch (kind) {
     case 0:
-      return mixed ? oq_lmem(k_team<OQ_N, OQ_TEAM_REFRESH, float, true>, out)
-                   : oq_lmem(k_team<OQ_N, OQ_TEAM_REFRESH, double, true>, out);
+    case 7:
+      return ext ? tile_lmem<true>(kind, mixed, out) : tile_lmem<false>(kind, mixed, out);
     case 1:
       return mixed ? oq_lmem(k_sweeps<OQ_N, float, float>, out)
                    : oq_lmem(k_sweeps<OQ_N, double, double>, out);
@@ -268,9 +276,6 @@ cudaError_t OQ_FN(oq_local_bytes)(int kind, int mixed, int M, size_t* out) {
       return mixed ? oq_lmem(k_moves<OQ_N, float, float, 1>, out)
                    : oq_lmem(k_moves<OQ_N, double, double, 1>, out);
 #endif
-    case 7:
-      return mixed ? oq_lmem(k_alle<OQ_N, float, true>, out)
-                   : oq_lmem(k_alle<OQ_N, double, true>, out);
   }
   return cudaErrorInvalidValue;
 }
