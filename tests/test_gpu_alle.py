@@ -159,3 +159,61 @@ def test_mixed_steps_count_every_accepted_walker(name, W):
         assert ctx.flags() == 0
     if W > 10**4:
         assert times["mixed"] < 2.5 * times["fp64"], times
+
+
+def _ext_system(name, kind):
+    mol = M.named_system(name)
+    cusp = M.synthetic_cusp_params(mol) if kind == "cusp" else None
+    pc, cfg = M.default_params_corr(mol, cusp=cusp is not None), None
+    els = sorted(set(mol.elements))
+    if kind == "bspline":
+        pc["J2_bspline"] = {"like": np.array([0.2, 0.1, 0.05]), "unlike": np.linspace(0.4, 0.0, 9)}
+        pc["J1_bspline"] = {e: np.array([-0.1, 0.05, 0.02, 0.01]) for e in els}
+        cfg = {"J2": {"r_cut": 3.5}, "J1": {e: {"r_cut": 3.0} for e in els}}
+    elif kind.startswith("j3"):
+        k = 3 if kind == "j33" else 2
+        rng = np.random.default_rng(4)
+        pc["J3_eeI"] = {p + e: rng.normal(size={2: 8, 3: 26}[k]) * 0.003 for e in els
+                        for p in ("like+", "unlike+") if p + e != "like+H"}
+        cfg = {"J3": {"N_eI": k, "N_ee": k, "r_cut": 4.0}}
+    import warnings
+    with warnings.catch_warnings():
+        warnings.simplefilter("ignore")
+        return build_system(M.make_mf(name), pc, cusp, cfg)
+
+
+@pytest.mark.parametrize("name,kind,prec,sizes", [("H2O", "j3", "fp64", (3, 65, 9001)),
+                                                  ("LiH", "j33", "fp64", (2, 4097)),
+                                                  ("H2O", "bspline", "fp64", (5, 4097)),
+                                                  ("H2O_dimer", "j3", "fp64", (1, 333)),
+                                                  ("H2O", "j3", "mixed", (3, 700)),
+                                                  ("LiH", "cusp", "fp64", (7, 2000))])
+def test_steps_with_every_jastrow_term(name, kind, prec, sizes):
+    """The general instantiation of the tile kernel (three-body and B-spline
+    terms on the proposals and in the fused local energy): chains that do not
+    depend on the tile, energies and log|psi| of the final walkers against the
+    oracle."""
+    s = _ext_system(name, kind)
+    X = seeded_walkers(s, max(sizes), 0.8, 5)
+    runs = []
+    for W in sizes:
+        ctx = GTOContext(s)
+        ctx.set_move_kind(1)
+        ens = WalkerEnsemble(ctx, X[:W], prec, seed=4, refresh_every=10**9)
+        ep = torch.zeros(W, 4, dtype=torch.float64, device="cuda")
+        ens.run(6, 0.1, measure_every=2, eparts_last=ep)
+        m = min(W, 60)
+        Xm = ens.X[:m].cpu().numpy()
+        o = O.evaluate(s, Xm)
+        sc = 0.5 * (np.sum(np.abs(o["lap"]), axis=1) + np.sum(o["grad"] ** 2, axis=(1, 2))) + 1.0
+        err = np.abs(ep[:m, 3].cpu().numpy() - o["e_loc"]) / (np.abs(o["e_loc"]) + sc)
+        assert np.max(err) < (1e-10 if prec == "fp64" else 2e-3)
+        st = ens.state_evaluate()
+        lp = st["logpsi"][:m].cpu().numpy()
+        assert np.max(np.abs(lp - o["logpsi"]) / (np.abs(o["logpsi"]) + 1)) < (
+            1e-10 if prec == "fp64" else 1e-5)
+        assert ctx.flags() == 0
+        runs.append(ens.X)
+    for a, b in zip(runs, runs[1:]):
+        assert torch.equal(a, b[: a.shape[0]])
+    assert not torch.equal(runs[-1], torch.as_tensor(X, device="cuda"))
