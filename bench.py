@@ -354,6 +354,19 @@ def fused_launches(ens, n_sweeps, measure_every=1, tensor_core_energy=False):
     return n
 
 
+def split_launches(ens, n_sweeps, generic, tensor_core_energy):
+    """Kernels that ``ens.run(n_sweeps)`` launches on the split path (E_L every
+    sweep).  Above 37,888 walkers a walker has one thread: table-driven sweeps
+    of four and more orbitals then move in a kernel of their own, as the learned
+    proposal's do, and FP64 ensembles of eight and more have their local
+    energies in one."""
+    one = ens.W > 148 * 256
+    if generic and one and ens.ctx.nocc >= 4:
+        return sweep_launches(ens, n_sweeps)
+    apart = one and not generic and ens.precision == "fp64" and ens.ctx.nocc >= 8
+    return fused_launches(ens, n_sweeps, 1, tensor_core_energy or apart)
+
+
 def adapt_step(ens, step, n_chunks=40, chunk=5, target=0.4):
     """Equilibrate with the reference's rule log s += 0.05 (acc - target)
     applied once per chunk of sweeps (OmegaQMC/vmc_gto.py:121-126)."""
@@ -453,7 +466,7 @@ def run_ours(a):
     sums = torch.zeros(K, NSUM, dtype=torch.float64, device=dev)
     ev0 = torch.cuda.Event(enable_timing=True)
     ev1 = torch.cuda.Event(enable_timing=True)
-    n_launch = fused_launches(ens, K, 1, a.eloc == "tc" and a.precision == "mixed")
+    n_launch = split_launches(ens, K, a.generic, a.eloc == "tc" and a.precision == "mixed")
     if world > 1:
         dist.barrier()
     torch.cuda.synchronize()
@@ -508,7 +521,7 @@ def run_ours(a):
         del pe
 
     # kernel-level timing of the dominant kernel on its own stream: one chunk
-    # of REFRESH_EVERY sweeps = one k_sweeps launch; the refresh separately
+    # of REFRESH_EVERY sweeps = one oqmc_sweeps call; the refresh separately
     chunk_sums = torch.zeros(REFRESH_EVERY, NSUM, dtype=torch.float64, device=dev)
     e0 = torch.cuda.Event(enable_timing=True)
     e1 = torch.cuda.Event(enable_timing=True)
@@ -563,7 +576,7 @@ def run_ours(a):
     peak_kind = 0 if a.precision == "fp64" else 1
     rate = ctypes_peak(L, peak_kind)
     achieved = work["flops"] * W * REFRESH_EVERY / (sweep_ms * 1e-3)
-    traffic = ncu_traffic(a.system, a.precision)
+    traffic = None if a.generic else ncu_traffic(a.system, a.precision)
     line = {
         "metric": "decorrelated samples/s (walker-steps/s / tau_int) vs plain FP64, H2O 64k walkers",
         "value": value, "unit": "decorrelated samples/s", "n_gpus": world, "steps": K,
@@ -594,7 +607,8 @@ def run_ours(a):
         "roofline": {"bound": "fp64" if peak_kind == 0 else "fp32",
                      "achieved": achieved / 1e12, "peak": rate / 1e12, "unit": "TFLOP/s",
                      "frac": achieved / rate if rate else None, "traffic": traffic,
-                     "kernel": "k_sweeps (one 50-sweep oqmc_sweeps call)",
+                     "kernel": ("k_moves and k_eloc" if a.generic else "k_sweeps") +
+                               " (one 50-sweep oqmc_sweeps call)",
                      "kernel_ms_per_launch": sweep_ms,
                      "refresh_ms_per_launch": refresh_ms,
                      "flops_per_walker_sweep": work["flops"],
@@ -1371,7 +1385,8 @@ def ctypes_peak(L, kind):
 
 
 def ncu_traffic(system, precision):
-    """DRAM bytes per k_sweeps launch from the committed ncu summary, if any."""
+    """DRAM bytes per generated k_sweeps launch of 50 sweeps from the committed
+    ncu summary, if any."""
     p = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     if not os.path.exists(p):
         return None
