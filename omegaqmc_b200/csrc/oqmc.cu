@@ -1429,10 +1429,6 @@ int oqmc_set_split(oqmc_ctx* ctx, double tight_alpha) {
 
 static size_t real_size(int precision);
 
-static size_t smem_sys_c64(const oqmc_ctx* ctx) {
-  return sizeof(OqSystem) + sizeof(double) * ctx->nbf * ctx->nocc;
-}
-
 static cudaError_t to_soa(const oqmc_ctx* ctx, const double* X, double* pos, int W,
                           cudaStream_t s);
 
@@ -1445,7 +1441,7 @@ int oqmc_eval(oqmc_ctx* ctx, const double* X, int W, double* logpsi, double* gra
   if (W < 0 || (W > 0 && (!X || !logpsi))) return set_err(ctx, OQ_ERR_ARG, "bad arguments%s");
   if (W == 0) return OQ_OK;
   if (ctx->md) return md_eval(ctx, X, W, logpsi, grad, lap, eparts, stream);
-  const OqLaunch L = make_launch(ctx, stream, smem_sys_c64(ctx));
+  const OqLaunch L = make_launch(ctx, stream, 0);
   cudaError_t err = cudaSuccess;
 #define OQ_X(N) err = oq_eval_##N(L, X, W, logpsi, grad, lap, eparts)
   OQ_SWITCH(ctx->nocc, OQ_X)
@@ -1459,7 +1455,7 @@ int oqmc_log_psi(oqmc_ctx* ctx, const double* X, int W, double* logpsi, void* st
   if (W < 0 || (W > 0 && (!X || !logpsi))) return set_err(ctx, OQ_ERR_ARG, "bad arguments%s");
   if (W == 0) return OQ_OK;
   if (ctx->md) return md_eval(ctx, X, W, logpsi, nullptr, nullptr, nullptr, stream);
-  const OqLaunch L = make_launch(ctx, stream, smem_sys_c64(ctx));
+  const OqLaunch L = make_launch(ctx, stream, 0);
   cudaError_t err = cudaSuccess;
 #define OQ_X(N) err = oq_logpsi_##N(L, X, W, logpsi)
   OQ_SWITCH(ctx->nocc, OQ_X)
@@ -1472,7 +1468,7 @@ int oqmc_mo_values(oqmc_ctx* ctx, const double* X, int W, double* out, void* str
   if (!ctx) return OQ_ERR_ARG;
   if (W < 0 || (W > 0 && (!X || !out))) return set_err(ctx, OQ_ERR_ARG, "bad arguments%s");
   if (W == 0) return OQ_OK;
-  const OqLaunch L = make_launch(ctx, stream, smem_sys_c64(ctx));
+  const OqLaunch L = make_launch(ctx, stream, 0);
   cudaError_t err = cudaSuccess;
 #define OQ_X(N) err = oq_movals_##N(L, X, W, out)
   OQ_SWITCH(ctx->nocc, OQ_X)
@@ -1636,7 +1632,7 @@ int oqmc_refresh(oqmc_ctx* ctx, const double* X, int W, void* state, int precisi
   }
   const OqStatePtrs st = state_ptrs(ctx, state, W, precision);
   OQ_CUDA(ctx, to_soa(ctx, X, st.pos, W, s));
-  const OqLaunch L = make_launch(ctx, stream, smem_sys_c64(ctx));
+  const OqLaunch L = make_launch(ctx, stream, 0);
   const int mixed = precision == OQ_PREC_MIXED;
   cudaError_t err = cudaSuccess;
 #define OQ_X(N) err = oq_refresh_##N(L, st.pos, W, st.ainv, st.logdet, mixed)

@@ -4,7 +4,8 @@
 // tiles from a global counter until the list is exhausted.  A tile of WT
 // walkers of one system is processed start to finish by one CTA:
 //   1. its positions are read from the system's (W, n_e, 3) walker array
-//      (one contiguous block, coalesced) into shared memory, walker-minor;
+//      (one contiguous block, coalesced) into shared memory, a walker's
+//      coordinates contiguous;
 //   2. the Slater inverses are rebuilt in FP64 (generated orbital code,
 //      Gauss-Jordan with partial pivoting), stored in shared memory as Real;
 //   3. n_sweeps single-electron sweeps run with the walkers' state resident
@@ -19,7 +20,9 @@
 //
 // Random numbers use the same Philox counters (walker, sweep, electron) as
 // the per-system move kernel, so a batched run reproduces the per-system
-// path (refresh, then sweeps) walker by walker for the same seed.
+// path (refresh, then sweeps) walker by walker for the same seed, up to a
+// decision that lies within rounding (the lanes of a walker add its pair terms
+// in an order of their own).
 //
 // The launch keeps its own bookkeeping in OqBatchCtl: the tile counter, a
 // count of finished CTAs, the sweep counter of the next launch and the next
@@ -371,7 +374,8 @@ __device__ __forceinline__ void oq_batch_tile(const OqBatchArgs& a, const OqBatc
   for (int t = 0; t < a.n_sweeps; ++t) {
     const uint32_t gstep = (uint32_t)(step0 + t);
     if (MODE != 1 && P > 1) {
-      nacc += oq_batch_sweep_lanes<NOCC, T, Real, B>(a, d, J, S, SP, C, pos, Ai, lane, P, live, (uint32_t)w, gstep, pf, logdet);
+      nacc += oq_batch_sweep_lanes<NOCC, T, Real, B>(a, d, J, S, SP, C, pos, Ai, lane, P, live,
+                                                     (uint32_t)w, gstep, pf, logdet);
     } else if (MODE != 2 && live) {
       for (int e = 0; e < NE; ++e) {
         float nf[3];

@@ -116,8 +116,8 @@ k_mlp_train(const unsigned short* __restrict__ feat, const float* __restrict__ t
   unsigned char* ht2 = smem + TR_HT2;
   unsigned char* ht3 = smem + TR_HT3;
   unsigned char* wreg = smem + TR_W;
-  // backward operands over the forward weights: W4^T (12 KB) at 0, dZ4^T (12 KB)
-  // at 32 KB, W3^T (32 KB) at 48 KB, W2^T over W4^T
+  // backward operands over the forward weights, in KB of wreg: W4^T at 0-12,
+  // dZ4^T at 32-44, W3^T at 48-80, later W2^T at 0-32 (over W4^T alone)
   unsigned char* z4t = wreg + 32768;
   unsigned char* w3t = wreg + 49152;
   float* bias = reinterpret_cast<float*>(smem + TR_BIAS);
@@ -212,7 +212,7 @@ k_mlp_train(const unsigned short* __restrict__ feat, const float* __restrict__ t
       oq_mlp_mma(tmem, act, w3t, OQ_MLP_H, OQ_MLP_H, nullptr);
       oq_mlp_mma(tmem + 128, ht2, ht3, OQ_MLP_H, OQ_MLP_H, bar);
     }
-    // W2^T over W4^T and dZ4^T, which the finished MMAs have read, while
+    // W2^T over W4^T, which the finished MMAs have read, while
     // these run
     oq_mlp_load_kmajor(wreg, wtbf + OQ_MLP_OFF_W2, OQ_MLP_H, OQ_MLP_H);
     ok = oq_mlp_wait(sy);

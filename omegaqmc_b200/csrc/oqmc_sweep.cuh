@@ -986,7 +986,7 @@ k_eloc(const OqSystem* __restrict__ gsys, const OqSplit* __restrict__ gsplit,
 // ---------------------------------------------------------------------------
 // Fused sweeps: moves and local energies of n_sweeps sweeps in one launch, with
 // P lanes (threads of one warp) per walker, P a power of two chosen from the
-// walker count (oq_sweep_lanes).
+// walker count (sweep_lanes, oqmc.cu).
 //
 // Why.  Separate move and local-energy launches per sweep with one thread per
 // walker leave most of the chip idle below some ten thousand walkers: 1,000

@@ -13,10 +13,11 @@
 // CTAs on 148 SMs.  One electron per thread gives 2 N times the threads and
 // an N-th of the chain, keeps one matrix column of N doubles in registers,
 // and costs one barrier per elimination step.  Measured per call (thread per
-// walker -> this): H2O, 1 walker 281 -> 25 us (launch and host time); N2,
-// 4,097 walkers 855 -> 60 us; (H2O)2, 16,384 walkers 1,653 -> 240 us (FP64
-// pipe 38% busy, issue slots 54%); log|psi| of 65,536 H2O walkers 181 -> 94
-// us.
+// walker -> this): H2O, 1 walker 280 -> 25 us (launch and host time); N2,
+// 4,097 walkers 855 -> 54 us, and 80 to 90 where walkers next to a node are
+// done again (see k_team); (H2O)2, 16,384 walkers, 1,653 -> 243 us, 270 to 310
+// with such walkers (FP64 pipe 38% busy, issue slots 54%); log|psi| of 65,536
+// H2O walkers 181 -> 94 us.
 #pragma once
 #include "oqmc_sweep.cuh"
 
@@ -53,7 +54,7 @@ inline int oq_team_walkers(int W) {
   return wb;
 }
 
-// The tables a tile reads, packed by the host (oq_pack_ao) into one block that
+// The tables a tile reads, packed by the host (pack_ao, oqmc.cu) into one block that
 // every CTA copies into shared memory: what the FP64 evaluation of a molecule
 // touches and nothing else (H2O: 2.5 KB against 14 KB of OqSystem and its MO
 // coefficients), laid out as the loops read it.
