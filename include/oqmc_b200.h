@@ -205,8 +205,12 @@ int oqmc_state_eval(oqmc_ctx* ctx, const void* state, int W, int precision,
  * (n_meas, W) per-walker E_L.  eparts_last: optional (W,4) parts of the
  * last measurement.  Random numbers: Philox4x32-10 keyed by seed, counter
  * (walker, step_base + sweep, electron).  walkers_per_block: CTA size (32,
- * 64 or 128; 0 = default).  Replaces the production scan body
- * (OmegaQMC/vmc_gto.py:985-1034) and metropolis_move_1w (841-905). */
+ * 64 or 128; 0 = default).  A walker's chain follows from its index, the
+ * seed and the counters.  In mixed precision it does not depend on W or
+ * walkers_per_block; in FP64 the order in which a move's pair terms are added
+ * does, so that two chains may part at a decision within rounding (1e-15).
+ * Replaces the production scan body (OmegaQMC/vmc_gto.py:985-1034) and
+ * metropolis_move_1w (841-905). */
 int oqmc_sweeps(oqmc_ctx* ctx, double* walkers, int W, void* state,
                 int precision, int n_sweeps, int measure_every, double step,
                 uint64_t seed, uint64_t step_base, double* sums,
