@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstring>
 #include <dlfcn.h>
+#include <exception>
 #include <mutex>
 #include <string>
 #include <system_error>
@@ -667,7 +668,14 @@ int oq_spec_build(const OqSystem& S, const OqSplit& SP, const double* C, int noc
   std::vector<std::string> low, low2;
   std::string err2;
   int rc = 0, rc2 = 0;
-  auto second = [&] { rc2 = oq_rtc_compile(src2, moves, &cubin2, &low2, &err2); };
+  auto second = [&] {
+    try {
+      rc2 = oq_rtc_compile(src2, moves, &cubin2, &low2, &err2);
+    } catch (const std::exception& e) {   // must not leave the thread
+      rc2 = -1;
+      err2 = e.what();
+    }
+  };
   std::thread th;
   if (two) {
     try {                       // beside the first module, on another host thread
@@ -676,7 +684,12 @@ int oq_spec_build(const OqSystem& S, const OqSplit& SP, const double* C, int noc
       second();                 // no thread to be had
     }
   }
-  rc = oq_rtc_compile(src, names, &cubin, &low, err);
+  try {
+    rc = oq_rtc_compile(src, names, &cubin, &low, err);
+  } catch (const std::exception& e) {
+    rc = -1;
+    *err = e.what();
+  }
   if (th.joinable()) th.join();
   if (rc == 0 && rc2 != 0) *err = err2;
   if (rc != 0 || rc2 != 0) return -1;

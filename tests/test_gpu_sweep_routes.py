@@ -108,3 +108,22 @@ def test_equilibration_with_one_thread_per_walker(name, prec, W, spec):
         ens2.run(1, float(w[k]))
     assert torch.equal(ens.X, ens2.X)
     assert torch.equal(ens.logdet(), ens2.logdet())
+
+
+def test_tensor_core_energies_after_one_thread_moves():
+    """The tensor-core local energy reads the state that k_moves leaves: the
+    walkers are those of the CUDA-core path and the energies the oracle's."""
+    s = _system("H2O")
+    W, out = 37889, []
+    for tc in (False, True):
+        ctx = GTOContext(s)
+        ctx.use_tensor_cores(tc)
+        ens = _ensemble(ctx, s, W, "mixed")
+        ep = torch.zeros(W, 4, dtype=torch.float64, device="cuda")
+        ens.run(4, 0.4, eparts_last=ep)
+        out.append((ens.X, ep, ens.logdet().clone()))
+        assert ctx.flags() == 0
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][2], out[1][2])
+    o = O.evaluate(s, out[1][0][:200].cpu().numpy())
+    err = np.abs(out[1][1][:200, 3].cpu().numpy() - o["e_loc"])
+    assert np.median(err) < 1e-4 and np.quantile(err, 0.99) < 2e-2
