@@ -127,19 +127,55 @@ static void compute_split(oqmc_ctx* ctx) {
 
 // Record an error on a context (used by entry points in other files).
 
-// Lanes per walker of the sweeps: as many as there are electrons (all orbital
-// rows of a sweep at once; 32 with three-body terms in FP64, which fill them),
-// halved while the threads would exceed 512 per SM.  Beyond that the register
-// file (128 per thread) is full and lanes only add shuffles.
+// Threads of a CTA of k_sweeps with `lanes` lanes per walker, and its shared
+// memory: `most` threads, halved until the walkers' state fits.
+static int sweep_cta(const oqmc_ctx* ctx, int mixed, int lanes, int most, size_t* smem) {
+  const size_t real = mixed ? sizeof(float) : sizeof(double);
+  const int cache = !mixed && lanes > 1 && ctx->hsys.has_j3;
+  const int len = cache && ctx->j3_len <= 2048 ? ctx->j3_len : 0;
+  const size_t head = sizeof(OqSystem) + sizeof(OqSplit) +
+                      (((size_t)ctx->nbf * ctx->nocc * real + 15) & ~(size_t)15);
+  for (int n = most;; n >>= 1) {
+    *smem = head + oq_sweep_tile_bytes(ctx->nocc, ctx->natm, n / lanes, real, cache, len);
+    if (*smem <= OQ_SMEM_OPTIN || n <= 32) return n;
+  }
+}
+
+// Times that W walkers on `lanes` lanes each fill the GPU: the CTAs over those
+// that are resident at once (registers: 512 threads per SM; shared memory:
+// 228 KB with 1 KB of each CTA's for the system).
+static int sweep_waves(const oqmc_ctx* ctx, int W, int mixed, int lanes) {
+  size_t smem;
+  const int n = sweep_cta(ctx, mixed, lanes, 128, &smem), wt = n / lanes;
+  const int fit = (int)(228 * 1024 / (smem + 1024)), per_sm = fit < 512 / n ? fit : 512 / n;
+  const int ctas = (W + wt - 1) / wt, room = 148 * (per_sm > 0 ? per_sm : 1);
+  return (ctas + room - 1) / room;
+}
+
+// Lanes per walker of the sweeps: at most as many as there are electrons (all
+// orbital rows of a sweep at once), and of these the number with the least
+// waves(P) x P^-e: lanes shorten a walker's chain, but by less than they add
+// threads, and what an SM holds at once is bounded by registers and, for larger
+// molecules, by the walkers' state.  e = 1/2 in FP64 and 1/5 in FP32, where
+// every lane sums all pair terms (one wave of H2O, four sweeps, FP64: 484, 340,
+// 260 and 172 us on 1, 2, 4 and 8 lanes; mixed 187, 162 and 114).  Four sweeps,
+// us, by threads alone (512 per SM) | by this: H2O FP64 30,000 walkers 557 | 485
+// (one lane), table-driven 1,348 | 999; N2 FP64 24,000: 887 | 707 (four lanes),
+// mixed 30,000: 437 | 332 (one); (H2O)2 mixed 16,384: 719 | 513 (two), FP64
+// 30,000: 4,400 | 2,236 (eight).  Above 37,888 walkers (148 x 512 threads on two
+// lanes) a walker has one lane.
 //
-// Three-body terms in FP32 are the exception: every lane sums all of them (the
-// order of that sum decides moves), so lanes repeat that work and pay only
-// while it hides in idle issue slots: all lanes up to a number of threads per
-// SM, one lane beyond.  Five sweeps, us, all lanes | one lane: H2O 2,048
-// walkers 3,316 | 3,459, 4,096: 3,933 | 3,459; orders (3, 3) 512 walkers 4,311
-// | 4,352, 4,096: 5,844 | 4,369; LiH
-// 8,192: 451 | 520, 16,384: 553 | 520; (H2O)2 2,048: 7,643 |
-// 11,000, 16 lanes at 4,096: 9,787 | 11,160.
+// Three-body terms in FP64 fill 32 lanes, halved while the threads would exceed
+// 512 per SM; they take the same time on any number of lanes once the SMs are
+// full ((H2O)2, 37,888 walkers, two | eight lanes: 20.7 | 29.1 ms).
+//
+// Three-body terms in FP32: every lane sums all of them (the order of that sum
+// decides moves), so lanes repeat that work and pay only while it hides in idle
+// issue slots: all lanes up to a number of threads per SM, one lane beyond.
+// Five sweeps, us, all lanes | one lane: H2O 2,048 walkers 3,316 | 3,459, 4,096:
+// 3,933 | 3,459; orders (3, 3) 512 walkers 4,311 | 4,352, 4,096: 5,844 | 4,369;
+// LiH 8,192: 451 | 520, 16,384: 553 | 520; (H2O)2 2,048: 7,643 | 11,000, 16 lanes
+// at 4,096: 9,787 | 11,160.
 static int sweep_lanes(const oqmc_ctx* ctx, int W, int mixed) {
   int P = 1;
   while (P < ctx->n_e && P < 32) P <<= 1;
@@ -150,9 +186,23 @@ static int sweep_lanes(const oqmc_ctx* ctx, int W, int mixed) {
     if (P == 32 && (long long)W * P > cap) P = 16;
     return (long long)W * P > cap ? 1 : P;
   }
-  if (S.has_j3) P = 32;
-  while (P > 1 && (long long)W * P > 148ll * 512) P >>= 1;
-  return P;
+  if (2ll * W > 148ll * 512) return 1;
+  if (S.has_j3) {
+    P = 32;
+    while ((long long)W * P > 148ll * 512) P >>= 1;
+    return P;
+  }
+  const double e = mixed ? 0.87 : 0.7071;          // 2^-e
+  double f = 1.0, best = 0.0;
+  int lanes = 0;
+  for (int q = 1; q <= P; q <<= 1, f *= e) {
+    const double cost = sweep_waves(ctx, W, mixed, q) * f;
+    if (!lanes || cost < 0.98 * best) {            // fewer lanes on a tie
+      best = cost;
+      lanes = q;
+    }
+  }
+  return lanes;
 }
 
 // With one lane per walker, whether the moves run in k_moves instead of
@@ -1705,17 +1755,11 @@ static int launch_moves(oqmc_ctx* ctx, const OqMoveArgs& m, int wpb, size_t sm, 
 // CTA size that fits with one lane.
 static int launch_sweeps(oqmc_ctx* ctx, OqSweepArgs a, int wpb1, int precision, void* stream) {
   const int mixed = precision == OQ_PREC_MIXED;
-  int nthr = a.lanes == 1 ? wpb1 : 128;
+  size_t smem;
+  const int nthr = sweep_cta(ctx, mixed, a.lanes, a.lanes == 1 ? wpb1 : 128, &smem);
   a.j3_cache = !mixed && a.lanes > 1 && ctx->hsys.has_j3;
   a.j3_len = a.j3_cache && ctx->j3_len <= 2048 ? ctx->j3_len : 0;
-  size_t head = sizeof(OqSystem) + sizeof(OqSplit);
-  head += ((size_t)ctx->nbf * ctx->nocc * real_size(precision) + 15) & ~(size_t)15;
-  auto bytes = [&](int n) {
-    return head + oq_sweep_tile_bytes(ctx->nocc, ctx->natm, n / a.lanes, real_size(precision),
-                                      a.j3_cache, a.j3_len);
-  };
-  while (bytes(nthr) > 227 * 1024 && nthr > 32) nthr >>= 1;
-  const OqLaunch L = make_launch(ctx, stream, bytes(nthr));
+  const OqLaunch L = make_launch(ctx, stream, smem);
   if (ctx->spec) {
     const void* C = mixed ? (const void*)ctx->d_C32 : (const void*)ctx->d_C64;
     void* args[4] = {(void*)&L.sys, (void*)&L.split, (void*)&C, (void*)&a};

@@ -41,12 +41,13 @@ def _ensemble(ctx, s, W, prec, wpb=0):
 
 
 # just above the counts at which the last lanes are given up (37,888 = 148 x 512 / 2;
+# 28,416 where three CTAs of two lanes no longer hold all walkers at once;
 # three-body terms in FP32: 148 x 256 / 16 = 2,368, 148 x 128 / 16 = 1,184 and
-# 148 x 256 / 4 = 9,472), with a
-# partial last CTA
+# 148 x 256 / 4 = 9,472), with a partial last CTA
 CASES = [("H2O", "mixed", 37889, 0, 0, 0), ("H2O", "fp64", 37889, 0, 1, 0),
          ("golden:h2o_cusp", "mixed", 40001, 0, 0, 0), ("H2O+j3", "mixed", 2369, 1, 0, 0),
          ("H2O+j3", "mixed", 2369, 1, 1, 0), ("H2O+j33", "mixed", 1185, 0, 0, 0),
+         ("H2O", "fp64", 28417, 0, 0, 0), ("N2", "mixed", 28417, 0, 1, 0),
          ("LiH+j3", "mixed", 9473, 1, 1, 0), ("LiH+j3", "fp64", 37889, 1, 0, 0),
          ("H2O+j3", "fp64", 37889, 1, 0, 0), ("H2O_dimer", "fp64", 37889, 1, 0, 0),
          ("H2O", "fp64", 1001, 1, 0, 32), ("H2O", "fp64", 1001, 1, 1, 128)]
